@@ -3,13 +3,13 @@
 //
 // Reference: the Bend prover keeps the same Montgomery representation in 16 x 16-bit limbs
 // (bend2/FORMAT.md:5-12; Fr.mul CIOS at bend2/src/fr.bend:269, Fq.mul at bend2/src/fq.bend:269,
-// n0' at fr.bend:4 / fq.bend:4).  Here one limb is 32 bits, so a product is 8 rows of
-// coarsely-integrated operand scanning (CIOS, Koc-Acar-Kaliski 1996) written as PTX
-// mad.lo/hi.cc carry chains.  Every carry chain lives inside a single asm statement so no
-// compiler-generated instruction can sit between two .cc instructions.
+// n0' at fr.bend:4 / fq.bend:4).  Here one limb is 32 bits and a product is 8 rows of operand
+// scanning with the reduction interleaved (CIOS, Koc-Acar-Kaliski 1996), written as PTX carry
+// chains of 64-bit multiply-adds (fp_wide.cuh).  Every carry chain lives inside a single asm
+// statement so no compiler-generated instruction can sit between two .cc instructions.
 //
 // Invariants: inputs and outputs of add/sub/mul are fully reduced (< p).  Both moduli are
-// below 2^254, so a CIOS row's running value stays below 2^288 (9 limbs) and the final
+// below 2^254, so a row's running value stays below 2^288 (9 limbs) and the final
 // result is below 2p; one conditional subtraction reduces it.
 #pragma once
 #include <cstdint>
@@ -168,79 +168,18 @@ template <class P>
 BG_DEV Fp<P> dbl(const Fp<P>& a) { return add(a, a); }
 
 // ---------------------------------------------------------------- Montgomery product
-// one CIOS row: t += a*bi; m = t0*n0'; t += m*p; (t0 becomes 0; the caller shifts)
-#define BG_CIOS_ROW(P)                                                                          \
-  asm("{\n\t.reg .u32 m;\n\t"                                                                   \
-      "mad.lo.cc.u32  %0, %9,  %17, %0;\n\t"                                                   \
-      "madc.lo.cc.u32 %1, %10, %17, %1;\n\t"                                                   \
-      "madc.lo.cc.u32 %2, %11, %17, %2;\n\t"                                                   \
-      "madc.lo.cc.u32 %3, %12, %17, %3;\n\t"                                                   \
-      "madc.lo.cc.u32 %4, %13, %17, %4;\n\t"                                                   \
-      "madc.lo.cc.u32 %5, %14, %17, %5;\n\t"                                                   \
-      "madc.lo.cc.u32 %6, %15, %17, %6;\n\t"                                                   \
-      "madc.lo.cc.u32 %7, %16, %17, %7;\n\t"                                                   \
-      "addc.u32       %8, %8, 0;\n\t"                                                          \
-      "mad.hi.cc.u32  %1, %9,  %17, %1;\n\t"                                                   \
-      "madc.hi.cc.u32 %2, %10, %17, %2;\n\t"                                                   \
-      "madc.hi.cc.u32 %3, %11, %17, %3;\n\t"                                                   \
-      "madc.hi.cc.u32 %4, %12, %17, %4;\n\t"                                                   \
-      "madc.hi.cc.u32 %5, %13, %17, %5;\n\t"                                                   \
-      "madc.hi.cc.u32 %6, %14, %17, %6;\n\t"                                                   \
-      "madc.hi.cc.u32 %7, %15, %17, %7;\n\t"                                                   \
-      "madc.hi.u32    %8, %16, %17, %8;\n\t"                                                   \
-      "mul.lo.u32     m, %0, %18;\n\t"                                                         \
-      "mad.lo.cc.u32  %0, m, %19, %0;\n\t"                                                     \
-      "madc.lo.cc.u32 %1, m, %20, %1;\n\t"                                                     \
-      "madc.lo.cc.u32 %2, m, %21, %2;\n\t"                                                     \
-      "madc.lo.cc.u32 %3, m, %22, %3;\n\t"                                                     \
-      "madc.lo.cc.u32 %4, m, %23, %4;\n\t"                                                     \
-      "madc.lo.cc.u32 %5, m, %24, %5;\n\t"                                                     \
-      "madc.lo.cc.u32 %6, m, %25, %6;\n\t"                                                     \
-      "madc.lo.cc.u32 %7, m, %26, %7;\n\t"                                                     \
-      "addc.u32       %8, %8, 0;\n\t"                                                          \
-      "mad.hi.cc.u32  %1, m, %19, %1;\n\t"                                                     \
-      "madc.hi.cc.u32 %2, m, %20, %2;\n\t"                                                     \
-      "madc.hi.cc.u32 %3, m, %21, %3;\n\t"                                                     \
-      "madc.hi.cc.u32 %4, m, %22, %4;\n\t"                                                     \
-      "madc.hi.cc.u32 %5, m, %23, %5;\n\t"                                                     \
-      "madc.hi.cc.u32 %6, m, %24, %6;\n\t"                                                     \
-      "madc.hi.cc.u32 %7, m, %25, %7;\n\t"                                                     \
-      "madc.hi.u32    %8, m, %26, %8;\n\t}"                                                    \
-      : "+r"(t0), "+r"(t1), "+r"(t2), "+r"(t3), "+r"(t4), "+r"(t5), "+r"(t6), "+r"(t7), "+r"(t8) \
-      : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]),         \
-        "r"(a.v[6]), "r"(a.v[7]), "r"(bi), "n"(P::N0), "n"(P::P0), "n"(P::P1), "n"(P::P2),     \
-        "n"(P::P3), "n"(P::P4), "n"(P::P5), "n"(P::P6), "n"(P::P7))
-
+// defined in fp_wide.cuh: a b R^-1 mod p for a < p and any 256-bit b; a R^-1 mod p (Montgomery ->
+// canonical)
 template <class P>
-BG_DEV Fp<P> mul(const Fp<P>& a, const Fp<P>& b) {
-  uint32_t t0 = 0, t1 = 0, t2 = 0, t3 = 0, t4 = 0, t5 = 0, t6 = 0, t7 = 0, t8 = 0;
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const uint32_t bi = b.v[i];
-    BG_CIOS_ROW(P);
-    // t0 is now zero: shift one limb down
-    t0 = t1; t1 = t2; t2 = t3; t3 = t4; t4 = t5; t5 = t6; t6 = t7; t7 = t8; t8 = 0;
-  }
-  uint32_t t[8] = {t0, t1, t2, t3, t4, t5, t6, t7};
-  Fp<P> r;
-  reduce_once<P>(r.v, t);
-  return r;
-}
-#undef BG_CIOS_ROW
+BG_DEV Fp<P> mul(const Fp<P>& a, const Fp<P>& b);
+template <class P>
+BG_DEV Fp<P> from_mont(const Fp<P>& a);
 
 // squaring product (28 off-diagonal limb products doubled, then one reduction; fp_wide.cuh)
 template <class P>
 BG_DEV Fp<P> sqr_wide(const Fp<P>& a);
 template <class P>
 BG_DEV Fp<P> sqr(const Fp<P>& a) { return sqr_wide(a); }
-
-// x * 2^-256: Montgomery -> canonical (multiply by the raw integer 1)
-template <class P>
-BG_DEV Fp<P> from_mont(const Fp<P>& a) {
-  Fp<P> one_raw = fp_zero<P>();
-  one_raw.v[0] = 1;
-  return mul(a, one_raw);
-}
 
 // a^e for a 256-bit exponent given as 8 limbs (square-and-multiply, MSB first)
 template <class P>

@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kPairThreads<F>, 2)
           const Affine<F> p = pair_point<F, kFirst>(src, cp), q = pair_point<F, kFirst>(src, cq);
           inverted = pair_kind(p, q, d) <= kPairTangent;
         }
-        if (inverted) acc = fmul(acc, d);
+        if (inverted) acc = imul(acc, d);
       }
       store_elem(dst + j * PW, acc);
     }
@@ -230,11 +230,11 @@ __global__ void __launch_bounds__(kPairThreads<F>, 2)
         if (t > 0) {
           F prev;
           load_elem(prev, dst + (j - 1) * PW);
-          dinv = fmul(inv, prev);
+          dinv = imul(inv, prev);
         } else {
           dinv = inv;
         }
-        inv = fmul(inv, d);
+        inv = imul(inv, d);
       }
       r = pair_finish(p, q, kind, dinv);
     } else if (kind_src == kSrcCopy) {

@@ -38,16 +38,6 @@ struct ScaleTab {
   int bits = 0;
 };
 
-// a b as the 512-bit Karatsuba product and one Montgomery reduction (232 multiply-adds instead
-// of CIOS's 264; the inputs are below r, so the product is below r R): 2^20 forward transform
-// 0.357 -> 0.352 ms, bit-identical.  Stage-pair register blocks (radix-4 sets, half the
-// shared-memory round trips) were measured slower, 0.40 ms.
-BG_DEV Fr mul_kara(const Fr& a, const Fr& b) {
-  Wide t;
-  wide_mul(t, a.v, b.v);
-  return redc<FrParams>(t);
-}
-
 BG_DEV Fr scale_factor(int mode, size_t j, int L, const ScaleTab& t) {
   if (mode == SC_CONST) return load_fp<FrParams>(t.hi);
   size_t i = j;
@@ -106,7 +96,7 @@ __global__ void __launch_bounds__(NT) k_ntt_pass(NttVecs vecs, const uint32_t* _
     const size_t j = (s0 == 0) ? ((gid << k) | (size_t)t)
                                : (((gid >> s0) << (s0 + k)) | ((size_t)t << s0) | (gid & lomask));
     Fr x = load_fp<FrParams>(data + 8 * j);
-    if (pre_mode != SC_NONE) x = mul(x, scale_factor(pre_mode, j, L, sc));
+    if (pre_mode != SC_NONE) x = mul(scale_factor(pre_mode, j, L, sc), x);
     tile_store(sm, E, (grp << k) | t, x);
   }
   __syncthreads();
@@ -132,12 +122,12 @@ __global__ void __launch_bounds__(NT) k_ntt_pass(NttVecs vecs, const uint32_t* _
       } else {
         const Fr w = load_fp<FrParams>(tw + 8 * widx);
         if (DIT) {
-          x2 = mul_kara(x2, w);
+          x2 = mul(w, x2);
           y1 = add(x1, x2);
           y2 = sub(x1, x2);
         } else {
           y1 = add(x1, x2);
-          y2 = mul_kara(sub(x1, x2), w);
+          y2 = mul(w, sub(x1, x2));
         }
       }
       tile_store(sm, E, e1, y1);
@@ -159,7 +149,7 @@ __global__ void __launch_bounds__(NT) k_ntt_pass(NttVecs vecs, const uint32_t* _
     const size_t j = (s0 == 0) ? ((gid << k) | (size_t)t)
                                : (((gid >> s0) << (s0 + k)) | ((size_t)t << s0) | (gid & lomask));
     Fr x = tile_load(sm, E, (grp << k) | t);
-    if (post_mode != SC_NONE) x = mul(x, scale_factor(post_mode, j, L, sc));
+    if (post_mode != SC_NONE) x = mul(scale_factor(post_mode, j, L, sc), x);
     store_fp(data + 8 * j, x);
   }
 }
