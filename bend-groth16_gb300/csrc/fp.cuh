@@ -28,9 +28,9 @@ struct FqParams {
   // R mod p (Montgomery one)
   static constexpr uint32_t ONE0 = 0xc58f0d9du, ONE1 = 0xd35d438du, ONE2 = 0xf5c70b3du, ONE3 = 0x0a78eb28u,
                             ONE4 = 0x7879462cu, ONE5 = 0x666ea36fu, ONE6 = 0x9a07df2fu, ONE7 = 0x0e0a77c1u;
-  // R^3 mod p (turns the inverse of a Montgomery representative into a Montgomery inverse)
-  static constexpr uint32_t R3_0 = 0xda1530dfu, R3_1 = 0xb1cd6dafu, R3_2 = 0xa7283db6u, R3_3 = 0x62f210e6u,
-                            R3_4 = 0x0ada0afbu, R3_5 = 0xef7f0b0cu, R3_6 = 0x2d592544u, R3_7 = 0x20fd6e90u;
+  // R^2 mod p (turns the inverse of a Montgomery representative into a Montgomery inverse)
+  static constexpr uint32_t R2_0 = 0x538afa89u, R2_1 = 0xf32cfc5bu, R2_2 = 0xd44501fbu, R2_3 = 0xb5e71911u,
+                            R2_4 = 0x0a417ff6u, R2_5 = 0x47ab1effu, R2_6 = 0xcab8351fu, R2_7 = 0x06d89f71u;
 };
 struct FrParams {
   static constexpr uint32_t P0 = 0xf0000001u, P1 = 0x43e1f593u, P2 = 0x79b97091u, P3 = 0x2833e848u,
@@ -38,8 +38,8 @@ struct FrParams {
   static constexpr uint32_t N0 = 0xefffffffu;
   static constexpr uint32_t ONE0 = 0x4ffffffbu, ONE1 = 0xac96341cu, ONE2 = 0x9f60cd29u, ONE3 = 0x36fc7695u,
                             ONE4 = 0x7879462eu, ONE5 = 0x666ea36fu, ONE6 = 0x9a07df2fu, ONE7 = 0x0e0a77c1u;
-  static constexpr uint32_t R3_0 = 0xb4bf0040u, R3_1 = 0x5e94d8e1u, R3_2 = 0x1cfbb6b8u, R3_3 = 0x2a489cbeu,
-                            R3_4 = 0xa19fcfedu, R3_5 = 0x893cc664u, R3_6 = 0x7fcc657cu, R3_7 = 0x0cf8594bu;
+  static constexpr uint32_t R2_0 = 0xae216da7u, R2_1 = 0x1bb8e645u, R2_2 = 0xe35c59e3u, R2_3 = 0x53fe3ab1u,
+                            R2_4 = 0x53bb8085u, R2_5 = 0x8c49833du, R2_6 = 0x7f4e44a5u, R2_7 = 0x0216d0b1u;
 };
 
 template <class P>
@@ -201,143 +201,160 @@ BG_DEV Fp<P> inv(const Fp<P>& a) {
   return pow_limbs(a, e);
 }
 
-// ---------------------------------------------------------------- inversion by binary Euclid
-// 1/a for a Montgomery element a (0 -> 0).  Binary extended Euclid (Hankerson, Menezes and
-// Vanstone, Guide to Elliptic Curve Cryptography, Algorithm 2.22) on the representative aR,
-// with the invariants (aR) x1 = u and (aR) x2 = v (mod p) from u = aR, v = p: strip the factors
-// of two from u (x1 follows with x1 / 2^k mod p), subtract the smaller of the odd u, v from the
-// larger (x1 or x2 follows), until u or v is 1; one Montgomery product by R^3 mod p then turns
-// (aR)^-1 into a^-1 R.  The k trailing zeros of u leave in one step: x1 / 2^k mod p is the exact
-// quotient (x1 + m p) / 2^k with m = x1 (-p^-1) mod 2^k, which is below p for x1 < p, so a
-// pass is a subtraction, a shift and one 8-limb multiply-add, about 250 passes in all.  One
-// thread computes the inversion that a whole CTA of the batch-affine bucket accumulation waits
-// for, so its latency is what counts (the Fermat power is 320 dependent products).  Variable
-// time (the inputs are public bucket coordinates).  Requires a < p (every stored element is).
-namespace binv {
-BG_DEV bool is_one8(const uint32_t* u) {
-  return u[0] == 1u && (u[1] | u[2] | u[3] | u[4] | u[5] | u[6] | u[7]) == 0u;
+// ---------------------------------------------------------------- inversion by division steps
+// 1/a for a Montgomery element a (0 -> 0): the division steps of Bernstein and Yang ("Fast
+// constant-time gcd computation and modular inversion", CHES 2019), in the variant that starts at
+// delta = 1/2 and needs at most 590 steps for inputs below 2^256.  30 steps at a time run on the
+// low words of f and g alone and give a 2 x 2 matrix (entries at most 2^30), which is then applied
+// to the whole f and g (exactly divisible by 2^30) and to d and e, which follow f and g modulo p:
+// (u d + v e + m p) / 2^30 with the m, centred in +-2^29, that makes it whole, so d and e grow by
+// at most p / 2 per matrix and need no reduction before the end.  e starts at R^2, so d ends as
+// +-(a R)^-1 R^2, the Montgomery inverse.  The inversion is what a CTA of the batch-affine bucket
+// accumulation waits for, so its latency counts: the steps are the same for every input (no
+// divergence between lanes that invert together), about 20 instructions each, and a matrix costs
+// 90 multiply-adds; binary Euclid with its compares and shifts of whole numbers took about three
+// times as long, the Fermat power is 320 dependent products.  Requires a < p (every stored element
+// is).
+namespace dsteps {
+constexpr int32_t kMask = 0x3fffffff;  // 30-bit limbs, nine of them, the top one signed
+// limb i of an 8-word number
+BG_DEV int32_t limb30(const uint32_t* w, int i) {
+  const int bit = 30 * i, l = bit >> 5, s = bit & 31;
+  const uint32_t lo = w[l] >> s;
+  const uint32_t hi = (s && l + 1 < 8) ? w[l + 1] << (32 - s) : 0u;
+  return (int32_t)((lo | hi) & (uint32_t)kMask);
 }
-BG_DEV int ctz32(uint32_t x) {
-#ifdef __CUDA_ARCH__
-  return __ffs((int)x) - 1;
-#else
-  return __builtin_ctz(x);
-#endif
-}
-// u >>= k, 1 <= k <= 31
-BG_DEV void shr8(uint32_t* u, int k) {
-#pragma unroll
-  for (int i = 0; i < 7; i++) u[i] = (u[i] >> k) | (u[i + 1] << (32 - k));
-  u[7] >>= k;
-}
-// x = x / 2^k mod p for x < p, 1 <= k <= 31: (x + m p) / 2^k, m = x n0' mod 2^k
-BG_DEV void div2k_mod(uint32_t* x, int k, const uint32_t* p, uint32_t n0) {
-  const uint32_t m = (x[0] * n0) & ((1u << k) - 1u);
-  uint32_t t[9];
-  uint64_t c = 0;
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    c += (uint64_t)x[i] + (uint64_t)m * p[i];
-    t[i] = (uint32_t)c;
-    c >>= 32;
+// 30 division steps on the low words: (f, g) -> matrix (u, v; q, r) / 2^30; eta = -delta - 1/2
+BG_DEV int32_t steps30(int32_t eta, uint32_t f, uint32_t g, int32_t* mat) {
+  uint32_t u = 1, v = 0, q = 0, r = 1;
+#pragma unroll 6
+  for (int i = 0; i < 30; i++) {
+    uint32_t c1 = (uint32_t)(eta >> 31);  // delta > 0
+    const uint32_t c2 = 0u - (g & 1u);
+    const uint32_t x = (f ^ c1) - c1, y = (u ^ c1) - c1, z = (v ^ c1) - c1;  // +-f, u, v
+    g += x & c2;
+    q += y & c2;
+    r += z & c2;
+    c1 &= c2;  // swap: delta > 0 and g odd
+    eta = (int32_t)(((uint32_t)eta ^ c1) - 1u);
+    f += g & c1;
+    u += q & c1;
+    v += r & c1;
+    g >>= 1;
+    u <<= 1;
+    v <<= 1;
   }
-  t[8] = (uint32_t)c;
-#pragma unroll
-  for (int i = 0; i < 8; i++) x[i] = (t[i] >> k) | (t[i + 1] << (32 - k));
+  mat[0] = (int32_t)u;
+  mat[1] = (int32_t)v;
+  mat[2] = (int32_t)q;
+  mat[3] = (int32_t)r;
+  return eta;
 }
-// strip the factors of two of u (u != 0), dividing x by the same power of two mod p
-BG_DEV void strip2(uint32_t* u, uint32_t* x, const uint32_t* p, uint32_t n0) {
-  for (int limb = 0; limb < 8 && u[0] == 0u; limb++) {  // rare: a whole zero limb, two steps of 16 bits
+BG_DEV void update_fg(int32_t* f, int32_t* g, const int32_t* m) {
+  int64_t cf = (int64_t)m[0] * f[0] + (int64_t)m[1] * g[0];
+  int64_t cg = (int64_t)m[2] * f[0] + (int64_t)m[3] * g[0];
+  cf >>= 30;
+  cg >>= 30;
 #pragma unroll
-    for (int i = 0; i < 7; i++) u[i] = u[i + 1];
-    u[7] = 0u;
-    div2k_mod(x, 16, p, n0);
-    div2k_mod(x, 16, p, n0);
+  for (int i = 1; i < 9; i++) {
+    const int32_t fi = f[i], gi = g[i];
+    cf += (int64_t)m[0] * fi + (int64_t)m[1] * gi;
+    cg += (int64_t)m[2] * fi + (int64_t)m[3] * gi;
+    f[i - 1] = (int32_t)cf & kMask;
+    g[i - 1] = (int32_t)cg & kMask;
+    cf >>= 30;
+    cg >>= 30;
   }
-  if (u[0] == 0u) return;  // u = 0: only for an input that is 0 mod p
-  const int k = ctz32(u[0]);
-  if (k) {
-    shr8(u, k);
-    div2k_mod(x, k, p, n0);
-  }
+  f[8] = (int32_t)cf;
+  g[8] = (int32_t)cg;
 }
-// u -= v when u >= v (returns true), else leaves u and returns false
-BG_DEV bool sub_if_geq(uint32_t* u, const uint32_t* v) {
-  uint32_t d[8];
-  uint64_t b = 0;
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const uint64_t t = (uint64_t)u[i] - v[i] - b;
-    d[i] = (uint32_t)t;
-    b = t >> 63;
-  }
-  if (b) return false;
-#pragma unroll
-  for (int i = 0; i < 8; i++) u[i] = d[i];
-  return true;
+// x -> m with x + m p divisible by 2^30, -2^29 <= m < 2^29 (n30 = -p^-1 mod 2^30)
+BG_DEV int32_t centre(int64_t x, uint32_t n30) {
+  return (int32_t)(((uint32_t)x * n30) << 2) >> 2;
 }
-BG_DEV void sub8(uint32_t* u, const uint32_t* v) {
-  uint64_t b = 0;
+BG_DEV void update_de(int32_t* d, int32_t* e, const int32_t* m, const int32_t* p, uint32_t n30) {
+  int64_t cd = (int64_t)m[0] * d[0] + (int64_t)m[1] * e[0];
+  int64_t ce = (int64_t)m[2] * d[0] + (int64_t)m[3] * e[0];
+  const int32_t md = centre(cd, n30), me = centre(ce, n30);
+  cd += (int64_t)md * p[0];
+  ce += (int64_t)me * p[0];
+  cd >>= 30;
+  ce >>= 30;
 #pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const uint64_t t = (uint64_t)u[i] - v[i] - b;
-    u[i] = (uint32_t)t;
-    b = t >> 63;
+  for (int i = 1; i < 9; i++) {
+    const int32_t di = d[i], ei = e[i];
+    cd += (int64_t)m[0] * di + (int64_t)m[1] * ei + (int64_t)md * p[i];
+    ce += (int64_t)m[2] * di + (int64_t)m[3] * ei + (int64_t)me * p[i];
+    d[i - 1] = (int32_t)cd & kMask;
+    e[i - 1] = (int32_t)ce & kMask;
+    cd >>= 30;
+    ce >>= 30;
   }
+  d[8] = (int32_t)cd;
+  e[8] = (int32_t)ce;
 }
-// x = x - y mod p (x, y < p)
-BG_DEV void sub_mod(uint32_t* x, const uint32_t* y, const uint32_t* p) {
-  uint64_t b = 0;
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const uint64_t t = (uint64_t)x[i] - y[i] - b;
-    x[i] = (uint32_t)t;
-    b = t >> 63;
-  }
-  if (b) {
-    uint64_t c = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      c += (uint64_t)x[i] + p[i];
-      x[i] = (uint32_t)c;
-      c >>= 32;
-    }
-  }
-}
-}  // namespace binv
+}  // namespace dsteps
 
 template <class P>
 BG_DEV Fp<P> inv_binary(const Fp<P>& a) {
-  if (is_zero(a)) return a;
-  const uint32_t p[8] = {P::P0, P::P1, P::P2, P::P3, P::P4, P::P5, P::P6, P::P7};
-  uint32_t u[8], v[8], x1[8], x2[8];
+  const uint32_t pw[8] = {P::P0, P::P1, P::P2, P::P3, P::P4, P::P5, P::P6, P::P7};
+  const uint32_t r2[8] = {P::R2_0, P::R2_1, P::R2_2, P::R2_3, P::R2_4, P::R2_5, P::R2_6, P::R2_7};
+  int32_t p[9], f[9], g[9], d[9], e[9], m[4];
 #pragma unroll
-  for (int i = 0; i < 8; i++) {
-    u[i] = a.v[i];
-    v[i] = p[i];
-    x1[i] = 0;
-    x2[i] = 0;
+  for (int i = 0; i < 9; i++) {
+    p[i] = f[i] = dsteps::limb30(pw, i);
+    g[i] = dsteps::limb30(a.v, i);
+    d[i] = 0;
+    e[i] = dsteps::limb30(r2, i);
   }
-  x1[0] = 1;
-  // v is odd from the start and after every strip; each pass removes at least one bit from
-  // u v (below 2^508), so 512 passes always suffice
-  for (int pass = 0; pass < 512; pass++) {
-    binv::strip2(u, x1, p, P::N0);
-    if (binv::is_one8(u) || binv::is_one8(v)) break;
-    if (binv::sub_if_geq(u, v)) {
-      binv::sub_mod(x1, x2, p);
-    } else {
-      binv::sub8(v, u);
-      binv::sub_mod(x2, x1, p);
-      binv::strip2(v, x2, p, P::N0);
+  int32_t eta = -1;  // delta = 1/2
+#pragma unroll 1
+  for (int b = 0; b < 20; b++) {  // 600 steps
+    eta = dsteps::steps30(eta, (uint32_t)(f[0] | (f[1] << 30)), (uint32_t)(g[0] | (g[1] << 30)), m);
+    dsteps::update_de(d, e, m, p, P::N0 & 0x3fffffffu);
+    dsteps::update_fg(f, g, m);
+    int32_t left = 0;
+#pragma unroll
+    for (int i = 0; i < 9; i++) left |= g[i];
+    if (left == 0) break;
+  }
+  // f = +-1, d = +-1/a with |d| <= (1/2 + 20/2) p: make it d f, then add 11 p and subtract 16 p, 8 p,
+  // 4 p, 2 p and p where they fit (a = 0 leaves d = 0)
+  const int32_t sign = f[8] >> 31;
+  int64_t c = 0;
+  int32_t t[9];
+#pragma unroll
+  for (int i = 0; i < 9; i++) {
+    c += (int64_t)((d[i] ^ sign) - sign) + (int64_t)11 * p[i];
+    t[i] = (int32_t)c & dsteps::kMask;
+    c >>= 30;  // ends at zero: the sum is below 22 p < 2^259
+  }
+#pragma unroll
+  for (int k = 4; k >= 0; k--) {
+    int32_t s[9];
+    int64_t bw = 0;
+#pragma unroll
+    for (int i = 0; i < 9; i++) {
+      bw += (int64_t)t[i] - ((int64_t)p[i] << k);
+      s[i] = (int32_t)bw & dsteps::kMask;
+      bw >>= 30;
+    }
+    if (bw >= 0) {
+#pragma unroll
+      for (int i = 0; i < 9; i++) t[i] = s[i];
     }
   }
-  Fp<P> r, r3;
+  Fp<P> r;
 #pragma unroll
-  for (int i = 0; i < 8; i++) r.v[i] = binv::is_one8(u) ? x1[i] : x2[i];
-  r3.v[0] = P::R3_0; r3.v[1] = P::R3_1; r3.v[2] = P::R3_2; r3.v[3] = P::R3_3;
-  r3.v[4] = P::R3_4; r3.v[5] = P::R3_5; r3.v[6] = P::R3_6; r3.v[7] = P::R3_7;
-  return mul(r, r3);
+  for (int i = 0; i < 8; i++) {
+    // word i spans 30-bit limbs l and l + 1 (and l + 2 never: 32 <= 60 - 28)
+    const int bit = 32 * i, l = bit / 30, sft = bit % 30;
+    uint32_t w = (uint32_t)t[l] >> sft;
+    w |= (uint32_t)t[l + 1] << (30 - sft);
+    if (60 - sft < 32 && l + 2 < 9) w |= (uint32_t)t[l + 2] << (60 - sft);
+    r.v[i] = w;
+  }
+  return r;
 }
 
 // ---------------------------------------------------------------- Fq2 = Fq[u]/(u^2 + 1)

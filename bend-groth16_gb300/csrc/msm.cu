@@ -43,15 +43,16 @@ constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
 
+// (inputs rounded up to multiples of pad + 1, pad + 1 a power of two)
 __global__ void k_scan_tile(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
-                            uint32_t* __restrict__ tile_sums, size_t n) {
+                            uint32_t* __restrict__ tile_sums, size_t n, uint32_t pad) {
   __shared__ uint32_t warp_tot[kScanThreads / 32];
   const size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
   uint32_t v[kScanItems];
   uint32_t sum = 0;
 #pragma unroll
   for (int k = 0; k < kScanItems; k++) {
-    v[k] = (base + k < n) ? in[base + k] : 0u;
+    v[k] = (base + k < n) ? (in[base + k] + pad) & ~pad : 0u;
     sum += v[k];
   }
   // inclusive warp scan of per-thread sums
@@ -90,18 +91,18 @@ __global__ void k_scan_add(uint32_t* __restrict__ out, const uint32_t* __restric
 
 // exclusive scan of n u32 (n >= 1); recursion depth log_2048(n)
 void exclusive_scan(Workspace& ws, const std::string& tag, const uint32_t* d_in, uint32_t* d_out, size_t n,
-                    cudaStream_t st, int depth) {
+                    cudaStream_t st, int depth, uint32_t pad) {
   const unsigned tiles = ceil_div(n, kScanTile);
   if (tiles == 1) {
-    k_scan_tile<<<1, kScanThreads, 0, st>>>(d_in, d_out, nullptr, n);
+    k_scan_tile<<<1, kScanThreads, 0, st>>>(d_in, d_out, nullptr, n, pad);
     BG_CHECK_LAUNCH();
     return;
   }
   uint32_t* sums = ws.get_t<uint32_t>(tag + ".scan_sums" + std::to_string(depth), tiles);
   uint32_t* offs = ws.get_t<uint32_t>(tag + ".scan_offs" + std::to_string(depth), tiles);
-  k_scan_tile<<<tiles, kScanThreads, 0, st>>>(d_in, d_out, sums, n);
+  k_scan_tile<<<tiles, kScanThreads, 0, st>>>(d_in, d_out, sums, n, pad);
   BG_CHECK_LAUNCH();
-  exclusive_scan(ws, tag, sums, offs, tiles, st, depth + 1);
+  exclusive_scan(ws, tag, sums, offs, tiles, st, depth + 1, 0);
   k_scan_add<<<ceil_div(n, 256), 256, 0, st>>>(d_out, offs, n);
   BG_CHECK_LAUNCH();
 }
@@ -433,6 +434,10 @@ inline uint32_t slice_entries(size_t max_entries, size_t nkeys, double piece_us 
   return best;
 }
 
+// Most positions a thread of a pair round takes: the CTA's batch that shares an inversion (18 us with
+// its tree, which the CTA's neighbours on the SM start together).  G1 MSM 2^20's two rounds: 1.82 ms
+// with at most 24 positions, 1.73 with 48, 1.71 with 128 (one wave of 115 and 57).
+constexpr double kPairPer = 64;
 // Resident threads of a pair round on the whole GPU (SMs x CTAs per SM x CTA size).
 template <class F>
 double pair_slots() {
@@ -442,7 +447,8 @@ double pair_slots() {
     int dev = 0, sms = 0, occ = 0;
     BG_CUDA(cudaGetDevice(&dev));
     BG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    BG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pair_round<F, true>, kPairThreads<F>, 0));
+    BG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pair_round<F, true>, kPairThreads<F>,
+                                                          pair_smem_bytes<F>()));
     s = (double)sms * (occ > 0 ? occ : 1) * kPairThreads<F>;
     slots.store(s);
   }
@@ -886,7 +892,7 @@ struct HostField<Fq2> {
 };
 
 void msm_sort(Ctx& ctx, cudaStream_t st, const std::string& tag, const uint32_t* d_scalars, size_t n, int c,
-              bool shared_set, MsmSort& out) {
+              bool shared_set, int rounds, MsmSort& out) {
   out = MsmSort();
   out.n = n;
   if (n == 0) return;
@@ -898,27 +904,33 @@ void msm_sort(Ctx& ctx, cudaStream_t st, const std::string& tag, const uint32_t*
   const size_t nkeys = (size_t)sets * nb;
   const uint32_t key_stride = shared_set ? 0u : nb;
   const uint32_t idx_stride = shared_set ? (uint32_t)n : 0u;
-  const size_t max_entries = n * (size_t)W;
+  size_t max_entries = n * (size_t)W;
   if (max_entries >= 0x80000000ull) throw Error(BG_E_ARG, "msm: n x windows must be below 2^31");
+  // buckets padded for the pair rounds, as many as the padding allows
+  while (rounds > 0 && (nkeys << rounds) > std::max(8 * max_entries, size_t(1) << 20)) rounds--;
+  const size_t padded = max_entries + nkeys * ((size_t(1) << rounds) - 1);
+  if (padded >= 0x80000000ull) throw Error(BG_E_ARG, "msm: n x windows must be below 2^31");
+  out.rounds = rounds;
   out.c = c;
   out.W = W;
   out.sets = sets;
   out.nb = nb;
   out.nkeys = nkeys;
-  out.max_entries = max_entries;
+  out.max_entries = padded;
 
   Workspace& ws = ctx.ws;
   uint32_t* counts = ws.get_t<uint32_t>(tag + ".counts", nkeys + 1);
   uint32_t* cursor = ws.get_t<uint32_t>(tag + ".cursor", nkeys + 1);
   out.offsets = ws.get_t<uint32_t>(tag + ".offsets", nkeys + 1);
-  out.sorted = ws.get_t<uint32_t>(tag + ".sorted", max_entries);
+  out.sorted = ws.get_t<uint32_t>(tag + ".sorted", padded);
   BG_CUDA(cudaMemsetAsync(counts, 0, (nkeys + 1) * sizeof(uint32_t), st));
+  if (rounds) BG_CUDA(cudaMemsetAsync(out.sorted, 0xff, padded * sizeof(uint32_t), st));  // null entries
   {
     KernelTimer kt(ctx, "msm_digits", st);
     k_digits_hist<<<ceil_div(n, 256), 256, 0, st>>>(d_scalars, n, c, W, key_stride, counts, ctx.d_status);
     BG_CHECK_LAUNCH();
   }
-  exclusive_scan(ws, tag, counts, out.offsets, nkeys + 1, st, 0);
+  exclusive_scan(ws, tag, counts, out.offsets, nkeys + 1, st, 0, (1u << rounds) - 1u);
   BG_CUDA(cudaMemcpyAsync(cursor, out.offsets, (nkeys + 1) * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
   {
     KernelTimer kt(ctx, "msm_scatter", st);
@@ -949,43 +961,43 @@ void msm_accumulate(Ctx& ctx, cudaStream_t st, const std::string& tag, const uin
   if (so.done) BG_CUDA(cudaStreamWaitEvent(st, so.done, 0));
   Ctx* prof = (ctx.profile || ctx.timeline) ? &ctx : nullptr;
 
-  // Batch-affine pair rounds, where the cost model (or the tuning override) takes them, halve
-  // every bucket in affine coordinates first (msm_pairs.cuh); the XYZZ accumulation, the heavy
-  // pass and the reduction then read the last level's points directly, with its offsets.
+  // Batch-affine pair rounds, as many as the sort padded its buckets for, halve every bucket in
+  // affine coordinates first (msm_pairs.cuh); the XYZZ accumulation, the heavy pass and the
+  // reduction then read the last level's points directly, with its offsets.  Accumulations queued
+  // on one stream share the levels' memory.
   const uint32_t* acc_points = d_points;
   const uint32_t* acc_sorted = so.sorted;
   const uint32_t* acc_offsets = so.offsets;
   size_t acc_entries = so.max_entries;
-  const int rounds = ctx.pair_rounds_override >= 0 ? ctx.pair_rounds_override
-                                                   : pair_rounds_model(so.max_entries, so.nkeys, FW == 16);
+  const int rounds = so.rounds;
   if (rounds > 0) {
     constexpr int NT = kPairThreads<F>;
     const double pslots = pair_slots<F>();
-    const uint32_t me = (uint32_t)so.max_entries;
+    const size_t me = so.max_entries;
     const uint32_t nk = (uint32_t)so.nkeys;
-    uint32_t* lvl[2] = {ws.get_t<uint32_t>(tag + ".pairs0", level_start(me, nk, 1) * 2 * FW), nullptr};
-    if (rounds > 1) lvl[1] = ws.get_t<uint32_t>(tag + ".pairs1", level_start(me, nk, 2) * 2 * FW);
+    const std::string lv = plan.own_stream ? tag : "acc";
+    uint32_t* lvl[2] = {ws.get_t<uint32_t>(lv + ".pairs0", (me >> 1) * 2 * FW), nullptr};
+    if (rounds > 1) lvl[1] = ws.get_t<uint32_t>(lv + ".pairs1", (me >> 2) * 2 * FW);
     uint32_t* fin = ws.get_t<uint32_t>(tag + ".pair_offsets", so.nkeys + 1);
     KernelTimer kt(ctx, FW == 8 ? "msm_pair_g1" : "msm_pair_g2", st);
     for (int r = 0; r < rounds; r++) {
-      // Up to 256 positions per thread, in a whole number of waves of resident threads: one
-      // wave of long batches amortises each CTA's product tree and inversion best (G1 MSM 2^20
-      // round 0: 1.99 ms with 32 positions per thread in 4 waves, 1.78 ms in one wave of 118).
-      const double outs = (double)level_start(me, nk, r + 1);
-      const double waves = std::max(1.0, std::ceil(outs / (pslots * 256.0)));
+      const double outs = (double)(me >> (r + 1));
+      const double waves = std::max(1.0, std::ceil(outs / (pslots * kPairPer)));
       const uint32_t per = (uint32_t)std::max(1.0, std::ceil(outs / (waves * pslots)));
       const unsigned grid = ceil_div(ceil_div((size_t)outs, per), NT);
+      if (!grid) continue;
       if (r == 0)
-        k_pair_round<F, true><<<grid, NT, 0, st>>>(d_points, so.sorted, so.offsets, nk, 0, per, lvl[0], rounds, fin);
+        k_pair_round<F, true><<<grid, NT, pair_smem_bytes<F>(), st>>>(d_points, so.sorted, so.offsets, nk, 0, per,
+                                                                      lvl[0], rounds, fin);
       else
-        k_pair_round<F, false><<<grid, NT, 0, st>>>(lvl[(r - 1) & 1], nullptr, so.offsets, nk, r, per, lvl[r & 1],
-                                                    rounds, nullptr);
+        k_pair_round<F, false><<<grid, NT, pair_smem_bytes<F>(), st>>>(lvl[(r - 1) & 1], nullptr, so.offsets, nk, r,
+                                                                       per, lvl[r & 1], rounds, nullptr);
       BG_CHECK_LAUNCH();
     }
     acc_points = lvl[(rounds - 1) & 1];
     acc_sorted = nullptr;
     acc_offsets = fin;
-    acc_entries = level_start(me, nk, rounds);
+    acc_entries = me >> rounds;
   }
   plan.entries = acc_entries;
   uint32_t* buckets = ws.get_t<uint32_t>(tag + ".buckets", so.nkeys * PW);
@@ -1068,26 +1080,33 @@ void msm_accumulate(Ctx& ctx, cudaStream_t st, const std::string& tag, const uin
   plan.host_window_sums = ctx.host_cache.get_t<uint32_t>(tag + ".window_sums", (size_t)so.sets * J * 2 * PW);
 }
 
+int msm_rounds(const Ctx& ctx, size_t n, int c, bool shared_set, bool g2) {
+  if (ctx.pair_rounds_override >= 0) return ctx.pair_rounds_override;
+  const size_t W = 254 / c + 1;
+  return pair_rounds_model(n, n * W, (shared_set ? 1 : W) << (c - 1), g2, shared_set);
+}
+
 template <class F>
 void msm_launch(Ctx& ctx, cudaStream_t st, const std::string& tag, const uint32_t* d_points,
                 const uint32_t* d_scalars, size_t n, MsmPlan& plan, cudaStream_t st_reduce, const MsmTable* table) {
   if (table && table->n != n) throw Error(BG_E_ARG, "msm: window table built for another size");
   const int c = table ? table->c : (plan.c > 0 ? plan.c : msm_pick_c(n, FieldWords<F>::value == 16));
   MsmSort so;
-  msm_sort(ctx, st, tag, d_scalars, n, c, table != nullptr, so);
+  msm_sort(ctx, st, tag, d_scalars, n, c, table != nullptr,
+           msm_rounds(ctx, n, c, table != nullptr, FieldWords<F>::value == 16), so);
   so.done = nullptr;  // same stream: already ordered
   msm_accumulate<F>(ctx, st, tag, d_points, so, plan, st_reduce, table);
 }
 
 int msm_pair_rounds_entries(size_t max_entries, size_t nkeys, bool g2) {
-  return pair_rounds_model(max_entries, nkeys, g2);
+  return pair_rounds_model(0, max_entries, nkeys, g2, false);
 }
 
 int msm_pair_rounds(size_t n, bool g2) {
   if (n == 0) return 0;
   const int c = msm_pick_c(n, g2);
   const size_t W = 254 / c + 1;
-  return pair_rounds_model(n * W, W << (c - 1), g2);
+  return pair_rounds_model(n, n * W, W << (c - 1), g2, false);
 }
 
 int msm_pick_c_proof(size_t n, bool g2) {
@@ -1230,6 +1249,13 @@ void msm_init_kernels() {
   if (dev < 0 || dev >= kInitMaxDevices) throw Error(BG_E_ARG, "msm: device index out of range");
   std::call_once(once[dev], [] {
     BG_CUDA(cudaFuncSetAttribute(k_window_reduce<Fq>, cudaFuncAttributeMaxDynamicSharedMemorySize, 256 * 32 * 4));
+    auto smem = [](auto* k, size_t bytes) {
+      BG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    };
+    smem(k_pair_round<Fq, true>, pair_smem_bytes<Fq>());
+    smem(k_pair_round<Fq, false>, pair_smem_bytes<Fq>());
+    smem(k_pair_round<Fq2, true>, pair_smem_bytes<Fq2>());
+    smem(k_pair_round<Fq2, false>, pair_smem_bytes<Fq2>());
     BG_CUDA(cudaFuncSetAttribute(k_window_reduce_sm<Fq2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)reduce_sm_bytes<Fq2>(256)));
   });
@@ -1350,12 +1376,12 @@ void msm_g1_noalloc(const uint32_t* d_points, const uint32_t* d_scalars, size_t 
   k_digits_hist<<<ceil_div(n, 256), 256, 0, st>>>(d_scalars, n, c, W, nb, counts, status);
   BG_CHECK_LAUNCH();
   if (tiles == 1) {
-    k_scan_tile<<<1, kScanThreads, 0, st>>>(counts, offsets, nullptr, nkeys + 1);
+    k_scan_tile<<<1, kScanThreads, 0, st>>>(counts, offsets, nullptr, nkeys + 1, 0);
     BG_CHECK_LAUNCH();
   } else {
-    k_scan_tile<<<tiles, kScanThreads, 0, st>>>(counts, offsets, tile_sums, nkeys + 1);
+    k_scan_tile<<<tiles, kScanThreads, 0, st>>>(counts, offsets, tile_sums, nkeys + 1, 0);
     BG_CHECK_LAUNCH();
-    k_scan_tile<<<1, kScanThreads, 0, st>>>(tile_sums, tile_offs, nullptr, tiles);
+    k_scan_tile<<<1, kScanThreads, 0, st>>>(tile_sums, tile_offs, nullptr, tiles, 0);
     BG_CHECK_LAUNCH();
     k_scan_add<<<ceil_div(nkeys + 1, 256), 256, 0, st>>>(offsets, tile_offs, nkeys + 1);
     BG_CHECK_LAUNCH();

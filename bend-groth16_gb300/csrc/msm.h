@@ -26,6 +26,8 @@ struct MsmPlan {
   // on the accumulation stream, which it should finish under; a longer reduction by the latency
   // model is treated as critical (0 = no budget known: trust latency_critical)
   double hidden_us = 0;
+  // the accumulation has a stream to itself: its level buffers are not shared with other MSMs'
+  bool own_stream = false;
   // the host pool is otherwise idle when this reduction ends (not one of a small proof's
   // reductions that end together), so its part sums are priced as the pool runs them
   bool host_pool_free = false;
@@ -47,6 +49,7 @@ struct MsmSort {
   size_t n = 0;
   int c = 0, W = 0, sets = 0;
   uint32_t nb = 0;
+  int rounds = 0;  // pair rounds the buckets are padded for: to multiples of 2^rounds entries
   size_t nkeys = 0, max_entries = 0;
   uint32_t* offsets = nullptr;  // nkeys + 1 bucket offsets into sorted
   uint32_t* sorted = nullptr;   // entries: point index (+ w n for tables) | sign << 31
@@ -68,7 +71,7 @@ void msm_init_kernels();
 template <class F>
 void msm_build_table(cudaStream_t st, const uint32_t* d_points, size_t n, MsmTable& t, int c = 0);
 void exclusive_scan(Workspace& ws, const std::string& tag, const uint32_t* d_in, uint32_t* d_out, size_t n,
-                    cudaStream_t st, int depth);
+                    cudaStream_t st, int depth, uint32_t pad = 0);
 
 // Enqueue every device phase of one MSM on `st` (the window reduction on `st_reduce` when
 // given, after an event); scratch buffers are named by `tag` so that MSMs in flight at the
@@ -81,7 +84,10 @@ void msm_launch(Ctx& ctx, cudaStream_t st, const std::string& tag, const uint32_
 // The two halves of msm_launch: the sort on `st` (records so.done), and everything after it
 // on `st` (waits for so.done) with the fixup and reduction on `st_reduce`.
 void msm_sort(Ctx& ctx, cudaStream_t st, const std::string& tag, const uint32_t* d_scalars, size_t n, int c,
-              bool shared_set, MsmSort& out);
+              bool shared_set, int rounds, MsmSort& out);
+// Batch-affine pair rounds of an MSM of n points with c-bit windows (the context's override, else
+// the cost model); MSMs that share a sort take the most of theirs
+int msm_rounds(const Ctx& ctx, size_t n, int c, bool shared_set, bool g2);
 template <class F>
 void msm_accumulate(Ctx& ctx, cudaStream_t st, const std::string& tag, const uint32_t* d_points, const MsmSort& so,
                     MsmPlan& plan, cudaStream_t st_reduce = nullptr, const MsmTable* table = nullptr);

@@ -2,179 +2,201 @@
 //
 // The bucket phase of Msm.g1 / Msm.g2 (bend2/src/msm.bend:120-158 adds every point of a
 // window into its bucket with a Jacobian mixed addition) may be preceded by rounds that halve
-// every bucket: round r adds the points of each bucket in pairs, in affine coordinates, and
-// writes the sums (plus the odd point out) as the bucket's points for round r + 1.  The
-// additions of a round are independent, so they share their field inversions: each thread
-// multiplies its denominators into a running product, the CTA multiplies the threads'
-// products in a tree in shared memory, one thread inverts the root (binary Euclid,
-// inv_binary), and the tree and the running products are walked back to give every
-// addition 1 / d (Montgomery's simultaneous inversion).  An addition then costs 5 products
-// and a square (3 of them for the shared inversion) against madd-2008-s's 8 products and 2
-// squares; the XYZZ accumulation that follows adds what the rounds left, and the window
-// reduction is unchanged.
+// every bucket: a round adds the points of each bucket in pairs, in affine coordinates, and
+// writes the sums as the bucket's points for the next round.  The additions of a round are
+// independent, so they share their field inversions: each thread multiplies its denominators
+// into a running product, the CTA multiplies the threads' products in a tree in shared memory,
+// one thread inverts the root (binary Euclid, inv_binary), and the tree and the running products
+// are walked back to give every addition 1 / d (Montgomery's simultaneous inversion).  An
+// addition then costs 5 products and a square (3 of them for the shared inversion) against
+// madd-2008-s's 8 products and 2 squares; the XYZZ accumulation that follows adds what the
+// rounds left, and the window reduction is unchanged.
 //
-// Layout.  The entry list of the sort holds bucket b's m_b entries at [o_b, o_b + m_b).  After
-// L rounds bucket b holds ceil(m_b / 2^L) points starting at
-//     start_L(b) = floor((o_b + (2^(L+1) - 2) b) / 2^L),
-// a closed form of the sort's offsets (start_{L+1}(b) = floor(start_L(b) / 2) + b), so no
-// round needs a scan.  A bucket's region [start_L(b), start_L(b + 1)) is at least its point
-// count (start_{L+1}(b) + ceil(m / 2) <= floor(start_L(b + 1) / 2) + b + 1 because
-// start_L(b + 1) >= start_L(b) + m), every region of a level L >= 1 has at least one slot, and
-// the slots past the points -- at most two per bucket after a few rounds -- hold the affine
-// infinity (0, 0), so the XYZZ accumulation reads level L's regions as ordinary buckets with
-// start_L as their offsets.
+// Layout.  The sort pads every bucket to a multiple of 2^L entries (L its number of rounds) with
+// null entries, so pair j of a round is the level's points 2 j and 2 j + 1, always of one bucket:
+// no round looks a bucket up, levels r >= 1 are read and written in order, and level r's bucket
+// offsets are the sort's shifted right by r.  Round 0 reads its points through the sort's entries
+// (index | sign << 31) from the MSM's point set or window table.  A missing point (a null entry,
+// a sum at infinity) is (0, 0) on every level, as an input at infinity is.
 //
-// Round r writes every position j of level r + 1: j in bucket b at index i = j - start_{r+1}(b)
-// is the sum of level-r points 2i and 2i + 1 when both exist, point 2i when only it does, and
-// infinity otherwise.  Round 0 reads its points through the sort's entries (index | sign << 31)
-// from the MSM's point set or window table; later rounds read the previous level directly.
+// Positions are dealt to the threads of a CTA in turn, so that neighbouring lanes read
+// neighbouring entries, and every operand is staged in shared memory by cp.async a few positions
+// ahead: the gathers of round 0 are 32 and 64-byte accesses all over the point set.
 
-// start_L(b) for the sort's offset o = o_b; b = nkeys gives the level's size
-__host__ __device__ inline uint64_t level_start(uint32_t o, uint64_t b, int level) {
-  return ((uint64_t)o + (((uint64_t)2 << level) - 2) * b) >> level;
-}
-// ceil(m / 2^L): points of a bucket of m entries after L rounds
-__host__ __device__ inline uint32_t level_count(uint32_t m, int level) {
-  return (uint32_t)(((uint64_t)m + (1ull << level) - 1) >> level);
-}
+// a null entry of a padded bucket
+constexpr uint32_t kNullEntry = 0xffffffffu;
 
-// CTA size (the batch of one shared inversion is CTA size x positions per thread); two CTAs per
-// SM (G1: 124 registers, G2: 228)
+// CTA size; four CTAs per SM in G1 (118 registers; five at 96 registers measured 1.57 -> 1.95 ms for
+// G1 MSM 2^20's two rounds), two in G2
 template <class F>
-constexpr int kPairThreads = FieldWords<F>::value == 8 ? 256 : 128;
+constexpr int kPairThreads = 128;
+// stages of the operand rings (power of two): x coordinates ahead in the forward pass, whole
+// points and a running product in the backward pass
+constexpr int kPairFwd = 4;
+constexpr int kPairBwd = 2;
 
-// Input point k of a round: round 0 reads it through the sort's entry (index | sign << 31) from
-// the MSM's point set or window table, later rounds read the previous level directly.  The
-// entry code is loaded apart from the point so that it can be fetched a position ahead.
-template <bool kFirst>
-BG_DEV uint32_t pair_code(const uint32_t* __restrict__ sorted, uint64_t k) {
-  if constexpr (kFirst) return sorted[k];
-  else return (uint32_t)k;
-}
-template <class F, bool kFirst>
-BG_DEV Affine<F> pair_point(const uint32_t* __restrict__ src, uint32_t code) {
-  constexpr int FW = FieldWords<F>::value;
-  const Affine<F> a = load_affine<F>(src + (size_t)(code & 0x7fffffffu) * 2 * FW);
-  return (kFirst && (code >> 31)) ? affine_neg(a) : a;
+// 16-byte chunks per field element
+template <class F>
+constexpr int kPairCh = FieldWords<F>::value / 4;
+// shared memory: the ring (the larger pass's), under which the product tree lies between the passes
+template <class F>
+constexpr size_t pair_ring_chunks() {
+  constexpr int fwd = kPairFwd * 2 * kPairCh<F>, bwd = kPairBwd * 5 * kPairCh<F>;
+  return (size_t)(fwd > bwd ? fwd : bwd) * kPairThreads<F>;
 }
 template <class F>
-BG_DEV F pair_x(const uint32_t* __restrict__ src, uint32_t code) {
-  constexpr int FW = FieldWords<F>::value;
-  F x;
-  load_elem(x, src + (size_t)(code & 0x7fffffffu) * 2 * FW);
-  return x;
+constexpr size_t pair_smem_bytes() {
+  const size_t tree = 2 * (size_t)kPairThreads<F> * FieldWords<F>::value * 4;
+  return pair_ring_chunks<F>() * 16 > tree ? pair_ring_chunks<F>() * 16 : tree;
 }
 
-// A bucket of the output level: its output region [out_lo, out_hi), its input points at
-// [in_lo, in_lo + m_in).
-struct PairBucket {
-  uint32_t b;
-  uint64_t out_lo, out_hi, in_lo;
-  uint32_t m_in;
-};
-BG_DEV void pair_bucket_set(PairBucket& k, const uint32_t* __restrict__ offsets, uint32_t b, int level) {
-  const uint32_t o0 = offsets[b], o1 = offsets[b + 1];
-  k.b = b;
-  k.out_lo = level_start(o0, b, level + 1);
-  k.out_hi = level_start(o1, (uint64_t)b + 1, level + 1);
-  k.in_lo = level_start(o0, b, level);
-  k.m_in = level_count(o1 - o0, level);
+BG_DEV Fq select(bool c, const Fq& a, const Fq& b) {
+  Fq r;
+#pragma unroll
+  for (int i = 0; i < 8; i++) r.v[i] = c ? a.v[i] : b.v[i];
+  return r;
 }
-
-// What output position j of a round reads: the input pair (in, in + 1), the single input in
-// (the odd point of a bucket), or nothing (a slot past the bucket's points: infinity).  The
-// bucket cursor k moves forward or backward to the bucket holding j.
-enum : uint32_t { kSrcPair = 0, kSrcCopy = 1, kSrcNone = 2 };
-template <bool kForward>
-BG_DEV uint32_t pair_source(PairBucket& k, const uint32_t* __restrict__ offsets, uint64_t j, int level,
-                            uint64_t& in) {
-  if (kForward) {
-    while (j >= k.out_hi) pair_bucket_set(k, offsets, k.b + 1, level);
+BG_DEV Fq2 select(bool c, const Fq2& a, const Fq2& b) { return {select(c, a.c0, b.c0), select(c, a.c1, b.c1)}; }
+template <class F>
+BG_DEV F elem_of_chunks(const uint4* c, int stride) {
+  if constexpr (FieldWords<F>::value == 16) {
+    return {fp_of(c[0], c[stride]), fp_of(c[2 * stride], c[3 * stride])};
   } else {
-    while (j < k.out_lo) pair_bucket_set(k, offsets, k.b - 1, level);
+    return fp_of(c[0], c[stride]);
   }
-  const uint64_t i = j - k.out_lo;
-  in = k.in_lo + 2 * i;
-  return 2 * i + 1 < k.m_in ? kSrcPair : (2 * i < k.m_in ? kSrcCopy : kSrcNone);
+}
+// 16 bytes global -> shared, or zeros
+BG_DEV void cp_async16_or_zero(void* smem, const void* gmem, bool take) {
+  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
+  const int bytes = take ? 16 : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
+}
+template <int N>
+BG_DEV void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// One round: input level `level` (src), output level + 1 (dst), `per_thread` consecutive output
-// positions per thread.  dst's x field of each position first holds the running product of the
-// thread's denominators up to it (read back by the backward pass) and is then overwritten by
-// the sum.  Round 0 also writes the offsets of level `final_level` (the accumulation's).
+// a - b as some representative below 2^256 (a, b < p): for the second factor of a product
+BG_DEV Fq sub_loose(const Fq& a, const Fq& b) {
+  Fq r;
+  asm("add.cc.u32  %0, %8,  %16;\n\t"
+      "addc.cc.u32 %1, %9,  %17;\n\t"
+      "addc.cc.u32 %2, %10, %18;\n\t"
+      "addc.cc.u32 %3, %11, %19;\n\t"
+      "addc.cc.u32 %4, %12, %20;\n\t"
+      "addc.cc.u32 %5, %13, %21;\n\t"
+      "addc.cc.u32 %6, %14, %22;\n\t"
+      "addc.u32    %7, %15, %23;"
+      : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]), "=r"(r.v[7])
+      : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7]),
+        "n"(FqParams::P0), "n"(FqParams::P1), "n"(FqParams::P2), "n"(FqParams::P3), "n"(FqParams::P4),
+        "n"(FqParams::P5), "n"(FqParams::P6), "n"(FqParams::P7));
+  asm("sub.cc.u32  %0, %0, %8;\n\t"
+      "subc.cc.u32 %1, %1, %9;\n\t"
+      "subc.cc.u32 %2, %2, %10;\n\t"
+      "subc.cc.u32 %3, %3, %11;\n\t"
+      "subc.cc.u32 %4, %4, %12;\n\t"
+      "subc.cc.u32 %5, %5, %13;\n\t"
+      "subc.cc.u32 %6, %6, %14;\n\t"
+      "subc.u32    %7, %7, %15;"
+      : "+r"(r.v[0]), "+r"(r.v[1]), "+r"(r.v[2]), "+r"(r.v[3]), "+r"(r.v[4]), "+r"(r.v[5]), "+r"(r.v[6]), "+r"(r.v[7])
+      : "r"(b.v[0]), "r"(b.v[1]), "r"(b.v[2]), "r"(b.v[3]), "r"(b.v[4]), "r"(b.v[5]), "r"(b.v[6]), "r"(b.v[7]));
+  return r;
+}
+// (an Fq2 product adds its factors' halves, which leaves no room)
+BG_DEV Fq2 sub_loose(const Fq2& a, const Fq2& b) { return sub(a, b); }
+
+// One round: `per_thread` positions per thread.  dst's x field of each position first holds the
+// thread's running product up to it (read back by the backward pass) and is then overwritten by
+// the sum.  Round 0 also writes the offsets of the accumulation's level, offsets >> rounds.
 template <class F, bool kFirst>
-__global__ void __launch_bounds__(kPairThreads<F>, 2)
+__global__ void __launch_bounds__(kPairThreads<F>, FieldWords<F>::value == 8 ? 4 : 2)
     k_pair_round(const uint32_t* __restrict__ src, const uint32_t* __restrict__ sorted,
                  const uint32_t* __restrict__ offsets, uint32_t nkeys, int level, uint32_t per_thread,
-                 uint32_t* __restrict__ dst, int final_level, uint32_t* __restrict__ final_offsets) {
+                 uint32_t* __restrict__ dst, int rounds, uint32_t* __restrict__ final_offsets) {
   constexpr int FW = FieldWords<F>::value;
   constexpr int PW = 2 * FW;
   constexpr int NT = kPairThreads<F>;
-  __shared__ __align__(16) uint32_t tree[2 * NT * FW];
+  constexpr int CH = kPairCh<F>;
+  constexpr int FD = kPairFwd;
+  extern __shared__ __align__(16) uint32_t sm[];
+  uint4* const ring = reinterpret_cast<uint4*>(sm) + threadIdx.x;  // chunk c of a stage at ring[c * NT]
+  uint32_t* const tree = sm;
   const uint32_t tid = threadIdx.x;
   if (final_offsets) {
     for (size_t g = (size_t)blockIdx.x * NT + tid; g <= nkeys; g += (size_t)gridDim.x * NT)
-      final_offsets[g] = (uint32_t)level_start(offsets[g], g, final_level);
+      final_offsets[g] = offsets[g] >> rounds;
   }
-  const uint64_t total = level_start(offsets[nkeys], nkeys, level + 1);
-  const uint64_t beg = ((uint64_t)blockIdx.x * NT + tid) * per_thread;
-  const uint32_t cnt = beg >= total ? 0u : (total - beg < per_thread ? (uint32_t)(total - beg) : per_thread);
+  const uint32_t total = offsets[nkeys] >> (level + 1);
+  const uint64_t base = (uint64_t)blockIdx.x * NT * per_thread + tid;
+  if ((uint64_t)blockIdx.x * NT * per_thread >= total) return;
+  // positions base, base + NT, ... below total
+  const uint32_t cnt =
+      base >= total ? 0u : (uint32_t)min((uint64_t)per_thread, (total - base + NT - 1) / (uint64_t)NT);
 
-  // ---- forward: classify each position, multiply the denominators into acc
+  auto entries = [&](uint32_t t) -> uint2 {
+    if constexpr (kFirst) return *reinterpret_cast<const uint2*>(sorted + 2 * (base + (uint64_t)t * NT));
+    else return make_uint2(0u, 0u);
+  };
+  auto stage_elem = [&](uint4* slot, const uint32_t* g, bool take) {
+#pragma unroll
+    for (int c = 0; c < CH; c++) cp_async16_or_zero(slot + c * NT, g + 4 * c, take);
+  };
+  // address of input point `k` (0 or 1) of position t
+  auto point = [&](uint32_t t, uint2 e, int k) -> const uint32_t* {
+    if constexpr (kFirst) {
+      const uint32_t c = k ? e.y : e.x;
+      return src + (size_t)(c == kNullEntry ? 0u : c & 0x7fffffffu) * PW;
+    } else {
+      return src + (2 * (size_t)(base + (uint64_t)t * NT) + k) * PW;
+    }
+  };
+
+  // ---- forward: the running product of the denominators x_Q - x_P (1 where there is no addition)
   F acc = field_one<F>();
-  PairBucket k{};
-  if (cnt) {
-    uint32_t lo = 0, hi = nkeys;  // start_{level+1}(lo) <= beg < start_{level+1}(hi)
-    while (hi - lo > 1) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (level_start(offsets[mid], mid, level + 1) <= beg) lo = mid;
-      else hi = mid;
-    }
-    pair_bucket_set(k, offsets, lo, level);
-    // The denominator of a pair is x_Q - x_P unless the x coordinates agree or one is zero (a
-    // point at infinity, or a rare point with x = 0): only then are the full points read.  The
-    // next pair's entry codes and x coordinates are fetched during this pair's product.
-    uint64_t in_n;
-    uint32_t src_n = pair_source<true>(k, offsets, beg, level, in_n);
-    uint32_t cp_n = 0, cq_n = 0;
-    F xp_n = field_zero<F>(), xq_n = field_zero<F>();
-    if (src_n == kSrcPair) {
-      cp_n = pair_code<kFirst>(sorted, in_n);
-      cq_n = pair_code<kFirst>(sorted, in_n + 1);
-      xp_n = pair_x<F>(src, cp_n);
-      xq_n = pair_x<F>(src, cq_n);
-    }
+  {
+    auto stage = [&](uint32_t t, uint2 e) {
+      if (t < cnt) {
+        uint4* s = ring + (size_t)(t & (FD - 1)) * 2 * CH * NT;
+        stage_elem(s, point(t, e, 0), !kFirst || e.x != kNullEntry);
+        stage_elem(s + CH * NT, point(t, e, 1), !kFirst || e.y != kNullEntry);
+      }
+      cp_async_commit();
+    };
+#pragma unroll
+    for (int t = 0; t < FD - 1; t++) stage(t, (uint32_t)t < cnt ? entries(t) : make_uint2(0u, 0u));
+    uint2 e = FD - 1 < cnt ? entries(FD - 1) : make_uint2(0u, 0u);
     for (uint32_t t = 0; t < cnt; t++) {
-      const uint64_t j = beg + t;
-      const uint32_t kind_src = src_n, cp = cp_n, cq = cq_n;
-      const F xp = xp_n, xq = xq_n;
-      if (t + 1 < cnt) {
-        src_n = pair_source<true>(k, offsets, j + 1, level, in_n);
-        if (src_n == kSrcPair) {
-          cp_n = pair_code<kFirst>(sorted, in_n);
-          cq_n = pair_code<kFirst>(sorted, in_n + 1);
-          xp_n = pair_x<F>(src, cp_n);
-          xq_n = pair_x<F>(src, cq_n);
-        }
+      stage(t + FD - 1, e);
+      if (t + FD < cnt) e = entries(t + FD);
+      cp_async_wait<FD - 1>();
+      const uint4* s = ring + (size_t)(t & (FD - 1)) * 2 * CH * NT;
+      const F xp = elem_of_chunks<F>(s, NT), xq = elem_of_chunks<F>(s + CH * NT, NT);
+      // A missing point has x = 0 and gives the other's +-x, as good a factor as any: the backward
+      // pass takes it out again.  Only a zero needs care: equal x or two missing points.
+      F d = sub(xq, xp);
+      if (is_zero(d)) {
+        const uint2 en = entries(t);
+        F yp = field_zero<F>(), yq = field_zero<F>();
+        if (!kFirst || en.x != kNullEntry) load_elem(yp, point(t, en, 0) + FW);
+        if (!kFirst || en.y != kNullEntry) load_elem(yq, point(t, en, 1) + FW);
+        if (kFirst && (en.x >> 31)) yp = neg(yp);
+        if (kFirst && (en.y >> 31)) yq = neg(yq);
+        d = eq(yp, yq) && !is_zero(yp) ? dbl(yp) : field_one<F>();  // the tangent's, or no addition
       }
-      if (kind_src == kSrcPair) {
-        F d = sub(xq, xp);
-        bool inverted = true;
-        if (is_zero(d) || is_zero(xp) || is_zero(xq)) {
-          const Affine<F> p = pair_point<F, kFirst>(src, cp), q = pair_point<F, kFirst>(src, cq);
-          inverted = pair_kind(p, q, d) <= kPairTangent;
-        }
-        if (inverted) acc = imul(acc, d);
-      }
-      store_elem(dst + j * PW, acc);
+      acc = imul(acc, d);
+      store_elem(dst + (base + (uint64_t)t * NT) * PW, acc);
     }
+    cp_async_wait<0>();
   }
 
-  // ---- the CTA's product tree (leaves NT..2NT-1, node i = node 2i * node 2i+1), one
-  // inversion of the root, and the tree walked back: leaf t ends as 1 / (thread t's product)
+  // ---- the CTA's product tree (leaves NT..2NT-1, node i = node 2i * node 2i+1) up to the 32
+  // nodes of one level, which a warp inverts side by side, and the tree walked back: leaf t ends
+  // as 1 / (thread t's product)
+  __syncthreads();
   store_elem(tree + (size_t)(NT + tid) * FW, acc);
   __syncthreads();
-  for (uint32_t half = NT / 2; half >= 1; half >>= 1) {
+  for (uint32_t half = NT / 2; half >= 32; half >>= 1) {
     if (tid < half) {
       const uint32_t i = half + tid;
       F a, b;
@@ -184,13 +206,13 @@ __global__ void __launch_bounds__(kPairThreads<F>, 2)
     }
     __syncthreads();
   }
-  if (tid == 0) {
+  if (tid < 32) {
     F root;
-    load_elem(root, tree + FW);
-    store_elem(tree + FW, field_inv_fast(root));
+    load_elem(root, tree + (size_t)(32 + tid) * FW);
+    store_elem(tree + (size_t)(32 + tid) * FW, field_inv_fast(root));
   }
   __syncthreads();
-  for (uint32_t half = 1; half < NT; half <<= 1) {
+  for (uint32_t half = 32; half < NT; half <<= 1) {
     if (tid < half) {
       const uint32_t i = half + tid;
       F iv, a, b;
@@ -202,63 +224,89 @@ __global__ void __launch_bounds__(kPairThreads<F>, 2)
     }
     __syncthreads();
   }
-  if (!cnt) return;
   F inv;
   load_elem(inv, tree + (size_t)(NT + tid) * FW);
+  __syncthreads();
+  if (!cnt) return;
 
-  // ---- backward: 1 / d_t = inv * (product up to t - 1), inv *= d_t, and the sums; the next
-  // position's entry codes are fetched a position ahead
-  uint64_t in_n;
-  uint32_t src_n = pair_source<false>(k, offsets, beg + cnt - 1, level, in_n);
-  uint32_t cp_n = 0, cq_n = 0;
-  if (src_n != kSrcNone) cp_n = pair_code<kFirst>(sorted, in_n);
-  if (src_n == kSrcPair) cq_n = pair_code<kFirst>(sorted, in_n + 1);
-  for (uint32_t t = cnt; t-- > 0;) {
-    const uint64_t j = beg + t;
-    const uint32_t kind_src = src_n, cp = cp_n, cq = cq_n;
-    if (t > 0) {
-      src_n = pair_source<false>(k, offsets, j - 1, level, in_n);
-      if (src_n != kSrcNone) cp_n = pair_code<kFirst>(sorted, in_n);
-      if (src_n == kSrcPair) cq_n = pair_code<kFirst>(sorted, in_n + 1);
+  // ---- backward: 1 / d_t = inv * (product up to t - 1), inv *= d_t, and the sums.  A slot holds
+  // x_P, y_P, x_Q, y_Q and the product before the position.
+  auto stage = [&](int64_t t, uint2 e) {
+    if (t >= 0) {
+      uint4* s = ring + (size_t)(t & (kPairBwd - 1)) * 5 * CH * NT;
+      const uint32_t *p = point((uint32_t)t, e, 0), *q = point((uint32_t)t, e, 1);
+      const bool tp = !kFirst || e.x != kNullEntry, tq = !kFirst || e.y != kNullEntry;
+      stage_elem(s, p, tp);
+      stage_elem(s + CH * NT, p + FW, tp);
+      stage_elem(s + 2 * CH * NT, q, tq);
+      stage_elem(s + 3 * CH * NT, q + FW, tq);
+      if (t > 0) stage_elem(s + 4 * CH * NT, dst + (base + (uint64_t)(t - 1) * NT) * PW, true);
     }
-    Affine<F> r;
-    if (kind_src == kSrcPair) {
-      const Affine<F> p = pair_point<F, kFirst>(src, cp), q = pair_point<F, kFirst>(src, cq);
-      F d = field_zero<F>(), dinv = field_zero<F>();
-      const uint32_t kind = pair_kind(p, q, d);
-      if (kind <= kPairTangent) {
-        if (t > 0) {
-          F prev;
-          load_elem(prev, dst + (j - 1) * PW);
-          dinv = imul(inv, prev);
-        } else {
-          dinv = inv;
-        }
-        inv = imul(inv, d);
+    cp_async_commit();
+  };
+  uint2 e = entries(cnt - 1), e_n = cnt > 1 ? entries(cnt - 2) : make_uint2(0u, 0u);
+  stage((int64_t)cnt - 1, e);
+  for (uint32_t t = cnt; t-- > 0;) {
+    const uint2 ec = e;
+    stage((int64_t)t - 1, e_n);
+    e = e_n;
+    if (t > 1) e_n = entries(t - 2);
+    cp_async_wait<1>();
+    const uint64_t j = base + (uint64_t)t * NT;
+    const uint4* s = ring + (size_t)(t & (kPairBwd - 1)) * 5 * CH * NT;
+    Affine<F> p, q;
+    p.x = elem_of_chunks<F>(s, NT);
+    q.x = elem_of_chunks<F>(s + 2 * CH * NT, NT);
+    p.y = elem_of_chunks<F>(s + CH * NT, NT);
+    q.y = elem_of_chunks<F>(s + 3 * CH * NT, NT);
+    const bool mp = is_inf(p), mq = is_inf(q);
+    if constexpr (kFirst) {
+      p.y = select(ec.x >> 31, neg(p.y), p.y);
+      q.y = select(ec.y >> 31, neg(q.y), q.y);
+    }
+    F d = sub(q.x, p.x), num = sub_loose(q.y, p.y);
+    bool none = mp && mq;  // no sum, or a sum at infinity
+    if (is_zero(d)) {
+      if (!none && eq(p.y, q.y) && !is_zero(p.y)) {
+        d = dbl(p.y);
+        const F x2 = fsqr(p.x);
+        num = add(dbl(x2), x2);
+      } else {
+        d = field_one<F>();
+        none = none || (!mp && !mq);
       }
-      r = pair_finish(p, q, kind, dinv);
-    } else if (kind_src == kSrcCopy) {
-      r = pair_point<F, kFirst>(src, cp);
-    } else {
-      r.x = field_zero<F>();
-      r.y = field_zero<F>();
+    }
+    F dinv = inv;
+    if (t > 0) dinv = imul(inv, elem_of_chunks<F>(s + 4 * CH * NT, NT));
+    inv = imul(inv, d);
+    const F l = imul(dinv, num);
+    Affine<F> r;
+    r.x = sub(sub(isqr(l), p.x), q.x);  // the tangent case has q.x = p.x
+    r.y = sub(imul(l, sub_loose(p.x, r.x)), p.y);
+    if (mp || mq || none) {
+      r = mp ? q : p;
+      if (none) {
+        r.x = field_zero<F>();
+        r.y = field_zero<F>();
+      }
     }
     store_affine(dst + j * PW, r);
   }
 }
 
-// Rounds before the XYZZ accumulation.  Measured on GB300 (G1 MSM 2^20 with one bucket set per
-// window, 17.8 M entries, 64 per bucket): a pair round costs 0.90 of the mixed additions it
-// replaces (the pair kernel issues 76% of their instructions but loses more of its cycles to
-// gathers and to the CTA's inversion: issue active 50% against 60%), and fewer entries per
-// bucket make the window reduction cheaper: two rounds take the MSM from 5.13 to 4.90 ms, more
-// rounds cost more than they save.  G2 pair rounds measured 0.95 of the mixed additions and
-// slower MSMs (G2 MSM 2^18: 5.32 ms without, 5.44 / 5.69 ms with one / two rounds), and proofs
-// over window tables (one bucket set, 3.9 M entries per SquareChain(2^18) G1 MSM, reductions
-// hidden under later accumulations) measured slower with any rounds (10.45 -> 10.73 ms with
-// one), so the model takes two rounds for large G1 MSMs only (SquareChain(2^20) proof, whose G1
-// table MSMs have 14.7 M entries: 36.85 -> 36.19 ms).
-inline int pair_rounds_model(size_t max_entries, size_t nkeys, bool g2) {
+// Rounds before the XYZZ accumulation.  A pair addition costs 3056 cycles of the multiply pipe per
+// warp against madd-2008-s's 4784 and about 1500 instructions against 2120; a round adds its share
+// of an inversion, a launch, and the gathers twice.  Measured on GB300, two rounds against none: G1
+// MSM 2^20 (17.8 M entries, 64 per bucket) 2.42 ms of mixed additions -> 1.57 + 0.65 ms, the MSM
+// 3.49 -> 3.19 ms (one round 3.33, three 3.3); SquareChain(2^20) 23.2 -> 20.75 ms, 2^19 12.2 ->
+// 11.15 ms, 16 mixed proofs in a batch 17.2 -> 16.5 ms; SquareChain(2^18) level (6.65-6.77 ms either
+// way), with tables of 2 M entries too 2^17 and the batch 2% slower.  Window tables of 2^18 points
+// and up, whose levels fit the scratch a proof reserves (SquareChain(2^17)'s msm_h, 262143 points,
+// would need 3% more).  The bucket sets of standalone MSMs hold fewer entries per bucket
+// (G2 MSM 2^18: 17) and their accumulation is not what its reduction waits behind, so only the
+// largest G1 ones take rounds.
+inline int pair_rounds_model(size_t n, size_t max_entries, size_t nkeys, bool g2, bool shared_set) {
+  if (shared_set) return n >= (size_t(1) << 18) && max_entries >= 3000000 && max_entries >= 24 * nkeys ? 2 : 0;
   if (g2 || max_entries < (size_t(1) << 23) || max_entries < 32 * nkeys) return 0;
   return 2;
 }

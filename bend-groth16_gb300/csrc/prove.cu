@@ -476,7 +476,11 @@ void prove_resident(Ctx& ctx, PkDev& pk, const uint32_t* witness16, const uint32
     for (auto& e : sorts)
       if (e.first.sc == k.sc && e.first.n == k.n && e.first.c == k.c && e.first.shared == k.shared) return e.second;
     sorts.emplace_back(k, MsmSort());
-    msm_sort(ctx, s, std::string(jb.tag) + ".sort", jb.sc, jb.n, k.c, k.shared, sorts.back().second);
+    int rounds = 0;
+    for (const Job& o : jobs)
+      if (o.sc == k.sc && o.n == k.n && width(o) == k.c && (o.tab != nullptr) == k.shared)
+        rounds = std::max(rounds, msm_rounds(ctx, o.n, k.c, k.shared, o.g2));
+    msm_sort(ctx, s, std::string(jb.tag) + ".sort", jb.sc, jb.n, k.c, k.shared, rounds, sorts.back().second);
     return sorts.back().second;
   };
   BG_CUDA(cudaStreamWaitEvent(acc_st, ev_scalars, 0));
@@ -497,6 +501,7 @@ void prove_resident(Ctx& ctx, PkDev& pk, const uint32_t* witness16, const uint32
     // others get the accumulation time queued after them (entries x about 0.3 ns for G1 and
     // 0.9 ns for G2 inside a proof), which the reduction should not outlast.
     p.latency_critical = overlap || j == 4;
+    p.own_stream = overlap;
     p.host_pool_free = !overlap && !ctx.shared_gpu;
     // (Batch and server lanes keep the fixed rule: other proofs fill the GPU there.)
     p.hidden_us = 0;
