@@ -412,7 +412,7 @@ int bg_qap_h(bg_ctx* ctx, const uint32_t* a16, const uint32_t* b16, const uint32
     if (log2d == 0) {
       // d = 1: h = (a b - c) / (g - 1) on the one-point coset; handled by the general path
     }
-    qap_h_run(c, c.stream, a, b, cc, h, (int)log2d);
+    qap_h_run(c, c.stream, a, b, cc, h, (int)log2d, false);
     stage_out(c, "api.qh", h, h16, d);
     check_status(c, c.stream);
   });

@@ -131,6 +131,7 @@ struct NttTables {
   uint32_t* g_hi = nullptr;        // g^(i 2^a)
   uint32_t* g_hi_ninv = nullptr;   // n^-1 g^(i 2^a)
   uint32_t* gi_hi_ninv = nullptr;  // n^-1 g^(-i 2^a)
+  uint32_t* gi_hi_ninv_canon = nullptr;  // the same, canonical: times a Montgomery x, a canonical product
   uint32_t* ninv = nullptr;        // n^-1
   uint32_t* zinv = nullptr;        // (g^n - 1)^-1
 };

@@ -321,10 +321,11 @@ BG_DEV void mul_row(uint32_t* e, uint32_t* o, const uint32_t* a, uint32_t b) {
   redc_row<P>(e, o);
 }
 
-// a b R^-1 mod p for a < p and any 256-bit b, product and reduction interleaved row by row (the
-// two accumulators take 16 registers instead of a 16-limb product's 31)
+// a b R^-1 mod p, below p + a b / R, for a < p and any 256-bit b (below 2p for b < 5p): product and
+// reduction interleaved row by row (the two accumulators take 16 registers instead of a 16-limb
+// product's 31)
 template <class P>
-BG_DEV Fp<P> mul(const Fp<P>& a, const Fp<P>& b) {
+BG_DEV Fp<P> mul_loose(const Fp<P>& a, const Fp<P>& b) {
   uint32_t u[8], w[8];
 #pragma unroll
   for (int j = 0; j < 4; j++) {
@@ -339,10 +340,16 @@ BG_DEV Fp<P> mul(const Fp<P>& a, const Fp<P>& b) {
   mul_row<P>(w, u, a.v, b.v[5]);
   mul_row<P>(u, w, a.v, b.v[6]);
   mul_row<P>(w, u, a.v, b.v[7]);
-  uint32_t t[8];
-  join_rows(t, w, u);
   Fp<P> r;
-  reduce_once<P>(r.v, t);
+  join_rows(r.v, w, u);
+  return r;
+}
+// the same, fully reduced
+template <class P>
+BG_DEV Fp<P> mul(const Fp<P>& a, const Fp<P>& b) {
+  const Fp<P> t = mul_loose(a, b);
+  Fp<P> r;
+  reduce_once<P>(r.v, t.v);
   return r;
 }
 

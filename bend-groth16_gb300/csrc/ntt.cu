@@ -8,15 +8,14 @@
 // chunk tree with running-product twiddles (ntt.bend:1-18).
 //
 // Here a transform is a few passes over HBM/L2; each pass loads a tile of up to 1024
-// elements into shared memory (limb-major, so a warp's 32 butterflies hit 32 banks), runs up
+// elements into shared memory, runs up
 // to 10 radix-2 stages there with twiddles from a resident table, and writes the tile back.
-// 1024-element tiles (32 KiB) give a 2^19 transform 512 CTAs instead of 256 with 64 KiB
-// tiles: measured 2^19 0.219 -> 0.210 ms, 2^20 0.407 -> 0.360 ms.
+// 1024-element tiles (32 KiB) give a 2^19 transform 512 CTAs instead of 256 with 64 KiB tiles.
 //   DIF (Gentleman-Sande): natural order in -> bit-reversed out (used for inverse transforms)
 //   DIT (Cooley-Tukey):    bit-reversed in -> natural order out (forward transforms)
 // so iNTT followed by a coset NTT needs no permutation: the coset factor g^j of coefficient j
-// is applied in bit-reversed position, fused with n^-1 into the last DIF pass.  Only the final
-// h needs one bit-reversal gather.
+// is applied in bit-reversed position, fused with n^-1 into the last DIF pass.  A transform that has
+// to end in natural order writes its last pass to the bit-reversed places of another buffer.
 #include <mutex>
 
 #include "common.cuh"
@@ -29,6 +28,10 @@ namespace bg {
 constexpr int kNttThreads = 256;
 constexpr int kNttTile = 1024;   // elements per CTA tile (32 KiB of shared memory)
 constexpr int kContigMax = 10;   // stages in one pass, contiguous or strided (a 1024-element tile)
+
+// 2r
+static constexpr uint32_t kTwoR[8] = {0xe0000002u, 0x87c3eb27u, 0xf372e122u, 0x5067d090u,
+                                      0x0302b0bau, 0x70a08b6du, 0xc2634053u, 0x60c89ce5u};
 
 enum ScaleMode { SC_NONE = 0, SC_NATURAL = 1, SC_BITREV = 2, SC_CONST = 3 };
 
@@ -48,10 +51,7 @@ BG_DEV Fr scale_factor(int mode, size_t j, int L, const ScaleTab& t) {
 }
 
 // The tile in shared memory: element e's low and high 16 bytes at uint4 slot e of two arrays
-// of E slots, so an element moves in two 128-bit accesses.  The pass is bound by instruction
-// issue, and a limb-major tile took eight 32-bit accesses per element for the same wavefronts:
-// 2^20 forward transform 0.362 -> 0.333 ms (76 registers, 3 CTAs per SM; forcing 4 CTAs per SM
-// at 64 registers spills and measured the same 0.332 ms).
+// of E slots, so an element moves in two 128-bit accesses.
 BG_DEV void tile_store(uint32_t* sm, int E, int e, const Fr& x) {
   uint4* lo = reinterpret_cast<uint4*>(sm);
   lo[e] = make_uint4(x.v[0], x.v[1], x.v[2], x.v[3]);
@@ -66,24 +66,124 @@ BG_DEV Fr tile_load(const uint32_t* sm, int E, int e) {
   return x;
 }
 
-// One pass: stages [s0, s0 + k) of a size-2^L transform.  A CTA owns G independent groups of
-// 2^k elements; group element t of group (hi, lo) sits at hi*2^(s0+k) + t*2^s0 + lo.
+// Values inside a pass are kept loosely reduced (after Harvey, "Faster arithmetic for
+// number-theoretic transforms", 2014): below 2r between DIF stages, below 4r between DIT ones, and
+// only stores to memory reduce fully.  A twiddle product takes any factor below 5r and returns
+// one below 2r without its final subtraction (mul_loose), a difference adds 2r instead of
+// testing its sign: a butterfly is 26 instructions of 313 shorter.
+BG_DEV Fr add_raw(const Fr& a, const Fr& b) {
+  Fr r;
+  raw_add8(r.v, a.v, b.v);
+  return r;
+}
+// a - b + 2r
+BG_DEV Fr sub_plus2(const Fr& a, const Fr& b) {
+  Fr t;
+  asm("add.cc.u32  %0, %8,  %16;\n\t"
+      "addc.cc.u32 %1, %9,  %17;\n\t"
+      "addc.cc.u32 %2, %10, %18;\n\t"
+      "addc.cc.u32 %3, %11, %19;\n\t"
+      "addc.cc.u32 %4, %12, %20;\n\t"
+      "addc.cc.u32 %5, %13, %21;\n\t"
+      "addc.cc.u32 %6, %14, %22;\n\t"
+      "addc.u32    %7, %15, %23;"
+      : "=r"(t.v[0]), "=r"(t.v[1]), "=r"(t.v[2]), "=r"(t.v[3]), "=r"(t.v[4]), "=r"(t.v[5]), "=r"(t.v[6]), "=r"(t.v[7])
+      : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7]),
+        "n"(kTwoR[0]), "n"(kTwoR[1]), "n"(kTwoR[2]), "n"(kTwoR[3]), "n"(kTwoR[4]), "n"(kTwoR[5]), "n"(kTwoR[6]),
+        "n"(kTwoR[7]));
+  asm("sub.cc.u32  %0, %0, %8;\n\t"
+      "subc.cc.u32 %1, %1, %9;\n\t"
+      "subc.cc.u32 %2, %2, %10;\n\t"
+      "subc.cc.u32 %3, %3, %11;\n\t"
+      "subc.cc.u32 %4, %4, %12;\n\t"
+      "subc.cc.u32 %5, %5, %13;\n\t"
+      "subc.cc.u32 %6, %6, %14;\n\t"
+      "subc.u32    %7, %7, %15;"
+      : "+r"(t.v[0]), "+r"(t.v[1]), "+r"(t.v[2]), "+r"(t.v[3]), "+r"(t.v[4]), "+r"(t.v[5]), "+r"(t.v[6]), "+r"(t.v[7])
+      : "r"(b.v[0]), "r"(b.v[1]), "r"(b.v[2]), "r"(b.v[3]), "r"(b.v[4]), "r"(b.v[5]), "r"(b.v[6]), "r"(b.v[7]));
+  return t;
+}
+// a below 4r -> below 2r
+BG_DEV Fr reduce2(const Fr& a) {
+  uint32_t d[8], bw;
+  asm("sub.cc.u32  %0, %9,  %17;\n\t"
+      "subc.cc.u32 %1, %10, %18;\n\t"
+      "subc.cc.u32 %2, %11, %19;\n\t"
+      "subc.cc.u32 %3, %12, %20;\n\t"
+      "subc.cc.u32 %4, %13, %21;\n\t"
+      "subc.cc.u32 %5, %14, %22;\n\t"
+      "subc.cc.u32 %6, %15, %23;\n\t"
+      "subc.cc.u32 %7, %16, %24;\n\t"
+      "subc.u32    %8, 0, 0;"
+      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]), "=r"(bw)
+      : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7]),
+        "n"(kTwoR[0]), "n"(kTwoR[1]), "n"(kTwoR[2]), "n"(kTwoR[3]), "n"(kTwoR[4]), "n"(kTwoR[5]), "n"(kTwoR[6]),
+        "n"(kTwoR[7]));
+  Fr r;
+#pragma unroll
+  for (int i = 0; i < 8; i++) r.v[i] = bw ? a.v[i] : d[i];
+  return r;
+}
+// a below 2r -> below r
+BG_DEV Fr reduce1(const Fr& a) {
+  Fr r;
+  reduce_once<FrParams>(r.v, a.v);
+  return r;
+}
+
+// one butterfly: DIF (x0 + x1, (x0 - x1) w), values below 2r; DIT (x0 + x1 w, x0 - x1 w), values
+// below 4r.  `unit`: w = 1, no product.
+template <bool DIT>
+BG_DEV void butterfly(Fr& x0, Fr& x1, const uint32_t* __restrict__ tw, size_t widx, bool unit) {
+  if (DIT) {
+    const Fr a = reduce2(x0);
+    Fr b;
+    if (unit) b = reduce2(x1);
+    else b = mul_loose(load_fp<FrParams>(tw + 8 * widx), x1);
+    x0 = add_raw(a, b);
+    x1 = sub_plus2(a, b);
+  } else {
+    const Fr d = sub_plus2(x0, x1);
+    x0 = reduce2(add_raw(x0, x1));
+    if (unit) x1 = reduce2(d);
+    else x1 = mul_loose(load_fp<FrParams>(tw + 8 * widx), d);
+  }
+}
+
 // Up to three vectors transformed by one launch (the QAP's a, b and c), blockIdx.y picks one.
 struct NttVecs {
-  uint32_t* p[3];
+  const uint32_t* src[3];
+  uint32_t* dst[3];
 };
+// what a pass does on load besides its scaling: nothing, or the QAP's quotient on the coset,
+// (src[0] src[1] - src[2]) zinv
+enum LoadMode { LD_PLAIN = 0, LD_QUOTIENT = 1 };
 
-template <bool DIT, int NT>
-__global__ void __launch_bounds__(NT) k_ntt_pass(NttVecs vecs, const uint32_t* __restrict__ tw, int L, int s0, int k,
-                                                 int G, int pre_mode, int post_mode, ScaleTab sc) {
+// One pass: stages [s0, s0 + k) of a size-2^L transform.  A CTA owns G independent groups of
+// 2^k elements; group element t of group (hi, lo) sits at hi*2^(s0+k) + t*2^s0 + lo, and goes back
+// there or (rev) to the bit-reversed place.  Two stages at a time on four elements in registers
+// (R4), so a tile crosses shared memory and its barrier once per two stages; the latency-bound
+// passes of small domains take one stage at a time, with twice the threads.
+//
+// Bound by the FMA-heavy pipe (10 M products of a 2^20 transform: 138 us) and, a third of the time,
+// by the latency of the twiddles (32 bytes from L2 per product of the strided pass).  Three
+// 256-thread CTAs per SM (80 registers): 2^20 forward 200 us, against 216 with two (102 registers)
+// and 208 with four (64, some spills); one stage at a time with full reductions, and the bit
+// reversal as a pass of its own and a copy back, took 239.  The QAP takes the four-CTA form (OCC): a
+// proof's accumulations take an SM's slots first, and smaller CTAs fit beside them (SquareChain(2^18)
+// 6.72 -> 6.67 ms).
+template <bool DIT, bool R4, int NT, int OCC>
+__global__ void __launch_bounds__(NT, OCC) k_ntt_pass(NttVecs vecs, const uint32_t* __restrict__ tw, int L, int s0, int k,
+                                                 int G, int pre_mode, int post_mode, ScaleTab sc, int load_mode,
+                                                 const uint32_t* __restrict__ zinv, int rev) {
   extern __shared__ __align__(16) uint32_t sm[];
-  uint32_t* __restrict__ data = vecs.p[blockIdx.y];
+  const uint32_t* src = blockIdx.y == 0 ? vecs.src[0] : blockIdx.y == 1 ? vecs.src[1] : vecs.src[2];
+  uint32_t* dst = blockIdx.y == 0 ? vecs.dst[0] : blockIdx.y == 1 ? vecs.dst[1] : vecs.dst[2];
   const int E = G << k;
   const uint32_t kmask = (1u << k) - 1u;
   const size_t lomask = (size_t(1) << s0) - 1;
   const size_t gid0 = (size_t)blockIdx.x * G;
-
-  for (int idx = threadIdx.x; idx < E; idx += blockDim.x) {
+  auto place = [&](int idx, int& e) -> size_t {
     int grp, t;
     if (s0 == 0) {
       grp = idx >> k;
@@ -92,65 +192,105 @@ __global__ void __launch_bounds__(NT) k_ntt_pass(NttVecs vecs, const uint32_t* _
       grp = idx % G;
       t = idx / G;
     }
+    e = (grp << k) | t;
     const size_t gid = gid0 + grp;
-    const size_t j = (s0 == 0) ? ((gid << k) | (size_t)t)
-                               : (((gid >> s0) << (s0 + k)) | ((size_t)t << s0) | (gid & lomask));
-    Fr x = load_fp<FrParams>(data + 8 * j);
+    return (s0 == 0) ? ((gid << k) | (size_t)t)
+                     : (((gid >> s0) << (s0 + k)) | ((size_t)t << s0) | (gid & lomask));
+  };
+
+  for (int idx = threadIdx.x; idx < E; idx += blockDim.x) {
+    int e;
+    const size_t j = place(idx, e);
+    Fr x = load_fp<FrParams>(src + 8 * j);
+    if (load_mode == LD_QUOTIENT) {
+      const Fr y = load_fp<FrParams>(vecs.src[1] + 8 * j), z = load_fp<FrParams>(vecs.src[2] + 8 * j);
+      x = mul(load_fp<FrParams>(zinv), sub(mul(x, y), z));
+    }
     if (pre_mode != SC_NONE) x = mul(scale_factor(pre_mode, j, L, sc), x);
-    tile_store(sm, E, (grp << k) | t, x);
+    tile_store(sm, E, e, x);
   }
   __syncthreads();
 
-  const int half = E >> 1;
-  for (int rr = 0; rr < k; rr++) {
-    const int r = DIT ? rr : (k - 1 - rr);
-    const int s = s0 + r;
-    const uint32_t rmask = (1u << r) - 1u;
-    for (int b = threadIdx.x; b < half; b += blockDim.x) {
-      const int grp = b >> (k - 1);
-      const uint32_t q = (uint32_t)b & ((1u << (k - 1)) - 1u);
-      const uint32_t t1 = ((q >> r) << (r + 1)) | (q & rmask);
-      const uint32_t t2 = t1 | (1u << r);
-      const size_t lo = (s0 == 0) ? 0 : ((gid0 + grp) & lomask);
-      const size_t widx = ((((size_t)(q & rmask)) << s0) + lo) << (L - s - 1);
-      const int e1 = (grp << k) | (int)t1, e2 = (grp << k) | (int)t2;
-      Fr x1 = tile_load(sm, E, e1), x2 = tile_load(sm, E, e2);
-      Fr y1, y2;
-      if (widx == 0) {  // w = 1
-        y1 = add(x1, x2);
-        y2 = sub(x1, x2);
-      } else {
-        const Fr w = load_fp<FrParams>(tw + 8 * widx);
-        if (DIT) {
-          x2 = mul(w, x2);
-          y1 = add(x1, x2);
-          y2 = sub(x1, x2);
-        } else {
-          y1 = add(x1, x2);
-          y2 = mul(w, sub(x1, x2));
-        }
+  // twiddle of the pair at stage r whose lower r bits are q, in group `lo`: w^(((q << s0) + lo) << (L - s - 1))
+  if constexpr (R4) {
+    const int quads = E >> 2;
+    int done = 0;
+    if (k & 1) {  // an odd stage by itself: the lowest for DIT, the highest for DIF
+      const int r = DIT ? 0 : k - 1;
+      const uint32_t rmask = (1u << r) - 1u;
+      for (int b = threadIdx.x; b < (E >> 1); b += blockDim.x) {
+        const int grp = b >> (k - 1);
+        const uint32_t q = (uint32_t)b & ((1u << (k - 1)) - 1u);
+        const int e1 = (grp << k) | (int)(((q >> r) << (r + 1)) | (q & rmask)), e2 = e1 | (1 << r);
+        const size_t lo = (s0 == 0) ? 0 : ((gid0 + grp) & lomask);
+        const size_t widx = ((((size_t)(q & rmask)) << s0) + lo) << (L - s0 - r - 1);
+        Fr x0 = tile_load(sm, E, e1), x1 = tile_load(sm, E, e2);
+        butterfly<DIT>(x0, x1, tw, widx, s0 == 0 && r == 0);
+        tile_store(sm, E, e1, x0);
+        tile_store(sm, E, e2, x1);
       }
-      tile_store(sm, E, e1, y1);
-      tile_store(sm, E, e2, y2);
+      __syncthreads();
+      done = 1;
     }
-    __syncthreads();
+    for (; done < k; done += 2) {
+      const int r = DIT ? done : k - 2 - done;  // the lower of the two stages
+      const uint32_t rmask = (1u << r) - 1u;
+      const bool unit = s0 == 0 && r == 0;
+      for (int b = threadIdx.x; b < quads; b += blockDim.x) {
+        const int grp = b >> (k - 2);
+        const uint32_t q = (uint32_t)b & ((1u << (k - 2)) - 1u);
+        const int e = (grp << k) | (int)(((q >> r) << (r + 2)) | (q & rmask));
+        const int st = 1 << r;
+        const size_t lo = (s0 == 0) ? 0 : ((gid0 + grp) & lomask);
+        // lower stage: both pairs at w^(2 h); upper stage: w^h and w^(h + 2^(L-2))
+        const size_t h = ((((size_t)(q & rmask)) << s0) + lo) << (L - s0 - r - 2), quarter = size_t(1) << (L - 2);
+        Fr x0 = tile_load(sm, E, e), x1 = tile_load(sm, E, e + st), x2 = tile_load(sm, E, e + 2 * st),
+           x3 = tile_load(sm, E, e + 3 * st);
+        if (DIT) {
+          butterfly<DIT>(x0, x1, tw, 2 * h, unit);
+          butterfly<DIT>(x2, x3, tw, 2 * h, unit);
+          butterfly<DIT>(x0, x2, tw, h, unit);
+          butterfly<DIT>(x1, x3, tw, h + quarter, false);
+        } else {
+          butterfly<DIT>(x0, x2, tw, h, unit);
+          butterfly<DIT>(x1, x3, tw, h + quarter, false);
+          butterfly<DIT>(x0, x1, tw, 2 * h, unit);
+          butterfly<DIT>(x2, x3, tw, 2 * h, unit);
+        }
+        tile_store(sm, E, e, x0);
+        tile_store(sm, E, e + st, x1);
+        tile_store(sm, E, e + 2 * st, x2);
+        tile_store(sm, E, e + 3 * st, x3);
+      }
+      __syncthreads();
+    }
+  } else {
+    const int half = E >> 1;
+    for (int rr = 0; rr < k; rr++) {
+      const int r = DIT ? rr : (k - 1 - rr);
+      const uint32_t rmask = (1u << r) - 1u;
+      for (int b = threadIdx.x; b < half; b += blockDim.x) {
+        const int grp = b >> (k - 1);
+        const uint32_t q = (uint32_t)b & ((1u << (k - 1)) - 1u);
+        const int e1 = (grp << k) | (int)(((q >> r) << (r + 1)) | (q & rmask)), e2 = e1 | (1 << r);
+        const size_t lo = (s0 == 0) ? 0 : ((gid0 + grp) & lomask);
+        const size_t widx = ((((size_t)(q & rmask)) << s0) + lo) << (L - s0 - r - 1);
+        Fr x0 = tile_load(sm, E, e1), x1 = tile_load(sm, E, e2);
+        butterfly<DIT>(x0, x1, tw, widx, s0 == 0 && r == 0);
+        tile_store(sm, E, e1, x0);
+        tile_store(sm, E, e2, x1);
+      }
+      __syncthreads();
+    }
   }
 
   for (int idx = threadIdx.x; idx < E; idx += blockDim.x) {
-    int grp, t;
-    if (s0 == 0) {
-      grp = idx >> k;
-      t = idx & kmask;
-    } else {
-      grp = idx % G;
-      t = idx / G;
-    }
-    const size_t gid = gid0 + grp;
-    const size_t j = (s0 == 0) ? ((gid << k) | (size_t)t)
-                               : (((gid >> s0) << (s0 + k)) | ((size_t)t << s0) | (gid & lomask));
-    Fr x = tile_load(sm, E, (grp << k) | t);
+    int e;
+    const size_t j = place(idx, e);
+    Fr x = tile_load(sm, E, e);
     if (post_mode != SC_NONE) x = mul(scale_factor(post_mode, j, L, sc), x);
-    store_fp(data + 8 * j, x);
+    else x = reduce1(DIT ? reduce2(x) : x);
+    store_fp(dst + 8 * (rev && L ? (size_t)(__brevll((unsigned long long)j) >> (64 - L)) : j), x);
   }
 }
 
@@ -162,23 +302,6 @@ __global__ void k_table_expand(uint32_t* __restrict__ out, const uint32_t* __res
   const Fr a = load_fp<FrParams>(lo + 8 * (i & ((size_t(1) << bits) - 1)));
   const Fr b = load_fp<FrParams>(hi + 8 * (i >> bits));
   store_fp(out + 8 * i, mul(a, b));
-}
-
-// out[bitrev_L(i)] = in[i]
-__global__ void k_bitrev(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, int L, size_t n) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const size_t j = L ? (__brevll((unsigned long long)i) >> (64 - L)) : 0;
-  store_fp(out + 8 * j, load_fp<FrParams>(in + 8 * i));
-}
-
-// a[i] = (a[i] * b[i] - c[i]) * zinv
-__global__ void k_qap_pointwise(uint32_t* __restrict__ a, const uint32_t* __restrict__ b,
-                                const uint32_t* __restrict__ c, const uint32_t* __restrict__ zinv, size_t n) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const Fr x = load_fp<FrParams>(a + 8 * i), y = load_fp<FrParams>(b + 8 * i), z = load_fp<FrParams>(c + 8 * i);
-  store_fp(a + 8 * i, mul(sub(mul(x, y), z), load_fp<FrParams>(zinv)));
 }
 
 // ---------------------------------------------------------------- host side
@@ -261,6 +384,7 @@ NttTables& ntt_tables(Ctx& ctx, int L) {
   slot.g_hi = ctx.ws.get_t<uint32_t>(tag + ".g_hi", chi * 8);
   slot.g_hi_ninv = ctx.ws.get_t<uint32_t>(tag + ".g_hi_ninv", chi * 8);
   slot.gi_hi_ninv = ctx.ws.get_t<uint32_t>(tag + ".gi_hi_ninv", chi * 8);
+  slot.gi_hi_ninv_canon = ctx.ws.get_t<uint32_t>(tag + ".gi_hi_ninv_canon", chi * 8);
   slot.ninv = ctx.ws.get_t<uint32_t>(tag + ".ninv", 8);
   slot.zinv = ctx.ws.get_t<uint32_t>(tag + ".zinv", 8);
   upload_fes(ctx, slot.g_lo, powers(g, clo, one));
@@ -268,6 +392,7 @@ NttTables& ntt_tables(Ctx& ctx, int L) {
   upload_fes(ctx, slot.g_hi, powers(ga, chi, one));
   upload_fes(ctx, slot.g_hi_ninv, powers(ga, chi, ninv));
   upload_fes(ctx, slot.gi_hi_ninv, powers(gia, chi, ninv));
+  upload_fes(ctx, slot.gi_hi_ninv_canon, powers(gia, chi, bgh::fe_from_mont(FR, ninv)));
   upload_fes(ctx, slot.ninv, {ninv});
   // Z(g x) on the coset is the constant g^n - 1
   const Fe zc = bgh::fe_sub(FR, bgh::fe_pow_u64(FR, g, n), one);
@@ -279,6 +404,7 @@ NttTables& ntt_tables(Ctx& ctx, int L) {
 struct PassPlan {
   int s0, k, G;
   int nt = kNttThreads;  // threads per CTA
+  bool r4 = true;        // two stages at a time
 };
 
 // Small domains (at most 2^kSmallMaxL elements, a small proof's QAP) are a chain of
@@ -289,6 +415,7 @@ struct PassPlan {
 // the SM's issue rate spread over 1024 butterflies a stage.
 constexpr int kSmallMaxL = 14;
 constexpr int kSmallTile = 128;
+constexpr int kSmallThreads = 64;
 
 static std::vector<PassPlan> plan_passes(int L) {
   const bool small = L <= kSmallMaxL;
@@ -298,6 +425,7 @@ static std::vector<PassPlan> plan_passes(int L) {
   auto add = [&](int s0, int k, int G) {
     PassPlan p{s0, k, G};
     p.nt = small ? std::max(32, (G << k) / 2) : kNttThreads;
+    p.r4 = !small;
     out.push_back(p);
   };
   const int k0 = std::min(L, kmax);
@@ -323,15 +451,35 @@ static std::vector<PassPlan> plan_passes(int L) {
   return out;
 }
 
+// how a pass reads, scales and writes
+struct PassIo {
+  int pre = SC_NONE, post = SC_NONE;
+  ScaleTab sc;
+  int load = LD_PLAIN;
+  const uint32_t* zinv = nullptr;
+  bool rev = false;
+  bool qap = false;
+};
+
 static void launch_pass(Ctx& ctx, cudaStream_t st, bool dit, const NttVecs& v, int nvec, const uint32_t* tw, int L,
-                        const PassPlan& p, int pre, int post, const ScaleTab& sc) {
+                        const PassPlan& p, const PassIo& io) {
   const size_t n = size_t(1) << L;
   const int E = p.G << p.k;
   const dim3 grid((unsigned)(n / E), (unsigned)nvec);
   const size_t smem = (size_t)E * 32;
   KernelTimer kt(ctx, "ntt_pass", st);
-  if (dit) k_ntt_pass<true, kNttThreads><<<grid, p.nt, smem, st>>>(v, tw, L, p.s0, p.k, p.G, pre, post, sc);
-  else k_ntt_pass<false, kNttThreads><<<grid, p.nt, smem, st>>>(v, tw, L, p.s0, p.k, p.G, pre, post, sc);
+  auto go = [&](auto kernel) {
+    kernel<<<grid, p.nt, smem, st>>>(v, tw, L, p.s0, p.k, p.G, io.pre, io.post, io.sc, io.load, io.zinv, io.rev);
+  };
+  if (!p.r4) {
+    if (dit) go(k_ntt_pass<true, false, kSmallThreads, 4>);
+    else go(k_ntt_pass<false, false, kSmallThreads, 4>);
+  } else if (io.qap) {
+    if (dit) go(k_ntt_pass<true, true, kNttThreads, 4>);
+    else go(k_ntt_pass<false, true, kNttThreads, 4>);
+  } else {
+    go(k_ntt_pass<false, true, kNttThreads, 3>);  // standalone transforms are DIF
+  }
   BG_CHECK_LAUNCH();
 }
 
@@ -344,36 +492,47 @@ void ntt_init_kernels() {
   BG_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= kMaxDevices) throw Error(BG_E_ARG, "ntt: device index out of range");
   std::call_once(once[dev], [] {
-    BG_CUDA(cudaFuncSetAttribute(k_ntt_pass<true, kNttThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kNttTile * 32));
-    BG_CUDA(cudaFuncSetAttribute(k_ntt_pass<false, kNttThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kNttTile * 32));
+    auto smem = [](auto* kernel) {
+      BG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kNttTile * 32));
+    };
+    smem(k_ntt_pass<true, true, kNttThreads, 4>);
+    smem(k_ntt_pass<false, true, kNttThreads, 4>);
+    smem(k_ntt_pass<false, true, kNttThreads, 3>);
   });
 }
 
-// DIF passes (natural -> bit-reversed).  `first_pre` scales on load in the first pass;
-// `last_post` scales on store in the last (contiguous) pass.
-static void dif(Ctx& ctx, cudaStream_t st, const NttVecs& v, int nvec, const uint32_t* tw, int L, int first_pre,
-                const ScaleTab& pre_sc, int last_post, const ScaleTab& post_sc) {
-  auto plan = plan_passes(L);
+// DIF passes (natural order in, bit-reversed out): from v.src into v.dst by way of `mid` (v.dst
+// itself, or where the last pass undoes the bit reversal into v.dst, whose elements then change
+// places, another buffer).  `first` and `last` say how the outer passes read and write.
+static void dif(Ctx& ctx, cudaStream_t st, const NttVecs& v, uint32_t* const* mid, int nvec, const uint32_t* tw, int L,
+                const PassIo& first, const PassIo& last) {
+  const auto plan = plan_passes(L);
   for (int i = (int)plan.size() - 1; i >= 0; i--) {
-    const bool first = i == (int)plan.size() - 1, last = i == 0;
-    if (first && last) {
-      // one pass: both scalings come from different tables; apply pre separately if needed
-      if (first_pre != SC_NONE && last_post != SC_NONE)
-        throw Error(BG_E_ARG, "ntt: pre and post scaling in a single-pass transform");
-      launch_pass(ctx, st, false, v, nvec, tw, L, plan[i], first_pre, last_post, first_pre ? pre_sc : post_sc);
-    } else {
-      launch_pass(ctx, st, false, v, nvec, tw, L, plan[i], first ? first_pre : SC_NONE, last ? last_post : SC_NONE,
-                  first ? pre_sc : post_sc);
+    const bool is_first = i == (int)plan.size() - 1, is_last = i == 0;
+    NttVecs w = v;
+    for (int k = 0; k < nvec; k++) {
+      if (!is_first) w.src[k] = mid[k];
+      if (!is_last) w.dst[k] = mid[k];
     }
+    PassIo io;
+    io.qap = last.qap;
+    if (is_first) io = first;
+    if (is_last) {
+      if (is_first && first.pre != SC_NONE && last.post != SC_NONE)
+        throw Error(BG_E_ARG, "ntt: pre and post scaling in a single-pass transform");
+      io.post = last.post;
+      io.rev = last.rev;
+      if (last.post != SC_NONE) io.sc = last.sc;
+    }
+    launch_pass(ctx, st, false, w, nvec, tw, L, plan[i], io);
   }
 }
 
 static void dit(Ctx& ctx, cudaStream_t st, const NttVecs& v, int nvec, const uint32_t* tw, int L) {
-  auto plan = plan_passes(L);
-  for (size_t i = 0; i < plan.size(); i++)
-    launch_pass(ctx, st, true, v, nvec, tw, L, plan[i], SC_NONE, SC_NONE, ScaleTab{});
+  const auto plan = plan_passes(L);
+  PassIo io;
+  io.qap = true;
+  for (size_t i = 0; i < plan.size(); i++) launch_pass(ctx, st, true, v, nvec, tw, L, plan[i], io);
 }
 
 void ntt_run(Ctx& ctx, cudaStream_t st, uint32_t* d_data, int L, int mode) {
@@ -381,57 +540,62 @@ void ntt_run(Ctx& ctx, cudaStream_t st, uint32_t* d_data, int L, int mode) {
   ntt_init_kernels();
   NttTables& T = ntt_tables(ctx, L);
   const size_t n = size_t(1) << L;
+  // the passes before the last leave their tiles in tmp; the last goes back in natural order
   uint32_t* tmp = ctx.ws.get_t<uint32_t>("ntt.tmp", n * 8);
-  ScaleTab none;
-  const NttVecs v{{d_data, d_data, d_data}};
+  const NttVecs v{{d_data, d_data, d_data}, {d_data, d_data, d_data}};
+  PassIo first, last;
+  last.rev = true;
+  const uint32_t* tw = T.tw_fwd;
   switch (mode) {
     case BG_NTT_FORWARD:
-      dif(ctx, st, v, 1, T.tw_fwd, L, SC_NONE, none, SC_NONE, none);
       break;
-    case BG_NTT_INVERSE: {
-      ScaleTab c;
-      c.hi = T.ninv;
-      dif(ctx, st, v, 1, T.tw_inv, L, SC_NONE, none, SC_CONST, c);
+    case BG_NTT_INVERSE:
+      tw = T.tw_inv;
+      last.post = SC_CONST;
+      last.sc.hi = T.ninv;
       break;
-    }
-    case BG_NTT_COSET_FORWARD: {
-      ScaleTab c{T.g_lo, T.g_hi, T.coset_bits};
-      dif(ctx, st, v, 1, T.tw_fwd, L, SC_NATURAL, c, SC_NONE, none);
+    case BG_NTT_COSET_FORWARD:
+      first.pre = SC_NATURAL;
+      first.sc = ScaleTab{T.g_lo, T.g_hi, T.coset_bits};
       break;
-    }
-    case BG_NTT_COSET_INVERSE: {
-      ScaleTab c{T.gi_lo, T.gi_hi_ninv, T.coset_bits};
-      dif(ctx, st, v, 1, T.tw_inv, L, SC_NONE, none, SC_BITREV, c);
+    case BG_NTT_COSET_INVERSE:
+      tw = T.tw_inv;
+      last.post = SC_BITREV;
+      last.sc = ScaleTab{T.gi_lo, T.gi_hi_ninv, T.coset_bits};
       break;
-    }
     default:
       throw Error(BG_E_ARG, "ntt: unknown mode");
   }
-  k_bitrev<<<ceil_div(n, 256), 256, 0, st>>>(d_data, tmp, L, n);
-  BG_CHECK_LAUNCH();
-  BG_CUDA(cudaMemcpyAsync(d_data, tmp, n * 32, cudaMemcpyDeviceToDevice, st));
+  dif(ctx, st, v, &tmp, 1, tw, L, first, last);
 }
 
 // h from the three evaluation vectors (all natural order, packed Montgomery, n = 2^L each).
-// a, b, c are overwritten; h receives n elements (h[n-1] = 0 for a satisfied R1CS).
-void qap_h_run(Ctx& ctx, cudaStream_t st, uint32_t* d_a, uint32_t* d_b, uint32_t* d_c, uint32_t* d_h, int L) {
+// a, b, c are overwritten; h receives n elements (h[n-1] = 0 for a satisfied R1CS), Montgomery or
+// (canonical) as MSM scalars: the factor of the last scaling then comes from a table that is not in
+// Montgomery form, which takes h's own factor R out.
+void qap_h_run(Ctx& ctx, cudaStream_t st, uint32_t* d_a, uint32_t* d_b, uint32_t* d_c, uint32_t* d_h, int L,
+               bool canonical) {
   ntt_init_kernels();
   NttTables& T = ntt_tables(ctx, L);
-  const size_t n = size_t(1) << L;
-  ScaleTab none;
-  ScaleTab to_coset{T.g_lo, T.g_hi_ninv, T.coset_bits};
-  ScaleTab from_coset{T.gi_lo, T.gi_hi_ninv, T.coset_bits};
   // a, b and c are transformed by the same launches (grid y = 3): each pass fills three times
-  // the CTAs, and a small proof's QAP is 8 launches instead of 16
-  const NttVecs abc{{d_a, d_b, d_c}};
-  dif(ctx, st, abc, 3, T.tw_inv, L, SC_NONE, none, SC_BITREV, to_coset);  // iNTT, then * n^-1 g^j
-  dit(ctx, st, abc, 3, T.tw_fwd, L);                                      // NTT on the coset
-  k_qap_pointwise<<<ceil_div(n, 256), 256, 0, st>>>(d_a, d_b, d_c, T.zinv, n);
-  BG_CHECK_LAUNCH();
-  const NttVecs a{{d_a, d_a, d_a}};
-  dif(ctx, st, a, 1, T.tw_inv, L, SC_NONE, none, SC_BITREV, from_coset);  // coset iNTT
-  k_bitrev<<<ceil_div(n, 256), 256, 0, st>>>(d_a, d_h, L, n);
-  BG_CHECK_LAUNCH();
+  // the CTAs, and a small proof's QAP is 6 launches instead of 16
+  uint32_t* const abc[3] = {d_a, d_b, d_c};
+  const NttVecs v{{d_a, d_b, d_c}, {d_a, d_b, d_c}};
+  PassIo plain, to_coset;  // iNTT, then * n^-1 g^j
+  plain.qap = to_coset.qap = true;
+  to_coset.post = SC_BITREV;
+  to_coset.sc = ScaleTab{T.g_lo, T.g_hi_ninv, T.coset_bits};
+  dif(ctx, st, v, abc, 3, T.tw_inv, L, plain, to_coset);
+  dit(ctx, st, v, 3, T.tw_fwd, L);  // NTT on the coset
+  PassIo quotient, from_coset;      // (a b - c) / Z, then the coset iNTT
+  quotient.qap = from_coset.qap = true;
+  quotient.load = LD_QUOTIENT;
+  quotient.zinv = T.zinv;
+  from_coset.post = SC_BITREV;
+  from_coset.sc = ScaleTab{T.gi_lo, canonical ? T.gi_hi_ninv_canon : T.gi_hi_ninv, T.coset_bits};
+  from_coset.rev = true;
+  const NttVecs q{{d_a, d_b, d_c}, {d_h, d_h, d_h}};
+  dif(ctx, st, q, abc, 1, T.tw_inv, L, quotient, from_coset);
 }
 
 }  // namespace bg

@@ -43,12 +43,20 @@ using bgh::Xyzz;
 // Row i < N: sum_e coeff_e * z[col_e] over the CSR row (a coefficient equal to Montgomery one
 // skips the product, as Ev.ent.s2 does, groth16.bend:108-113).  Rows N .. N+ni-1 of A carry the
 // libsnark input-consistency entries a[N+i] = z[i] (groth16.bend:182-188); all other rows are 0.
-__global__ void k_evals(const uint32_t* __restrict__ offs, const uint32_t* __restrict__ cols,
-                        const uint32_t* __restrict__ coeffs, const uint32_t* __restrict__ z, uint32_t nz,
-                        uint32_t nrows, uint32_t ni_rows, size_t d, uint32_t* __restrict__ out,
-                        uint32_t* __restrict__ status) {
+// One launch for the three matrices, blockIdx.y picks one.
+struct EvalJobs {
+  const uint32_t *offs[3], *cols[3], *coeffs[3];
+  uint32_t* out[3];
+};
+__global__ void k_evals(EvalJobs jobs, const uint32_t* __restrict__ z, uint32_t nz, uint32_t nrows, uint32_t ni,
+                        size_t d, uint32_t* __restrict__ status) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= d) return;
+  const uint32_t* __restrict__ offs = jobs.offs[blockIdx.y];
+  const uint32_t* __restrict__ cols = jobs.cols[blockIdx.y];
+  const uint32_t* __restrict__ coeffs = jobs.coeffs[blockIdx.y];
+  uint32_t* __restrict__ out = jobs.out[blockIdx.y];
+  const uint32_t ni_rows = blockIdx.y == 0 ? ni : 0u;
   Fr acc = fp_zero<FrParams>();
   if (i < nrows) {
     const Fr one = fp_one<FrParams>();
@@ -433,7 +441,6 @@ void prove_resident(Ctx& ctx, PkDev& pk, const uint32_t* witness16, const uint32
   // ---- the MSMs whose scalars are the assignment go first (host launch order matters for
   // small proofs, whose kernels are shorter than the host's launches): msm_a, msm_b1, msm_b2,
   // msm_l; msm_h follows the QAP
-  uint32_t* hh = ws.get_t<uint32_t>("prove.h", d * 8);
   uint32_t* hc = ws.get_t<uint32_t>("prove.hc", d * 8);
   MsmPlan plan[5];  // a, b1, b2, h, l
   struct Job {
@@ -529,15 +536,14 @@ void prove_resident(Ctx& ctx, PkDev& pk, const uint32_t* witness16, const uint32
   uint32_t* ea = ws.get_t<uint32_t>("prove.ea", d * 8);
   uint32_t* eb = ws.get_t<uint32_t>("prove.eb", d * 8);
   uint32_t* ec = ws.get_t<uint32_t>("prove.ec", d * 8);
-  const CsrDev* m[3] = {&pk.ca, &pk.cb, &pk.cc};
-  uint32_t* ev[3] = {ea, eb, ec};
+  const EvalJobs ev{{pk.ca.offs, pk.cb.offs, pk.cc.offs},
+                    {pk.ca.cols, pk.cb.cols, pk.cc.cols},
+                    {pk.ca.coeffs, pk.cb.coeffs, pk.cc.coeffs},
+                    {ea, eb, ec}};
   if (pk.csr_ready) BG_CUDA(cudaStreamWaitEvent(st, pk.csr_ready, 0));
   std::unique_ptr<KernelTimer> kt_evals(new KernelTimer(ctx, "evals", st));
-  for (int k = 0; k < 3; k++) {
-    k_evals<<<ceil_div(d, 128), 128, 0, st>>>(m[k]->offs, m[k]->cols, m[k]->coeffs, z, (uint32_t)nz, h.nc,
-                                              k == 0 ? h.ni : 0, d, ev[k], ctx.d_status);
-    BG_CHECK_LAUNCH();
-  }
+  k_evals<<<dim3(ceil_div(d, 128), 3), 128, 0, st>>>(ev, z, (uint32_t)nz, h.nc, h.ni, d, ctx.d_status);
+  BG_CHECK_LAUNCH();
   kt_evals.reset();
   t_evals.stop(st);
 
@@ -545,8 +551,7 @@ void prove_resident(Ctx& ctx, PkDev& pk, const uint32_t* witness16, const uint32
   t_qap.start(st);
   {
     KernelTimer kt(ctx, "qap", st);
-    qap_h_run(ctx, st, ea, eb, ec, hh, h.lg);
-    fr_from_mont(st, hh, hc, h.nh);
+    qap_h_run(ctx, st, ea, eb, ec, hc, h.lg, true);
   }
   t_qap.stop(st);
 
