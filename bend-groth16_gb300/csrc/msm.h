@@ -82,7 +82,8 @@ void msm_launch(Ctx& ctx, cudaStream_t st, const std::string& tag, const uint32_
                 const uint32_t* d_scalars, size_t n, MsmPlan& plan, cudaStream_t st_reduce = nullptr,
                 const MsmTable* table = nullptr);
 // The two halves of msm_launch: the sort on `st` (records so.done), and everything after it
-// on `st` (waits for so.done) with the fixup and reduction on `st_reduce`.
+// on `st` (waits for so.done) with the fixup and reduction on `st_reduce`.  A context's sorts
+// share a rank buffer: sorts on different streams must be ordered by the caller.
 void msm_sort(Ctx& ctx, cudaStream_t st, const std::string& tag, const uint32_t* d_scalars, size_t n, int c,
               bool shared_set, int rounds, MsmSort& out);
 // Batch-affine pair rounds of an MSM of n points with c-bit windows (the context's override, else

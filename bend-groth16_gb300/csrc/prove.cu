@@ -529,6 +529,8 @@ void prove_resident(Ctx& ctx, PkDev& pk, const uint32_t* witness16, const uint32
   };
   const MsmSort* so[4];
   for (int j = 0; j < 4; j++) so[j] = &sort_for(jobs[j], sort_st);
+  cudaEvent_t ev_sorted = ctx.event("prove.sorted");
+  BG_CUDA(cudaEventRecord(ev_sorted, sort_st));
   for (int j = 0; j < 4; j++) launch(j, *so[j]);
 
   // ---- evals
@@ -555,7 +557,9 @@ void prove_resident(Ctx& ctx, PkDev& pk, const uint32_t* witness16, const uint32
   }
   t_qap.stop(st);
 
-  // ---- msm_h: its sort on the main stream after the QAP, then its accumulation last
+  // ---- msm_h: its sort on the main stream after the QAP (and the other sorts, whose rank buffer
+  // it takes over), then its accumulation last
+  BG_CUDA(cudaStreamWaitEvent(st, ev_sorted, 0));
   launch(4, sort_for(jobs[4], st));
 
   // ---- host work that needs no MSM result, overlapped with the device
