@@ -18,18 +18,8 @@ struct Mod {
   uint64_t r2[4];   // R^2 mod p
 };
 
-// p from bend2/src/fq.bend:2 and bend2/src/fr.bend:2; compile-time constants, so every product
-// below is built for its modulus
-inline constexpr Mod FQ = {
-    {0x3c208c16d87cfd47ull, 0x97816a916871ca8dull, 0xb85045b68181585dull, 0x30644e72e131a029ull},
-    0x87d20782e4866389ull,
-    {0xd35d438dc58f0d9dull, 0x0a78eb28f5c70b3dull, 0x666ea36f7879462cull, 0x0e0a77c19a07df2full},
-    {0xf32cfc5b538afa89ull, 0xb5e71911d44501fbull, 0x47ab1eff0a417ff6ull, 0x06d89f71cab8351full}};
-inline constexpr Mod FR = {
-    {0x43e1f593f0000001ull, 0x2833e84879b97091ull, 0xb85045b68181585dull, 0x30644e72e131a029ull},
-    0xc2e1f593efffffffull,
-    {0xac96341c4ffffffbull, 0x36fc76959f60cd29ull, 0x666ea36f7879462eull, 0x0e0a77c19a07df2full},
-    {0x1bb8e645ae216da7ull, 0x53fe3ab1e35c59e3ull, 0x8c49833d53bb8085ull, 0x0216d0b17f4e44a5ull}};
+extern const Mod FQ;
+extern const Mod FR;
 
 struct Fe {
   uint64_t v[4];
@@ -51,127 +41,66 @@ inline bool geq(const uint64_t* a, const uint64_t* b) {
   return true;
 }
 inline uint64_t sub4(uint64_t* r, const uint64_t* a, const uint64_t* b) {
-  u128 d = (u128)a[0] - b[0];
-  r[0] = (uint64_t)d;
-  d = (u128)a[1] - b[1] - ((uint64_t)(d >> 64) & 1);
-  r[1] = (uint64_t)d;
-  d = (u128)a[2] - b[2] - ((uint64_t)(d >> 64) & 1);
-  r[2] = (uint64_t)d;
-  d = (u128)a[3] - b[3] - ((uint64_t)(d >> 64) & 1);
-  r[3] = (uint64_t)d;
-  return (uint64_t)(d >> 64) & 1;
+  uint64_t borrow = 0;
+  for (int i = 0; i < 4; i++) {
+    u128 d = (u128)a[i] - b[i] - borrow;
+    r[i] = (uint64_t)d;
+    borrow = (uint64_t)(d >> 64) & 1;
+  }
+  return borrow;
 }
 inline uint64_t add4(uint64_t* r, const uint64_t* a, const uint64_t* b) {
-  u128 s = (u128)a[0] + b[0];
-  r[0] = (uint64_t)s;
-  s = (u128)a[1] + b[1] + (uint64_t)(s >> 64);
-  r[1] = (uint64_t)s;
-  s = (u128)a[2] + b[2] + (uint64_t)(s >> 64);
-  r[2] = (uint64_t)s;
-  s = (u128)a[3] + b[3] + (uint64_t)(s >> 64);
-  r[3] = (uint64_t)s;
-  return (uint64_t)(s >> 64);
-}
-// r = t - p when t >= p, else t (t < 2p), without a branch
-inline Fe fe_cond_sub(const Mod& m, const uint64_t* t) {
-  uint64_t d[4];
-  const uint64_t keep = 0 - sub4(d, t, m.p);  // all ones when t < p
-  Fe r;
-  for (int i = 0; i < 4; i++) r.v[i] = d[i] ^ ((d[i] ^ t[i]) & keep);
-  return r;
+  uint64_t c = 0;
+  for (int i = 0; i < 4; i++) {
+    u128 s = (u128)a[i] + b[i] + c;
+    r[i] = (uint64_t)s;
+    c = (uint64_t)(s >> 64);
+  }
+  return c;
 }
 
 inline Fe fe_add(const Mod& m, const Fe& a, const Fe& b) {
-  uint64_t t[4];
-  add4(t, a.v, b.v);  // < 2p < 2^255, no carry out
-  return fe_cond_sub(m, t);
+  Fe r;
+  add4(r.v, a.v, b.v);  // < 2p < 2^255, no carry out
+  if (geq(r.v, m.p)) sub4(r.v, r.v, m.p);
+  return r;
 }
 inline Fe fe_sub(const Mod& m, const Fe& a, const Fe& b) {
   Fe r;
-  const uint64_t mask = 0 - sub4(r.v, a.v, b.v);
-  const uint64_t pm[4] = {m.p[0] & mask, m.p[1] & mask, m.p[2] & mask, m.p[3] & mask};
-  add4(r.v, r.v, pm);
+  if (sub4(r.v, a.v, b.v)) add4(r.v, r.v, m.p);
   return r;
 }
 inline Fe fe_neg(const Mod& m, const Fe& a) { return fe_sub(m, fe_zero(), a); }
 inline Fe fe_dbl(const Mod& m, const Fe& a) { return fe_add(m, a, a); }
 
-// Row b of a CIOS Montgomery product: t = (t + a b + q p) / 2^64 with the q that clears limb 0.
-// For a < p < 2^254 the sum stays below 2p after every row, so four limbs hold it and the two
-// carry words can be added without overflow.
-inline __attribute__((always_inline)) void fe_mul_row(const Mod& m, uint64_t* t, const uint64_t* a, uint64_t b) {
-  u128 s = (u128)a[0] * b + t[0];
-  const uint64_t q = (uint64_t)s * m.n0;
-  uint64_t c = (uint64_t)(s >> 64);
-  u128 u = (u128)q * m.p[0] + (uint64_t)s;
-  s = (u128)a[1] * b + t[1] + c;
-  c = (uint64_t)(s >> 64);
-  u = (u128)q * m.p[1] + (uint64_t)s + (uint64_t)(u >> 64);
-  t[0] = (uint64_t)u;
-  s = (u128)a[2] * b + t[2] + c;
-  c = (uint64_t)(s >> 64);
-  u = (u128)q * m.p[2] + (uint64_t)s + (uint64_t)(u >> 64);
-  t[1] = (uint64_t)u;
-  s = (u128)a[3] * b + t[3] + c;
-  c = (uint64_t)(s >> 64);
-  u = (u128)q * m.p[3] + (uint64_t)s + (uint64_t)(u >> 64);
-  t[2] = (uint64_t)u;
-  t[3] = (uint64_t)(u >> 64) + c;
-}
-// a b 2^-256 mod p for a < p and any 256-bit b
-inline __attribute__((always_inline)) Fe fe_mul(const Mod& m, const Fe& a, const Fe& b) {
-  uint64_t t[4] = {0, 0, 0, 0};
-  fe_mul_row(m, t, a.v, b.v[0]);
-  fe_mul_row(m, t, a.v, b.v[1]);
-  fe_mul_row(m, t, a.v, b.v[2]);
-  fe_mul_row(m, t, a.v, b.v[3]);
-  return fe_cond_sub(m, t);
-}
-// t = a b (512 bits)
-inline __attribute__((always_inline)) void fe_wide_row(uint64_t* t, const uint64_t* a, uint64_t b) {
-  u128 s = (u128)a[0] * b + t[0];
-  t[0] = (uint64_t)s;
-  s = (u128)a[1] * b + t[1] + (uint64_t)(s >> 64);
-  t[1] = (uint64_t)s;
-  s = (u128)a[2] * b + t[2] + (uint64_t)(s >> 64);
-  t[2] = (uint64_t)s;
-  s = (u128)a[3] * b + t[3] + (uint64_t)(s >> 64);
-  t[3] = (uint64_t)s;
-  t[4] = (uint64_t)(s >> 64);
-}
-inline __attribute__((always_inline)) void fe_wide(uint64_t* t, const uint64_t* a, const uint64_t* b) {
-  t[0] = t[1] = t[2] = t[3] = 0;
-  fe_wide_row(t, a, b[0]);
-  fe_wide_row(t + 1, a, b[1]);
-  fe_wide_row(t + 2, a, b[2]);
-  fe_wide_row(t + 3, a, b[3]);
-}
-// t -= u (512 bits), returns the borrow
-inline __attribute__((always_inline)) uint64_t fe_wide_sub(uint64_t* t, const uint64_t* u) {
-  uint64_t borrow = 0;
-  for (int i = 0; i < 8; i++) {
-    const u128 d = (u128)t[i] - u[i] - borrow;
-    t[i] = (uint64_t)d;
-    borrow = (uint64_t)(d >> 64) & 1;
-  }
-  return borrow;
-}
-// t 2^-256 mod p for t < p 2^256: the low half reduced alone (at most p) plus the high half
-inline __attribute__((always_inline)) Fe fe_wide_redc(const Mod& m, const uint64_t* t) {
-  uint64_t r[4] = {t[0], t[1], t[2], t[3]};
+// CIOS Montgomery product a*b*2^-256 mod p
+inline Fe fe_mul(const Mod& m, const Fe& a, const Fe& b) {
+  uint64_t t[6] = {0, 0, 0, 0, 0, 0};
   for (int i = 0; i < 4; i++) {
-    const uint64_t q = r[0] * m.n0;
-    u128 u = (u128)q * m.p[0] + r[0];
-    u = (u128)q * m.p[1] + r[1] + (uint64_t)(u >> 64);
-    r[0] = (uint64_t)u;
-    u = (u128)q * m.p[2] + r[2] + (uint64_t)(u >> 64);
-    r[1] = (uint64_t)u;
-    u = (u128)q * m.p[3] + r[3] + (uint64_t)(u >> 64);
-    r[2] = (uint64_t)u;
-    r[3] = (uint64_t)(u >> 64);
+    uint64_t c = 0;
+    for (int j = 0; j < 4; j++) {
+      u128 s = (u128)a.v[j] * b.v[i] + t[j] + c;
+      t[j] = (uint64_t)s;
+      c = (uint64_t)(s >> 64);
+    }
+    u128 s = (u128)t[4] + c;
+    t[4] = (uint64_t)s;
+    t[5] = (uint64_t)(s >> 64);
+    const uint64_t q = t[0] * m.n0;
+    s = (u128)q * m.p[0] + t[0];
+    c = (uint64_t)(s >> 64);
+    for (int j = 1; j < 4; j++) {
+      s = (u128)q * m.p[j] + t[j] + c;
+      t[j - 1] = (uint64_t)s;
+      c = (uint64_t)(s >> 64);
+    }
+    s = (u128)t[4] + c;
+    t[3] = (uint64_t)s;
+    t[4] = t[5] + (uint64_t)(s >> 64);
   }
-  add4(r, r, t + 4);
-  return fe_cond_sub(m, r);
+  Fe r{{t[0], t[1], t[2], t[3]}};
+  if (t[4] || geq(r.v, m.p)) sub4(r.v, r.v, m.p);
+  return r;
 }
 inline Fe fe_sqr(const Mod& m, const Fe& a) { return fe_mul(m, a, a); }
 inline Fe fe_to_mont(const Mod& m, const Fe& a) {
@@ -227,21 +156,10 @@ struct Fq2Ops {
   static T add(const T& a, const T& b) { return {fe_add(FQ, a.c0, b.c0), fe_add(FQ, a.c1, b.c1)}; }
   static T sub(const T& a, const T& b) { return {fe_sub(FQ, a.c0, b.c0), fe_sub(FQ, a.c1, b.c1)}; }
   static T neg(const T& a) { return {fe_neg(FQ, a.c0), fe_neg(FQ, a.c1)}; }
-  // Karatsuba on unreduced sums with two reductions; c0 = a0 b0 - a1 b1 takes p 2^256 back when it
-  // goes below zero
   static T mul(const T& a, const T& b) {
-    uint64_t t0[8], t1[8], t2[8], sa[4], sb[4];
-    fe_wide(t0, a.c0.v, b.c0.v);
-    fe_wide(t1, a.c1.v, b.c1.v);
-    add4(sa, a.c0.v, a.c1.v);
-    add4(sb, b.c0.v, b.c1.v);
-    fe_wide(t2, sa, sb);
-    fe_wide_sub(t2, t0);
-    fe_wide_sub(t2, t1);
-    const uint64_t mask = 0 - fe_wide_sub(t0, t1);
-    const uint64_t pm[4] = {FQ.p[0] & mask, FQ.p[1] & mask, FQ.p[2] & mask, FQ.p[3] & mask};
-    add4(t0 + 4, t0 + 4, pm);
-    return {fe_wide_redc(FQ, t0), fe_wide_redc(FQ, t2)};
+    Fe t0 = fe_mul(FQ, a.c0, b.c0), t1 = fe_mul(FQ, a.c1, b.c1);
+    Fe t2 = fe_mul(FQ, fe_add(FQ, a.c0, a.c1), fe_add(FQ, b.c0, b.c1));
+    return {fe_sub(FQ, t0, t1), fe_sub(FQ, fe_sub(FQ, t2, t0), t1)};
   }
   static T sqr(const T& a) {
     return {fe_mul(FQ, fe_add(FQ, a.c0, a.c1), fe_sub(FQ, a.c0, a.c1)), fe_mul(FQ, fe_dbl(FQ, a.c0), a.c1)};

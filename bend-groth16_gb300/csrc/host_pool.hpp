@@ -37,17 +37,17 @@ class HostPool {
     auto job = std::make_shared<Job>();
     job->n = n;
     job->f = &f;
+    job->pending = helpers;
     {
       std::lock_guard<std::mutex> lk(mu_);
       for (unsigned h = 0; h < helpers; h++) queue_.push_back(job);
     }
     cv_.notify_all();
     job->run();
-    // Wait for the indices that helpers took, not for the helpers: one that wakes after the last
-    // index is taken (tens of microseconds later, longer than a small MSM's whole window sum)
-    // finds none left, so it never reads `f`, which lives in the caller's frame.
+    // helpers that start after the indices are gone return at once; wait for all of them
+    // (they read `f`, which lives in the caller's frame)
     std::unique_lock<std::mutex> lk(job->mu);
-    job->cv.wait(lk, [&] { return job->done == n; });
+    job->cv.wait(lk, [&] { return job->pending == 0; });
     if (job->error) std::rethrow_exception(job->error);
   }
 
@@ -65,25 +65,18 @@ class HostPool {
     int n = 0;
     const std::function<void(int)>* f = nullptr;
     std::atomic<int> next{0};
-    int done = 0;  // indices finished (guarded by mu)
+    unsigned pending = 0;  // helper runs not finished yet (guarded by mu)
     std::exception_ptr error;
     std::mutex mu;
     std::condition_variable cv;
     void run() {
-      int mine = 0;
-      std::exception_ptr err;
-      for (int i; (i = next.fetch_add(1)) < n; mine++) {
-        try {
-          if (!err) (*f)(i);
-        } catch (...) {
-          err = std::current_exception();
-        }
+      try {
+        for (int i; (i = next.fetch_add(1)) < n;) (*f)(i);
+      } catch (...) {
+        std::lock_guard<std::mutex> lk(mu);
+        if (!error) error = std::current_exception();
+        next.store(n);
       }
-      if (mine == 0) return;
-      std::lock_guard<std::mutex> lk(mu);
-      if (err && !error) error = err;
-      done += mine;
-      if (done == n) cv.notify_all();
     }
   };
 
@@ -102,6 +95,11 @@ class HostPool {
         queue_.pop_front();
       }
       job->run();
+      {
+        std::lock_guard<std::mutex> lk(job->mu);
+        job->pending--;
+      }
+      job->cv.notify_all();
     }
   }
 

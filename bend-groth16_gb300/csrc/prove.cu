@@ -247,12 +247,14 @@ static void upload_csr(Ctx& ctx, const void* src, uint32_t nc, CsrDev& out, cuda
   }
 }
 
-// waits for `st` and raises what its kernels reported (the status word is pinned host memory)
 void check_status(Ctx& ctx, cudaStream_t st) {
+  uint32_t s = 0;
+  BG_CUDA(cudaMemcpyAsync(&s, ctx.d_status, 4, cudaMemcpyDeviceToHost, st));
+  ctx.d2h_bytes += 4;
   BG_CUDA(cudaStreamSynchronize(st));
-  const uint32_t s = *static_cast<volatile uint32_t*>(ctx.d_status);
   if (s) {
-    *static_cast<volatile uint32_t*>(ctx.d_status) = 0;
+    BG_CUDA(cudaMemsetAsync(ctx.d_status, 0, 4, st));
+    BG_CUDA(cudaStreamSynchronize(st));
     if (s & BG_DSTATUS_SCALAR_RANGE) throw Error(BG_E_ARG, "an MSM scalar is not below 2^254 (not a canonical Fr)");
     if (s & BG_DSTATUS_FORMAT) throw Error(BG_E_FORMAT, "a wire word has bits above its 16-bit limb");
     if (s & BG_DSTATUS_COLUMN) throw Error(BG_E_FORMAT, "an R1CS column index is outside the assignment");
