@@ -149,7 +149,7 @@ struct Ctx {
   PinnedBuf pinned[4];
   PinnedCache host_cache;
   std::string last_error;
-  uint32_t* d_status = nullptr;           // device-side error flags (see BG_DSTATUS_*)
+  uint32_t* d_status = nullptr;           // error flags kernels set (BG_DSTATUS_*), in pinned host memory
   uint64_t h2d_bytes = 0, d2h_bytes = 0;  // host <-> device bytes this context has copied
   // window widths forced for tuning (bg_msm_window_override): [0] per-window bucket sets,
   // [1] window tables of keys uploaded afterwards; [curve]; 0 = the library's choice

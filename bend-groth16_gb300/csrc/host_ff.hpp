@@ -18,8 +18,18 @@ struct Mod {
   uint64_t r2[4];   // R^2 mod p
 };
 
-extern const Mod FQ;
-extern const Mod FR;
+// p from bend2/src/fq.bend:2 and bend2/src/fr.bend:2; compile-time constants, so every product
+// below is built for its modulus
+inline constexpr Mod FQ = {
+    {0x3c208c16d87cfd47ull, 0x97816a916871ca8dull, 0xb85045b68181585dull, 0x30644e72e131a029ull},
+    0x87d20782e4866389ull,
+    {0xd35d438dc58f0d9dull, 0x0a78eb28f5c70b3dull, 0x666ea36f7879462cull, 0x0e0a77c19a07df2full},
+    {0xf32cfc5b538afa89ull, 0xb5e71911d44501fbull, 0x47ab1eff0a417ff6ull, 0x06d89f71cab8351full}};
+inline constexpr Mod FR = {
+    {0x43e1f593f0000001ull, 0x2833e84879b97091ull, 0xb85045b68181585dull, 0x30644e72e131a029ull},
+    0xc2e1f593efffffffull,
+    {0xac96341c4ffffffbull, 0x36fc76959f60cd29ull, 0x666ea36f7879462eull, 0x0e0a77c19a07df2full},
+    {0x1bb8e645ae216da7ull, 0x53fe3ab1e35c59e3ull, 0x8c49833d53bb8085ull, 0x0216d0b17f4e44a5ull}};
 
 struct Fe {
   uint64_t v[4];
@@ -41,66 +51,127 @@ inline bool geq(const uint64_t* a, const uint64_t* b) {
   return true;
 }
 inline uint64_t sub4(uint64_t* r, const uint64_t* a, const uint64_t* b) {
-  uint64_t borrow = 0;
-  for (int i = 0; i < 4; i++) {
-    u128 d = (u128)a[i] - b[i] - borrow;
-    r[i] = (uint64_t)d;
-    borrow = (uint64_t)(d >> 64) & 1;
-  }
-  return borrow;
+  u128 d = (u128)a[0] - b[0];
+  r[0] = (uint64_t)d;
+  d = (u128)a[1] - b[1] - ((uint64_t)(d >> 64) & 1);
+  r[1] = (uint64_t)d;
+  d = (u128)a[2] - b[2] - ((uint64_t)(d >> 64) & 1);
+  r[2] = (uint64_t)d;
+  d = (u128)a[3] - b[3] - ((uint64_t)(d >> 64) & 1);
+  r[3] = (uint64_t)d;
+  return (uint64_t)(d >> 64) & 1;
 }
 inline uint64_t add4(uint64_t* r, const uint64_t* a, const uint64_t* b) {
-  uint64_t c = 0;
-  for (int i = 0; i < 4; i++) {
-    u128 s = (u128)a[i] + b[i] + c;
-    r[i] = (uint64_t)s;
-    c = (uint64_t)(s >> 64);
-  }
-  return c;
+  u128 s = (u128)a[0] + b[0];
+  r[0] = (uint64_t)s;
+  s = (u128)a[1] + b[1] + (uint64_t)(s >> 64);
+  r[1] = (uint64_t)s;
+  s = (u128)a[2] + b[2] + (uint64_t)(s >> 64);
+  r[2] = (uint64_t)s;
+  s = (u128)a[3] + b[3] + (uint64_t)(s >> 64);
+  r[3] = (uint64_t)s;
+  return (uint64_t)(s >> 64);
+}
+// r = t - p when t >= p, else t (t < 2p), without a branch
+inline Fe fe_cond_sub(const Mod& m, const uint64_t* t) {
+  uint64_t d[4];
+  const uint64_t keep = 0 - sub4(d, t, m.p);  // all ones when t < p
+  Fe r;
+  for (int i = 0; i < 4; i++) r.v[i] = d[i] ^ ((d[i] ^ t[i]) & keep);
+  return r;
 }
 
 inline Fe fe_add(const Mod& m, const Fe& a, const Fe& b) {
-  Fe r;
-  add4(r.v, a.v, b.v);  // < 2p < 2^255, no carry out
-  if (geq(r.v, m.p)) sub4(r.v, r.v, m.p);
-  return r;
+  uint64_t t[4];
+  add4(t, a.v, b.v);  // < 2p < 2^255, no carry out
+  return fe_cond_sub(m, t);
 }
 inline Fe fe_sub(const Mod& m, const Fe& a, const Fe& b) {
   Fe r;
-  if (sub4(r.v, a.v, b.v)) add4(r.v, r.v, m.p);
+  const uint64_t mask = 0 - sub4(r.v, a.v, b.v);
+  const uint64_t pm[4] = {m.p[0] & mask, m.p[1] & mask, m.p[2] & mask, m.p[3] & mask};
+  add4(r.v, r.v, pm);
   return r;
 }
 inline Fe fe_neg(const Mod& m, const Fe& a) { return fe_sub(m, fe_zero(), a); }
 inline Fe fe_dbl(const Mod& m, const Fe& a) { return fe_add(m, a, a); }
 
-// CIOS Montgomery product a*b*2^-256 mod p
-inline Fe fe_mul(const Mod& m, const Fe& a, const Fe& b) {
-  uint64_t t[6] = {0, 0, 0, 0, 0, 0};
-  for (int i = 0; i < 4; i++) {
-    uint64_t c = 0;
-    for (int j = 0; j < 4; j++) {
-      u128 s = (u128)a.v[j] * b.v[i] + t[j] + c;
-      t[j] = (uint64_t)s;
-      c = (uint64_t)(s >> 64);
-    }
-    u128 s = (u128)t[4] + c;
-    t[4] = (uint64_t)s;
-    t[5] = (uint64_t)(s >> 64);
-    const uint64_t q = t[0] * m.n0;
-    s = (u128)q * m.p[0] + t[0];
-    c = (uint64_t)(s >> 64);
-    for (int j = 1; j < 4; j++) {
-      s = (u128)q * m.p[j] + t[j] + c;
-      t[j - 1] = (uint64_t)s;
-      c = (uint64_t)(s >> 64);
-    }
-    s = (u128)t[4] + c;
-    t[3] = (uint64_t)s;
-    t[4] = t[5] + (uint64_t)(s >> 64);
+// Row b of a CIOS Montgomery product: t = (t + a b + q p) / 2^64 with the q that clears limb 0.
+// For a < p < 2^254 the sum stays below 2p after every row, so four limbs hold it and the two
+// carry words can be added without overflow.
+inline __attribute__((always_inline)) void fe_mul_row(const Mod& m, uint64_t* t, const uint64_t* a, uint64_t b) {
+  u128 s = (u128)a[0] * b + t[0];
+  const uint64_t q = (uint64_t)s * m.n0;
+  uint64_t c = (uint64_t)(s >> 64);
+  u128 u = (u128)q * m.p[0] + (uint64_t)s;
+  s = (u128)a[1] * b + t[1] + c;
+  c = (uint64_t)(s >> 64);
+  u = (u128)q * m.p[1] + (uint64_t)s + (uint64_t)(u >> 64);
+  t[0] = (uint64_t)u;
+  s = (u128)a[2] * b + t[2] + c;
+  c = (uint64_t)(s >> 64);
+  u = (u128)q * m.p[2] + (uint64_t)s + (uint64_t)(u >> 64);
+  t[1] = (uint64_t)u;
+  s = (u128)a[3] * b + t[3] + c;
+  c = (uint64_t)(s >> 64);
+  u = (u128)q * m.p[3] + (uint64_t)s + (uint64_t)(u >> 64);
+  t[2] = (uint64_t)u;
+  t[3] = (uint64_t)(u >> 64) + c;
+}
+// a b 2^-256 mod p for a < p and any 256-bit b
+inline __attribute__((always_inline)) Fe fe_mul(const Mod& m, const Fe& a, const Fe& b) {
+  uint64_t t[4] = {0, 0, 0, 0};
+  fe_mul_row(m, t, a.v, b.v[0]);
+  fe_mul_row(m, t, a.v, b.v[1]);
+  fe_mul_row(m, t, a.v, b.v[2]);
+  fe_mul_row(m, t, a.v, b.v[3]);
+  return fe_cond_sub(m, t);
+}
+// t = a b (512 bits)
+inline __attribute__((always_inline)) void fe_wide_row(uint64_t* t, const uint64_t* a, uint64_t b) {
+  u128 s = (u128)a[0] * b + t[0];
+  t[0] = (uint64_t)s;
+  s = (u128)a[1] * b + t[1] + (uint64_t)(s >> 64);
+  t[1] = (uint64_t)s;
+  s = (u128)a[2] * b + t[2] + (uint64_t)(s >> 64);
+  t[2] = (uint64_t)s;
+  s = (u128)a[3] * b + t[3] + (uint64_t)(s >> 64);
+  t[3] = (uint64_t)s;
+  t[4] = (uint64_t)(s >> 64);
+}
+inline __attribute__((always_inline)) void fe_wide(uint64_t* t, const uint64_t* a, const uint64_t* b) {
+  t[0] = t[1] = t[2] = t[3] = 0;
+  fe_wide_row(t, a, b[0]);
+  fe_wide_row(t + 1, a, b[1]);
+  fe_wide_row(t + 2, a, b[2]);
+  fe_wide_row(t + 3, a, b[3]);
+}
+// t -= u (512 bits), returns the borrow
+inline __attribute__((always_inline)) uint64_t fe_wide_sub(uint64_t* t, const uint64_t* u) {
+  uint64_t borrow = 0;
+  for (int i = 0; i < 8; i++) {
+    const u128 d = (u128)t[i] - u[i] - borrow;
+    t[i] = (uint64_t)d;
+    borrow = (uint64_t)(d >> 64) & 1;
   }
-  Fe r{{t[0], t[1], t[2], t[3]}};
-  if (t[4] || geq(r.v, m.p)) sub4(r.v, r.v, m.p);
-  return r;
+  return borrow;
+}
+// t 2^-256 mod p for t < p 2^256: the low half reduced alone (at most p) plus the high half
+inline __attribute__((always_inline)) Fe fe_wide_redc(const Mod& m, const uint64_t* t) {
+  uint64_t r[4] = {t[0], t[1], t[2], t[3]};
+  for (int i = 0; i < 4; i++) {
+    const uint64_t q = r[0] * m.n0;
+    u128 u = (u128)q * m.p[0] + r[0];
+    u = (u128)q * m.p[1] + r[1] + (uint64_t)(u >> 64);
+    r[0] = (uint64_t)u;
+    u = (u128)q * m.p[2] + r[2] + (uint64_t)(u >> 64);
+    r[1] = (uint64_t)u;
+    u = (u128)q * m.p[3] + r[3] + (uint64_t)(u >> 64);
+    r[2] = (uint64_t)u;
+    r[3] = (uint64_t)(u >> 64);
+  }
+  add4(r, r, t + 4);
+  return fe_cond_sub(m, r);
 }
 inline Fe fe_sqr(const Mod& m, const Fe& a) { return fe_mul(m, a, a); }
 inline Fe fe_to_mont(const Mod& m, const Fe& a) {
@@ -121,10 +192,95 @@ inline Fe fe_pow_u64(const Mod& m, const Fe& a, uint64_t e) {
   const uint64_t ee[4] = {e, 0, 0, 0};
   return fe_pow(m, a, ee);
 }
-// 1/a (Fermat); 0 -> 0
+// 1/a for a Montgomery element below p (0 -> 0): Bernstein and Yang's division steps, as the
+// device's inversion (fp.cuh), 62 steps to a matrix and five signed 62-bit limbs.  2 us against the
+// Fermat power's 8; a proof's host tail makes three, a standalone MSM's one.
+namespace dsteps {
+constexpr int64_t kMask = ((int64_t)1 << 62) - 1;
+struct S62 {
+  int64_t v[5];
+};
+inline S62 split(const uint64_t* w) {
+  return {{(int64_t)(w[0] & kMask), (int64_t)((w[0] >> 62 | w[1] << 2) & kMask), (int64_t)((w[1] >> 60 | w[2] << 4) & kMask),
+           (int64_t)((w[2] >> 58 | w[3] << 6) & kMask), (int64_t)(w[3] >> 56)}};
+}
+inline int64_t steps62(int64_t eta, uint64_t f, uint64_t g, int64_t* m) {
+  uint64_t u = 1, v = 0, q = 0, r = 1;
+  for (int i = 0; i < 62; i++) {
+    uint64_t c1 = (uint64_t)(eta >> 63);  // delta > 0
+    const uint64_t c2 = 0 - (g & 1);
+    const uint64_t x = (f ^ c1) - c1, y = (u ^ c1) - c1, z = (v ^ c1) - c1;
+    g += x & c2;
+    q += y & c2;
+    r += z & c2;
+    c1 &= c2;
+    eta = (int64_t)(((uint64_t)eta ^ c1) - 1);
+    f += g & c1;
+    u += q & c1;
+    v += r & c1;
+    g >>= 1;
+    u <<= 1;
+    v <<= 1;
+  }
+  m[0] = (int64_t)u;
+  m[1] = (int64_t)v;
+  m[2] = (int64_t)q;
+  m[3] = (int64_t)r;
+  return eta;
+}
+// (a, b) = (m0 a + m1 b + k p, m2 a + m3 b + l p) / 2^62 with the k, l (n62 = -p^-1 mod 2^62) that make
+// them whole, centred; without p (n62 = 0) for the pair that is divisible by itself
+inline void apply(S62& a, S62& b, const int64_t* m, const S62& p, uint64_t n62) {
+  typedef __int128 i128;
+  i128 ca = (i128)m[0] * a.v[0] + (i128)m[1] * b.v[0], cb = (i128)m[2] * a.v[0] + (i128)m[3] * b.v[0];
+  const int64_t k = (int64_t)(((uint64_t)ca * n62) << 2) >> 2, l = (int64_t)(((uint64_t)cb * n62) << 2) >> 2;
+  ca = (ca + (i128)k * p.v[0]) >> 62;
+  cb = (cb + (i128)l * p.v[0]) >> 62;
+  for (int i = 1; i < 5; i++) {
+    const int64_t ai = a.v[i], bi = b.v[i];
+    ca += (i128)m[0] * ai + (i128)m[1] * bi + (i128)k * p.v[i];
+    cb += (i128)m[2] * ai + (i128)m[3] * bi + (i128)l * p.v[i];
+    a.v[i - 1] = (int64_t)ca & kMask;
+    b.v[i - 1] = (int64_t)cb & kMask;
+    ca >>= 62;
+    cb >>= 62;
+  }
+  a.v[4] = (int64_t)ca;
+  b.v[4] = (int64_t)cb;
+}
+}  // namespace dsteps
 inline Fe fe_inv(const Mod& m, const Fe& a) {
-  uint64_t e[4] = {m.p[0] - 2, m.p[1], m.p[2], m.p[3]};
-  return fe_pow(m, a, e);
+  using dsteps::S62;
+  const S62 p = dsteps::split(m.p);
+  S62 f = p, g = dsteps::split(a.v), d = {{0, 0, 0, 0, 0}}, e = dsteps::split(m.r2);
+  int64_t eta = -1, mat[4];
+  for (int i = 0; i < 10; i++) {  // 620 steps, of which 590 suffice
+    eta = dsteps::steps62(eta, (uint64_t)f.v[0] | (uint64_t)f.v[1] << 62, (uint64_t)g.v[0] | (uint64_t)g.v[1] << 62, mat);
+    dsteps::apply(d, e, mat, p, m.n0 & (uint64_t)dsteps::kMask);
+    dsteps::apply(f, g, mat, p, 0);
+    if ((g.v[0] | g.v[1] | g.v[2] | g.v[3] | g.v[4]) == 0) break;
+  }
+  // f = +-1 and |d| <= (1/2 + 10/2) p: d f + 6 p lies in (0, 12 p), below 2^258
+  const int64_t sign = f.v[4] >> 63;
+  __int128 c = 0;
+  uint64_t t[5];
+  for (int i = 0; i < 5; i++) {
+    c += (__int128)((d.v[i] ^ sign) - sign) + (__int128)6 * p.v[i];
+    t[i] = (uint64_t)c & (uint64_t)dsteps::kMask;
+    c >>= 62;
+  }
+  for (int k = 3; k >= 0; k--) {  // minus 8 p, 4 p, 2 p, p where they fit
+    uint64_t s[5];
+    __int128 bw = 0;
+    for (int i = 0; i < 5; i++) {
+      bw += (__int128)t[i] - ((__int128)p.v[i] << k);
+      s[i] = (uint64_t)bw & (uint64_t)dsteps::kMask;
+      bw >>= 62;
+    }
+    if (bw >= 0)
+      for (int i = 0; i < 5; i++) t[i] = s[i];
+  }
+  return Fe{{t[0] | t[1] << 62, t[1] >> 2 | t[2] << 60, t[2] >> 4 | t[3] << 58, t[3] >> 6 | t[4] << 56}};
 }
 
 // ---------------------------------------------------------------- Fq2 = Fq[u]/(u^2+1)
@@ -156,10 +312,21 @@ struct Fq2Ops {
   static T add(const T& a, const T& b) { return {fe_add(FQ, a.c0, b.c0), fe_add(FQ, a.c1, b.c1)}; }
   static T sub(const T& a, const T& b) { return {fe_sub(FQ, a.c0, b.c0), fe_sub(FQ, a.c1, b.c1)}; }
   static T neg(const T& a) { return {fe_neg(FQ, a.c0), fe_neg(FQ, a.c1)}; }
+  // Karatsuba on unreduced sums with two reductions; c0 = a0 b0 - a1 b1 takes p 2^256 back when it
+  // goes below zero
   static T mul(const T& a, const T& b) {
-    Fe t0 = fe_mul(FQ, a.c0, b.c0), t1 = fe_mul(FQ, a.c1, b.c1);
-    Fe t2 = fe_mul(FQ, fe_add(FQ, a.c0, a.c1), fe_add(FQ, b.c0, b.c1));
-    return {fe_sub(FQ, t0, t1), fe_sub(FQ, fe_sub(FQ, t2, t0), t1)};
+    uint64_t t0[8], t1[8], t2[8], sa[4], sb[4];
+    fe_wide(t0, a.c0.v, b.c0.v);
+    fe_wide(t1, a.c1.v, b.c1.v);
+    add4(sa, a.c0.v, a.c1.v);
+    add4(sb, b.c0.v, b.c1.v);
+    fe_wide(t2, sa, sb);
+    fe_wide_sub(t2, t0);
+    fe_wide_sub(t2, t1);
+    const uint64_t mask = 0 - fe_wide_sub(t0, t1);
+    const uint64_t pm[4] = {FQ.p[0] & mask, FQ.p[1] & mask, FQ.p[2] & mask, FQ.p[3] & mask};
+    add4(t0 + 4, t0 + 4, pm);
+    return {fe_wide_redc(FQ, t0), fe_wide_redc(FQ, t2)};
   }
   static T sqr(const T& a) {
     return {fe_mul(FQ, fe_add(FQ, a.c0, a.c1), fe_sub(FQ, a.c0, a.c1)), fe_mul(FQ, fe_dbl(FQ, a.c0), a.c1)};
@@ -237,6 +404,56 @@ Xyzz<F> xyzz_add(const Xyzz<F>& p, const Xyzz<F>& q) {
   r.zz = F::mul(F::mul(p.zz, q.zz), pp);
   r.zzz = F::mul(F::mul(p.zzz, q.zzz), ppp);
   return r;
+}
+// Jacobian points (x = X / Z^2, y = Y / Z^3) for the Horner chain of an MSM, most of whose steps are
+// doublings: dbl-2009-l takes 2 products and 5 squares where the XYZZ doubling takes 6 and 3.
+template <class F>
+struct Jac {
+  typename F::T x, y, z;
+};
+template <class F>
+Jac<F> jac_inf() {
+  return {F::one(), F::one(), F::zero()};
+}
+template <class F>
+Jac<F> jac_dbl(const Jac<F>& p) {
+  if (F::is_zero(p.z)) return p;
+  const auto a = F::sqr(p.x), b = F::sqr(p.y), c = F::sqr(b);
+  auto d = F::sub(F::sub(F::sqr(F::add(p.x, b)), a), c);
+  d = F::add(d, d);
+  const auto e = F::add(F::add(a, a), a);
+  Jac<F> r;
+  r.x = F::sub(F::sqr(e), F::add(d, d));
+  auto c8 = F::add(c, c);
+  c8 = F::add(c8, c8);
+  c8 = F::add(c8, c8);
+  r.y = F::sub(F::mul(e, F::sub(d, r.x)), c8);
+  const auto yz = F::mul(p.y, p.z);
+  r.z = F::add(yz, yz);
+  return r;
+}
+// p + q for Jacobian p and XYZZ q (x = X / ZZ, y = Y / ZZZ): q with Z = ZZZ is (X ZZ^2, Y ZZZ^2, ZZZ)
+template <class F>
+Jac<F> jac_add(const Jac<F>& p, const Xyzz<F>& q) {
+  if (F::is_zero(q.zz)) return p;
+  const auto qz2 = F::sqr(q.zzz), qx = F::mul(q.x, F::sqr(q.zz)), qy = F::mul(q.y, qz2);
+  if (F::is_zero(p.z)) return {qx, qy, q.zzz};
+  const auto pz2 = F::sqr(p.z);
+  const auto u1 = F::mul(p.x, qz2), u2 = F::mul(qx, pz2);
+  const auto s1 = F::mul(p.y, F::mul(q.zzz, qz2)), s2 = F::mul(qy, F::mul(p.z, pz2));
+  const auto h = F::sub(u2, u1), r_ = F::sub(s2, s1);
+  if (F::is_zero(h)) return F::is_zero(r_) ? jac_dbl(p) : jac_inf<F>();
+  const auto hh = F::sqr(h), hhh = F::mul(h, hh), v = F::mul(u1, hh);
+  Jac<F> r;
+  r.x = F::sub(F::sub(F::sqr(r_), hhh), F::add(v, v));
+  r.y = F::sub(F::mul(r_, F::sub(v, r.x)), F::mul(s1, hhh));
+  r.z = F::mul(F::mul(p.z, q.zzz), h);
+  return r;
+}
+template <class F>
+Xyzz<F> xyzz_from_jac(const Jac<F>& p) {
+  const auto zz = F::sqr(p.z);
+  return {p.x, p.y, zz, F::mul(zz, p.z)};
 }
 template <class F>
 Xyzz<F> xyzz_neg(const Xyzz<F>& p) {

@@ -27,28 +27,22 @@ class HostPool {
 
   unsigned workers() const { return (unsigned)threads_.size(); }
 
+  // f(0..n-1), begun on idle workers while the caller goes on; wait() runs what no worker has taken
+  // and returns when all are done.  The handle waits when it goes out of scope.
+  class Task;
+  Task start(int n, std::function<void(int)> f);
+
   void parallel_for(int n, const std::function<void(int)>& f) {
     if (n <= 0) return;
-    const unsigned helpers = std::min<unsigned>(workers(), (unsigned)n - 1u);
-    if (helpers == 0) {
+    if (n == 1 || workers() == 0) {
       for (int i = 0; i < n; i++) f(i);
       return;
     }
     auto job = std::make_shared<Job>();
     job->n = n;
-    job->f = &f;
-    job->pending = helpers;
-    {
-      std::lock_guard<std::mutex> lk(mu_);
-      for (unsigned h = 0; h < helpers; h++) queue_.push_back(job);
-    }
-    cv_.notify_all();
-    job->run();
-    // helpers that start after the indices are gone return at once; wait for all of them
-    // (they read `f`, which lives in the caller's frame)
-    std::unique_lock<std::mutex> lk(job->mu);
-    job->cv.wait(lk, [&] { return job->pending == 0; });
-    if (job->error) std::rethrow_exception(job->error);
+    job->f = f;
+    submit(job, std::min<unsigned>(workers(), (unsigned)n - 1u));
+    job->finish();
   }
 
   ~HostPool() {
@@ -63,22 +57,46 @@ class HostPool {
  private:
   struct Job {
     int n = 0;
-    const std::function<void(int)>* f = nullptr;
+    std::function<void(int)> f;
     std::atomic<int> next{0};
-    unsigned pending = 0;  // helper runs not finished yet (guarded by mu)
+    int done = 0;  // indices finished (guarded by mu)
     std::exception_ptr error;
     std::mutex mu;
     std::condition_variable cv;
     void run() {
-      try {
-        for (int i; (i = next.fetch_add(1)) < n;) (*f)(i);
-      } catch (...) {
-        std::lock_guard<std::mutex> lk(mu);
-        if (!error) error = std::current_exception();
-        next.store(n);
+      int mine = 0;
+      std::exception_ptr err;
+      for (int i; (i = next.fetch_add(1)) < n; mine++) {
+        try {
+          if (!err) f(i);
+        } catch (...) {
+          err = std::current_exception();
+        }
       }
+      if (mine == 0) return;
+      std::lock_guard<std::mutex> lk(mu);
+      if (err && !error) error = err;
+      done += mine;
+      if (done == n) cv.notify_all();
+    }
+    // Waits for the indices that helpers took, not for the helpers: one that wakes after the last
+    // index is taken (tens of microseconds later, longer than a small MSM's whole window sum) finds
+    // none left.
+    void finish() {
+      run();
+      std::unique_lock<std::mutex> lk(mu);
+      cv.wait(lk, [&] { return done == n; });
+      if (error) std::rethrow_exception(error);
     }
   };
+  void submit(const std::shared_ptr<Job>& job, unsigned helpers) {
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      for (unsigned h = 0; h < helpers; h++) queue_.push_back(job);
+    }
+    if (helpers == 1) cv_.notify_one();
+    else cv_.notify_all();
+  }
 
   explicit HostPool(unsigned n) {
     for (unsigned i = 0; i < n; i++) threads_.emplace_back([this] { loop(); });
@@ -95,11 +113,6 @@ class HostPool {
         queue_.pop_front();
       }
       job->run();
-      {
-        std::lock_guard<std::mutex> lk(job->mu);
-        job->pending--;
-      }
-      job->cv.notify_all();
     }
   }
 
@@ -109,5 +122,35 @@ class HostPool {
   std::condition_variable cv_;
   bool stop_ = false;
 };
+
+class HostPool::Task {
+ public:
+  Task() = default;
+  explicit Task(std::shared_ptr<Job> j) : job_(std::move(j)) {}
+  Task(Task&&) = default;
+  Task& operator=(Task&&) = default;
+  void wait() {
+    if (!job_) return;
+    const std::shared_ptr<Job> j = std::move(job_);
+    j->finish();
+  }
+  ~Task() {
+    try {
+      wait();  // what it runs refers to the caller's frame
+    } catch (...) {
+    }
+  }
+
+ private:
+  std::shared_ptr<Job> job_;
+};
+
+inline HostPool::Task HostPool::start(int n, std::function<void(int)> f) {
+  auto job = std::make_shared<Job>();
+  job->n = n;
+  job->f = std::move(f);
+  submit(job, std::min<unsigned>(workers(), (unsigned)n));
+  return Task(job);
+}
 
 }  // namespace bg

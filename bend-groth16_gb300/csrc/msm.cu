@@ -1250,13 +1250,16 @@ void msm_fetch(Ctx& ctx, cudaStream_t st, MsmPlan& plan) {
   ctx.d2h_bytes += (uint64_t)plan.W * plan.J * 2 * PW * sizeof(uint32_t);
 }
 
-// Window w = sum_j S_j + span * sum_j j R_j; total = sum_w 2^(o_w) window_w (Horner).
-template <class F>
-void msm_finish(const MsmPlan& plan, uint32_t* out_affine_words32) {
-  typedef typename HostField<F>::T H;
+// Window w = s_w + span u_w with s_w = sum_j S_j and u_w = sum_j j R_j; total = sum_w 2^(o_w)
+// window_w (Horner, span a power of two below the window's: u_w joins log2(span) doublings above
+// s_w, so no window doubles by itself).
+template <class H>
+bgh::Xyzz<H> msm_sum(const MsmPlan& plan) {
   constexpr int PW = 4 * H::WORDS;
-  // window w's sum from its J parts: sum_j S_j + span sum_{j>=1} j R_j (independent per window)
-  std::vector<bgh::Xyzz<H>> wsum(plan.W);
+  int span_log = 0;
+  while ((1u << span_log) < plan.part_span) span_log++;
+  // s_w and u_w from window w's J parts (independent per window)
+  std::vector<bgh::Xyzz<H>> wsum(plan.W), wjr(plan.W, bgh::xyzz_inf<H>());
   auto window_sum = [&](int w) {
     const uint32_t* pw = plan.host_window_sums + (size_t)w * plan.J * 2 * PW;
     bgh::Xyzz<H> s = bgh::xyzz_inf<H>(), run = bgh::xyzz_inf<H>(), jr = bgh::xyzz_inf<H>();
@@ -1267,8 +1270,8 @@ void msm_finish(const MsmPlan& plan, uint32_t* out_affine_words32) {
         jr = bgh::xyzz_add(jr, run);  // sum_{j>=1} j R_j
       }
     }
-    for (uint32_t m = plan.part_span; m > 1; m >>= 1) jr = bgh::xyzz_dbl(jr);
-    wsum[w] = bgh::xyzz_add(s, jr);
+    wsum[w] = s;
+    wjr[w] = jr;
   };
   // One window of many parts (the shared bucket set of a key's window tables, e.g. J = 128 for
   // msm_h of a SquareChain(2^18) proof: ~390 host additions after the proof's last kernel) is
@@ -1303,9 +1306,8 @@ void msm_finish(const MsmPlan& plan, uint32_t* out_affine_words32) {
       }
     }
     for (uint32_t m = C; m > 1; m >>= 1) ctop = bgh::xyzz_dbl(ctop);
-    jr = bgh::xyzz_add(jr, ctop);  // sum_{j>=1} j R_j
-    for (uint32_t m = plan.part_span; m > 1; m >>= 1) jr = bgh::xyzz_dbl(jr);
-    wsum[0] = bgh::xyzz_add(s, jr);
+    wsum[0] = s;
+    wjr[0] = bgh::xyzz_add(jr, ctop);  // sum_{j>=1} j R_j
   };
   // The window sums of a bucket-set-per-window MSM are about two thirds of its host work
   // (17 windows x 8 parts: ~550 of ~850 point operations); they run on the host pool, the
@@ -1313,15 +1315,24 @@ void msm_finish(const MsmPlan& plan, uint32_t* out_affine_words32) {
   // the tail of the proof.
   const bool pow2_parts = plan.J >= 32 && (plan.J & (plan.J - 1)) == 0;
   if (plan.W == 1 && pow2_parts && HostPool::get().workers() > 0) single_window_chunked();
-  else if (plan.W >= 4 && (size_t)plan.W * plan.J >= 32) HostPool::get().parallel_for(plan.W, window_sum);
+  else if (plan.W >= 4 && (size_t)plan.W * (plan.J - 1) >= 64)  // fewer additions take less than the pool's wake-up
+    HostPool::get().parallel_for(plan.W, window_sum);
   else
     for (int w = 0; w < plan.W; w++) window_sum(w);
-  bgh::Xyzz<H> acc = bgh::xyzz_inf<H>();
+  bgh::Jac<H> acc = bgh::jac_inf<H>();
   for (int w = plan.W - 1; w >= 0; w--) {
-    for (int d = 0; d < window_width(w, plan.W); d++) acc = bgh::xyzz_dbl(acc);
-    acc = bgh::xyzz_add(acc, wsum[w]);
+    for (int d = window_width(w, plan.W); d > span_log; d--) acc = bgh::jac_dbl(acc);
+    acc = bgh::jac_add(acc, wjr[w]);
+    for (int d = 0; d < span_log; d++) acc = bgh::jac_dbl(acc);
+    acc = bgh::jac_add(acc, wsum[w]);
   }
-  bgh::aff_to_words32<H>(out_affine_words32, bgh::xyzz_to_affine(acc));
+  return bgh::xyzz_from_jac(acc);
+}
+
+template <class F>
+void msm_finish(const MsmPlan& plan, uint32_t* out_affine_words32) {
+  typedef typename HostField<F>::T H;
+  bgh::aff_to_words32<H>(out_affine_words32, bgh::xyzz_to_affine(msm_sum<H>(plan)));
 }
 
 // Kernel attributes (the opt-in to large dynamic shared memory) apply to the device that is
@@ -1358,6 +1369,8 @@ template void msm_launch<Fq2>(Ctx&, cudaStream_t, const std::string&, const uint
                               MsmPlan&, cudaStream_t, const MsmTable*);
 template void msm_fetch<Fq>(Ctx&, cudaStream_t, MsmPlan&);
 template void msm_fetch<Fq2>(Ctx&, cudaStream_t, MsmPlan&);
+template bgh::Xyzz<bgh::FqOps> msm_sum<bgh::FqOps>(const MsmPlan&);
+template bgh::Xyzz<bgh::Fq2Ops> msm_sum<bgh::Fq2Ops>(const MsmPlan&);
 template void msm_finish<Fq>(const MsmPlan&, uint32_t*);
 template void msm_finish<Fq2>(const MsmPlan&, uint32_t*);
 

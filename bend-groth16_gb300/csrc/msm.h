@@ -4,6 +4,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "host_ff.hpp"
 
 namespace bg {
 
@@ -95,8 +96,11 @@ void msm_accumulate(Ctx& ctx, cudaStream_t st, const std::string& tag, const uin
 // Enqueue the copy of the window sums to the host.
 template <class F>
 void msm_fetch(Ctx& ctx, cudaStream_t st, MsmPlan& plan);
-// After the stream is synchronised: Horner over windows, affine result (packed words,
-// 16 for G1, 32 for G2; all zero = infinity).
+// After the stream is synchronised: the sum, by Horner over the windows (H: bgh::FqOps for G1,
+// bgh::Fq2Ops for G2)
+template <class H>
+bgh::Xyzz<H> msm_sum(const MsmPlan& plan);
+// the same, affine (packed words, 16 for G1, 32 for G2; all zero = infinity)
 template <class F>
 void msm_finish(const MsmPlan& plan, uint32_t* out_affine_words32);
 

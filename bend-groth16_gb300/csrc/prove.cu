@@ -247,14 +247,12 @@ static void upload_csr(Ctx& ctx, const void* src, uint32_t nc, CsrDev& out, cuda
   }
 }
 
+// waits for `st` and raises what its kernels reported (the status word is pinned host memory)
 void check_status(Ctx& ctx, cudaStream_t st) {
-  uint32_t s = 0;
-  BG_CUDA(cudaMemcpyAsync(&s, ctx.d_status, 4, cudaMemcpyDeviceToHost, st));
-  ctx.d2h_bytes += 4;
   BG_CUDA(cudaStreamSynchronize(st));
+  const uint32_t s = *static_cast<volatile uint32_t*>(ctx.d_status);
   if (s) {
-    BG_CUDA(cudaMemsetAsync(ctx.d_status, 0, 4, st));
-    BG_CUDA(cudaStreamSynchronize(st));
+    *static_cast<volatile uint32_t*>(ctx.d_status) = 0;
     if (s & BG_DSTATUS_SCALAR_RANGE) throw Error(BG_E_ARG, "an MSM scalar is not below 2^254 (not a canonical Fr)");
     if (s & BG_DSTATUS_FORMAT) throw Error(BG_E_FORMAT, "a wire word has bits above its 16-bit limb");
     if (s & BG_DSTATUS_COLUMN) throw Error(BG_E_FORMAT, "an R1CS column index is outside the assignment");
@@ -426,6 +424,33 @@ void prove_resident(Ctx& ctx, PkDev& pk, const uint32_t* witness16, const uint32
   cudaStream_t st = ctx.stream;
   Workspace& ws = ctx.ws;
 
+  // ---- host products that need no MSM result, on the host pool while this thread launches.  The
+  // products of the key's delta points by r, s and r s are independent chains of about 320 point
+  // operations; with a resident key each splits into four 64-bit pieces over precomputed
+  // 2^(64 j) delta.
+  uint64_t r[4], s[4], rs[4];
+  scalar_from_mont_wire(rs16, r);
+  scalar_from_mont_wire(rs16 + 16, s);
+  {
+    const Fe rm = bgh::fe_from_words16(rs16), sm = bgh::fe_from_words16(rs16 + 16);
+    const Fe prod = bgh::fe_from_mont(bgh::FR, bgh::fe_mul(bgh::FR, rm, sm));
+    for (int i = 0; i < 4; i++) rs[i] = prod.v[i];
+  }
+  const uint64_t* const ks[3] = {r, s, rs};
+  const int pieces = pk.delta_pow_ready ? 4 : 1;
+  Xyzz<FqOps> piece[3][4];
+  Xyzz<Fq2Ops> piece2[4];
+  HostPool::Task products = HostPool::get().start(4 * pieces, [&](int t) {
+    const int j = t % pieces, m = t / pieces;  // the G2 pieces first: they are the longest
+    if (pieces == 4) {
+      if (m == 0) piece2[j] = bgh::xyzz_mul64(pk.delta2_pow[j], s[j]);
+      else piece[m - 1][j] = bgh::xyzz_mul64(pk.delta_pow[j], ks[m - 1][j]);
+    } else {
+      if (m == 0) piece2[0] = bgh::xyzz_mul(bgh::xyzz_from(pk.delta2), s);
+      else piece[m - 1][0] = bgh::xyzz_mul(bgh::xyzz_from(pk.delta), ks[m - 1]);
+    }
+  });
+
   // ---- load: witness to the device
   Timer t_load, t_evals, t_qap, t_msm[5];
   t_load.start(st);
@@ -564,86 +589,71 @@ void prove_resident(Ctx& ctx, PkDev& pk, const uint32_t* witness16, const uint32
   BG_CUDA(cudaStreamWaitEvent(st, ev_sorted, 0));
   launch(4, sort_for(jobs[4], st));
 
-  // ---- host work that needs no MSM result, overlapped with the device
-  uint64_t r[4], s[4], rs[4];
-  scalar_from_mont_wire(rs16, r);
-  scalar_from_mont_wire(rs16 + 16, s);
-  {
-    const Fe rm = bgh::fe_from_words16(rs16), sm = bgh::fe_from_words16(rs16 + 16);
-    const Fe prod = bgh::fe_from_mont(bgh::FR, bgh::fe_mul(bgh::FR, rm, sm));
-    for (int i = 0; i < 4; i++) rs[i] = prod.v[i];
-  }
-  // The four products of the key's delta points by r, s and r s are independent chains of
-  // about 320 host point operations (146 us in G1, 404 us in G2 on one core): they run at once
-  // on the host pool, and with a resident key each splits into four 64-bit pieces over
-  // precomputed 2^(64 j) delta.  A small proof's device work is shorter than them one after
-  // another (SquareChain(2^10): kernels end about 0.63 ms into the proof).
-  const Xyzz<FqOps> dj = bgh::xyzz_from(pk.delta);
-  const Xyzz<Fq2Ops> dj2 = bgh::xyzz_from(pk.delta2);
-  Xyzz<FqOps> r_delta, s_delta, rs_delta;
-  Xyzz<Fq2Ops> s_delta2;
-  if (pk.delta_pow_ready) {
-    // resident key: each product is four 64-bit pieces k_j (2^(64 j) delta), 16 tasks
-    Xyzz<FqOps> piece[3][4];
-    Xyzz<Fq2Ops> piece2[4];
-    const uint64_t* ks[3] = {r, s, rs};
-    HostPool::get().parallel_for(16, [&](int t) {
-      const int j = t & 3, m = t >> 2;  // the four G2 pieces first: they are the longest
-      if (m == 0) piece2[j] = bgh::xyzz_mul64(pk.delta2_pow[j], s[j]);
-      else piece[m - 1][j] = bgh::xyzz_mul64(pk.delta_pow[j], ks[m - 1][j]);
-    });
-    Xyzz<FqOps>* out[3] = {&r_delta, &s_delta, &rs_delta};
-    for (int m = 0; m < 3; m++)
-      *out[m] = bgh::xyzz_add(bgh::xyzz_add(piece[m][0], piece[m][1]), bgh::xyzz_add(piece[m][2], piece[m][3]));
-    s_delta2 = bgh::xyzz_add(bgh::xyzz_add(piece2[0], piece2[1]), bgh::xyzz_add(piece2[2], piece2[3]));
-  } else {
-    HostPool::get().parallel_for(4, [&](int i) {
-      if (i == 0) s_delta2 = bgh::xyzz_mul(dj2, s);
-      else if (i == 1) r_delta = bgh::xyzz_mul(dj, r);
-      else if (i == 2) s_delta = bgh::xyzz_mul(dj, s);
-      else rs_delta = bgh::xyzz_mul(dj, rs);
-    });
-  }
-
-  // ---- finish each MSM on the host as soon as its reduction stream drains (accumulation order
-  // a, b1, b2, l, h); everything that does not need msm_h -- A, B1, B2 and s A + r B1 - r s delta
-  // + mL -- is computed while msm_h is still on the device.  Combine (groth16.bend:298-308):
-  // A = alpha + mA + r delta; B1 = beta + mB1 + s delta; B2 = beta2 + mB2 + s delta2;
-  // C = s A + r B1 - r s delta + (mL + mH)
-  auto g1 = [](const uint32_t* w) { return bgh::xyzz_from(bgh::aff_from_words32<FqOps>(w)); };
-  uint32_t res[5][32];
+  // ---- finish each MSM on the host when its reduction stream drains.  Combine
+  // (groth16.bend:298-308): A = alpha + mA + r delta; B1 = beta + mB1 + s delta; B2 = beta2 + mB2 +
+  // s delta2; C = s A + r B1 - r s delta + (mL + mH).  s A and r B1 are chains of 90 us, mB2's sum up
+  // to 140: a proof that has the GPU to itself hands each MSM's part to the pool as it drains, in
+  // whatever order, and this thread takes msm_h; one after another they were the longer half of a
+  // small proof (SquareChain(2^10): 430 of 600 us).  A lane of a batch or a server shares the pool
+  // with others and takes them in turn.
+  products.wait();
+  auto total = [&](auto* q) {
+    auto t = q[0];
+    for (int j = 1; j < pieces; j++) t = bgh::xyzz_add(t, q[j]);
+    return t;
+  };
+  const Xyzz<FqOps> r_delta = total(piece[0]), s_delta = total(piece[1]), rs_delta = total(piece[2]);
+  const Xyzz<Fq2Ops> s_delta2 = total(piece2);
+  Xyzz<FqOps> sA, rB1, mL, mH;
+  Aff<FqOps> a_aff;
+  Aff<Fq2Ops> b_aff;
+  auto finish = [&](int k) {
+    if (k == 0) {
+      const auto A = bgh::xyzz_add(bgh::xyzz_add(msm_sum<FqOps>(plan[0]), r_delta), bgh::xyzz_from(pk.alpha));
+      sA = bgh::xyzz_mul(A, s);
+      a_aff = bgh::xyzz_to_affine(A);
+    } else if (k == 1) {
+      rB1 = bgh::xyzz_mul(
+          bgh::xyzz_add(bgh::xyzz_add(msm_sum<FqOps>(plan[1]), s_delta), bgh::xyzz_from(pk.beta)), r);
+    } else if (k == 2) {
+      b_aff = bgh::xyzz_to_affine(
+          bgh::xyzz_add(bgh::xyzz_add(msm_sum<Fq2Ops>(plan[2]), s_delta2), bgh::xyzz_from(pk.beta2)));
+    } else {
+      (k == 3 ? mH : mL) = msm_sum<FqOps>(plan[k]);
+    }
+  };
   // an MSM's window parts are on the host once its reduction stream drains (an empty MSM has
   // no stream: nothing to wait for)
-  auto drain = [](const MsmPlan& p) {
-    if (p.fetch_stream) BG_CUDA(cudaStreamSynchronize(p.fetch_stream));
-  };
-  drain(plan[0]);
-  msm_finish<Fq>(plan[0], res[0]);
-  const Xyzz<FqOps> A = bgh::xyzz_add(bgh::xyzz_add(g1(res[0]), r_delta), bgh::xyzz_from(pk.alpha));
-  drain(plan[1]);
-  msm_finish<Fq>(plan[1], res[1]);
-  const Xyzz<FqOps> B1 = bgh::xyzz_add(bgh::xyzz_add(g1(res[1]), s_delta), bgh::xyzz_from(pk.beta));
-  Xyzz<FqOps> sA, rB1;
-  HostPool::get().parallel_for(2, [&](int i) {
-    if (i == 0) sA = bgh::xyzz_mul(A, s);
-    else rB1 = bgh::xyzz_mul(B1, r);
-  });
-  Xyzz<FqOps> c_part = bgh::xyzz_add(bgh::xyzz_add(sA, rB1), bgh::xyzz_neg(rs_delta));
-  drain(plan[2]);
-  msm_finish<Fq2>(plan[2], res[2]);
-  const Xyzz<Fq2Ops> B2 = bgh::xyzz_add(
-      bgh::xyzz_add(bgh::xyzz_from(bgh::aff_from_words32<Fq2Ops>(res[2])), s_delta2), bgh::xyzz_from(pk.beta2));
-  // A and B are final here: their inversions to affine run while msm_h is still on the device
-  const auto a_aff = bgh::xyzz_to_affine(A);
-  const auto b_aff = bgh::xyzz_to_affine(B2);
-  drain(plan[4]);
-  msm_finish<Fq>(plan[4], res[4]);
-  c_part = bgh::xyzz_add(c_part, g1(res[4]));
-  for (int j = 0; j < kStreams; j++) BG_CUDA(cudaStreamSynchronize(ctx.side[j]));
-  BG_CUDA(cudaStreamSynchronize(st));
+  if (ctx.shared_gpu || HostPool::get().workers() < 4) {
+    for (int k : {0, 1, 2, 4, 3}) {
+      if (plan[k].fetch_stream) BG_CUDA(cudaStreamSynchronize(plan[k].fetch_stream));
+      finish(k);
+    }
+  } else {
+    HostPool::Task tasks[5];
+    bool taken[5] = {};
+    for (int left = 5; left;) {
+      const int before = left;
+      for (int k : {0, 1, 2, 4, 3}) {
+        if (taken[k]) continue;
+        if (plan[k].fetch_stream) {
+          const cudaError_t e = cudaStreamQuery(plan[k].fetch_stream);
+          if (e == cudaErrorNotReady) continue;
+          BG_CUDA(e);
+        }
+        taken[k] = true;
+        left--;
+        if (k == 3) finish(3);
+        else tasks[k] = HostPool::get().start(1, [&finish, k](int) { finish(k); });
+      }
+      if (left == before) std::this_thread::yield();
+    }
+    for (HostPool::Task& t : tasks) t.wait();
+  }
+  // the drained streams were behind everything but the main stream's own tail
   check_status(ctx, st);
-  msm_finish<Fq>(plan[3], res[3]);
-  const Xyzz<FqOps> C = bgh::xyzz_add(c_part, g1(res[3]));
+  const Xyzz<FqOps> C =
+      bgh::xyzz_add(bgh::xyzz_add(bgh::xyzz_add(sA, rB1), bgh::xyzz_neg(rs_delta)), bgh::xyzz_add(mL, mH));
   wire_from_affine<FqOps>(out->a, a_aff);
   wire_from_affine<Fq2Ops>(out->b, b_aff);
   wire_from_affine<FqOps>(out->c, bgh::xyzz_to_affine(C));
