@@ -1210,10 +1210,11 @@ int msm_pick_c_proof(size_t n, bool g2) {
 int msm_pick_c_table(size_t n, bool g2) {
   // one shared bucket set: wider windows (fewer additions) at the price of 2^(c-1) buckets
   if (const int t = tuned(kTuneTables, n, g2)) return t;
-  int c = floor_log2(n) - 1;
-  if (c < 6) c = 6;
-  if (c > 18) c = 18;
-  return c;
+  const int lg = floor_log2(n);
+  // the smallest proofs are bound by the chains of their reductions, whose length is the entries per
+  // bucket: SquareChain(2^8) 0.54 ms at 7 bits, 0.44 at 10; 2^9 0.53 ms at 8, 0.46 at 10 and 11
+  if (lg == 8 || lg == 9) return g2 ? lg + 2 : 10;
+  return std::min(18, std::max(6, lg - 1));
 }
 
 template <class F>

@@ -695,9 +695,27 @@ static size_t msm_footprint_c(size_t n, bool g2, int c) {
                        W * J * 2 * PW + 2 * ((nkeys + 1) / 2048 + 1) + pairs;
   return words * 4;
 }
+// Window widths the reservation is made for, per floor(log2 n) from 10, G1 and G2: a standalone MSM's
+// and a one-shot proof's.  They are wider than the tuned ones in places and stay as they are when
+// those change, so that a budget admits what it admitted; a proof's scratch lies below the
+// reservation (SquareChain(2^10): 6 of 30 MB, 2^18: 0.8 of 1.5 GB, 2^20: 2.6 of 7.7 GB).
+static int reserved_c(size_t n, bool g2, bool in_proof) {
+  static const signed char sets[2][13] = {{8, 8, 9, 9, 9, 10, 11, 12, 15, 15, 15, 15, 17},
+                                          {8, 9, 9, 9, 9, 10, 11, 12, 15, 15, 15, 0, 0}};
+  static const signed char proof[2][13] = {{10, 0, 11, 0, 10, 0, 12, 0, 13, 0, 15, 0, 0},
+                                           {8, 0, 9, 0, 9, 0, 12, 0, 14, 0, 15, 0, 0}};
+  int lg = 0;
+  while ((size_t(1) << (lg + 1)) <= n) lg++;
+  const int i = lg - 10;
+  if (i >= 0 && i < 13) {
+    if (in_proof && proof[g2][i]) return proof[g2][i];
+    if (sets[g2][i]) return sets[g2][i];
+  }
+  return std::min(16, std::max(3, lg - 3));
+}
 static size_t msm_footprint(size_t n, bool g2) {
   if (n == 0) return 0;
-  return std::max(msm_footprint_c(n, g2, msm_pick_c(n, g2)), msm_footprint_c(n, g2, msm_pick_c_proof(n, g2)));
+  return std::max(msm_footprint_c(n, g2, reserved_c(n, g2, false)), msm_footprint_c(n, g2, reserved_c(n, g2, true)));
 }
 
 size_t prove_footprint(const Header& h) {
