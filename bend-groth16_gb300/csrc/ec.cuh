@@ -194,6 +194,34 @@ BG_DEV XYZZ<F> xyzz_add(const XYZZ<F>& p, const XYZZ<F>& q) {
   return r;
 }
 
+// the same with its Fq products inlined, for an addition that is itself out of line
+template <class F>
+BG_DEV XYZZ<F> xyzz_add_inline(const XYZZ<F>& p, const XYZZ<F>& q) {
+  if (is_inf(q)) return p;
+  if (is_inf(p)) return q;
+  const F u1 = imul(p.x, q.zz);
+  const F u2 = imul(q.x, p.zz);
+  const F s1 = imul(p.y, q.zzz);
+  const F s2 = imul(q.y, p.zzz);
+  const F zz12 = imul(p.zz, q.zz);
+  const F zzz12 = imul(p.zzz, q.zzz);
+  const F pp_ = sub(u2, u1);
+  const F r_ = sub(s2, s1);
+  if (is_zero(pp_)) {
+    if (is_zero(r_)) return xyzz_dbl(XYZZ<F>{u1, s1, zz12, zzz12});
+    return xyzz_inf<F>();
+  }
+  const F pp = isqr(pp_);
+  const F ppp = imul(pp_, pp);
+  const F qq = imul(u1, pp);
+  XYZZ<F> r;
+  r.x = sub(sub(isqr(r_), ppp), dbl(qq));
+  r.y = imul_sub(r_, sub(qq, r.x), s1, ppp);
+  r.zz = imul(zz12, pp);
+  r.zzz = imul(zzz12, ppp);
+  return r;
+}
+
 // ---------------------------------------------------------------- affine pair additions
 // P + Q for affine P and Q where the caller supplies 1/d for the denominator d: the
 // batch-affine accumulation inverts the denominators of many additions at once (Montgomery's

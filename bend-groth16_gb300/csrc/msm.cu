@@ -303,8 +303,8 @@ __global__ void __launch_bounds__(128) k_build_table(const uint32_t* __restrict_
 // boundary becomes a piece: entry 2t of the piece list if the run started in an earlier slice,
 // entry 2t+1 if the bucket starts in slice t and continues into a later one.  So a bucket with
 // entries [o, o') cut into slices t0 = o / K .. t1 = (o' - 1) / K has its pieces at 2 t0 + 1
-// and 2 u for t0 < u <= t1; the window reduction adds them where it reads the bucket
-// (bucket_value), which costs the same additions as a separate join pass without its launch
+// and 2 u for t0 < u <= t1; the window reduction adds them where it reads the
+// bucket, which costs the same additions as a separate join pass without its launch
 // and its mostly idle lanes.  A bucket of more than kPieceLimit + 1 pieces (a scalar value
 // repeated thousands of times) is joined beforehand by k_bucket_heavy: the thread that owns its
 // first piece lists it in heavy[1 + i] (heavy[0] counts, cleared before the accumulation).
@@ -478,21 +478,6 @@ constexpr uint32_t kHeavyGrid = 152;
 
 #include "msm_pairs.cuh"
 
-// acc += value of bucket `key` (entries [offsets[key], offsets[key+1])): nothing when empty, the
-// stored bucket when it lies in one slice or is heavy, else its pieces.
-template <class F>
-BG_DEV XYZZ<F> add_bucket(XYZZ<F> acc, const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ buckets,
-                          const uint32_t* __restrict__ parts, uint32_t K, size_t key) {
-  constexpr int PW = 4 * FieldWords<F>::value;
-  const uint32_t o0 = offsets[key], o1 = offsets[key + 1];
-  if (o1 == o0) return acc;
-  const uint32_t t0 = o0 / K, t1 = (o1 - 1) / K;
-  if (t0 == t1 || t1 - t0 > kPieceLimit) return xyzz_add(acc, load_xyzz<F>(buckets + key * PW));
-  acc = xyzz_add(acc, load_xyzz<F>(parts + (2 * (size_t)t0 + 1) * PW));
-  for (uint32_t u = t0 + 1; u <= t1; u++) acc = xyzz_add(acc, load_xyzz<F>(parts + 2 * (size_t)u * PW));
-  return acc;
-}
-
 // Entries per accumulation thread, from a latency model with constants measured on GB300 (G1;
 // G2 scales them alike): a thread's K mixed additions take K x 6.6 us at low occupancy, the
 // whole accumulation cannot beat its throughput (4.58 entries per ns), and a bucket of e
@@ -620,60 +605,15 @@ void bucket_heavy(Ctx* prof, cudaStream_t st, const uint32_t* offsets, uint32_t*
 //   S_j = sum_{local b} (b+1) B_b = sum_t T_t + M sum_{t>=1} Suf_t,   Suf_t = sum_{t'>=t} R_t'
 // comes from an in-CTA suffix scan of R and a tree sum; the part also reports R_j = Suf_0.
 // The host finishes window w as sum_j S_j + (RT M) sum_j j R_j.
-// Bucket values are read through add_bucket (stored bucket or its pieces).
-template <class F>
-__global__ void k_window_reduce(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ buckets,
-                                const uint32_t* __restrict__ pieces, uint32_t K, uint32_t nb, uint32_t M, uint32_t J,
-                                uint32_t* __restrict__ out) {
-  constexpr int PW = 4 * FieldWords<F>::value;
-  extern __shared__ uint32_t sm[];
-  const uint32_t RT = blockDim.x;
-  const uint32_t w = blockIdx.x / J, j = blockIdx.x % J, t = threadIdx.x;
-  const size_t key0 = (size_t)w * nb + ((size_t)j * RT + t) * M;
-  XYZZ<F> run = xyzz_inf<F>(), acc = xyzz_inf<F>();
-  for (int k = (int)M - 1; k >= 0; k--) {
-    run = add_bucket(run, offsets, buckets, pieces, K, key0 + k);
-    acc = xyzz_add(acc, run);
-  }
-  // inclusive suffix scan of R over the CTA (Hillis-Steele)
-  store_xyzz(sm + (size_t)t * PW, run);
-  __syncthreads();
-  for (uint32_t d = 1; d < RT; d <<= 1) {
-    XYZZ<F> v = xyzz_inf<F>();
-    if (t + d < RT) v = load_xyzz<F>(sm + (size_t)(t + d) * PW);
-    __syncthreads();
-    run = xyzz_add(run, v);
-    store_xyzz(sm + (size_t)t * PW, run);
-    __syncthreads();
-  }
-  // R_j, written at once so that it holds no registers through the tree below
-  if (t == 0) store_xyzz(out + ((size_t)blockIdx.x * 2 + 1) * PW, run);
-  // Y_t = T_t + M Suf_t (t >= 1), Y_0 = T_0
-  if (t >= 1) {
-    for (uint32_t m = M; m > 1; m >>= 1) run = xyzz_dbl(run);
-    acc = xyzz_add(acc, run);
-  }
-  __syncthreads();
-  store_xyzz(sm + (size_t)t * PW, acc);
-  __syncthreads();
-  for (uint32_t d = RT >> 1; d >= 1; d >>= 1) {
-    if (t < d) {
-      acc = xyzz_add(acc, load_xyzz<F>(sm + (size_t)(t + d) * PW));
-      store_xyzz(sm + (size_t)t * PW, acc);
-    }
-    __syncthreads();
-  }
-  if (t == 0) store_xyzz(out + (size_t)blockIdx.x * 2 * PW, acc);
-}
-
-// The same reduction with the points a thread owns in shared memory (word i of thread t's
-// point at base[i * RT + t]): R, T and a staging column for the scan.  One out-of-line body
-// adds a point into another (and one doubles in place), so no point is live in registers
-// across a call.  The register-resident form above spills in G2 (R, T and the addend are
-// 3 x 64 words across inlined Fq2 additions: 2.4 KB of spill stores per thread); this one
-// leaves 0.4 KB, and an addition's latency falls with it (G2 MSM 2^18 5.59 -> 5.33 ms,
-// SquareChain(2^10) proof 1.24 -> 1.11 ms, 2^12 1.66 -> 1.46 ms, 2^18 10.74 -> 10.62 ms).  For
-// G1 (no spills either way) it was measured level, so G1 keeps the register form.
+//
+// The points a thread owns lie in shared memory (word i of thread t's point at base[i * RT + t]): R,
+// T and a staging column for the scan.  One out-of-line body adds a point into another (and one
+// doubles in place), so no point is live in registers across a call.  Bound by the latency of that
+// chain of additions, with one CTA per SM in use.  The register-resident form this replaced spilled
+// in G2 (2.4 KB per thread; G2 MSM 2^18 5.59 -> 5.33 ms then); in G1 it did not, but its fourteen
+// calls per addition cost more than the one call here with the products inlined: reductions of
+// 16000 points 207 -> 185 us, 2^18 points 448 -> 410 us.  Bounded to two CTAs per SM (128
+// registers, spills) G1 measured no gain and SquareChain(2^14) 10% slower.
 BG_DEV void elem_load(Fq& e, const uint32_t* src, uint32_t stride) {
 #pragma unroll
   for (int l = 0; l < 8; l++) e.v[l] = src[l * stride];
@@ -715,7 +655,7 @@ static __device__ __noinline__ void pt_add_into(uint32_t* dst, uint32_t stride, 
   pt_load(p, dst, stride);
   if (sstride == 1) q = load_xyzz<F>(src);
   else pt_load(q, src, sstride);
-  pt_store(dst, stride, xyzz_add(p, q));
+  pt_store(dst, stride, xyzz_add_inline(p, q));
 }
 template <class F>
 static __device__ __noinline__ void pt_dbl_in(uint32_t* dst, uint32_t stride) {
@@ -723,16 +663,17 @@ static __device__ __noinline__ void pt_dbl_in(uint32_t* dst, uint32_t stride) {
   pt_load(p, dst, stride);
   pt_store(dst, stride, xyzz_dbl(p));
 }
-// shared memory of k_window_reduce_sm: R, T and the scan's staging column
+// shared memory of k_window_reduce: R, T and the scan's staging column
 template <class F>
 constexpr size_t reduce_sm_bytes(uint32_t RT) {
   return 3 * (size_t)RT * 4 * FieldWords<F>::value * sizeof(uint32_t);
 }
 
 template <class F>
-__global__ void k_window_reduce_sm(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ buckets,
-                                   const uint32_t* __restrict__ pieces, uint32_t K, uint32_t nb, uint32_t M,
-                                   uint32_t J, uint32_t* __restrict__ out) {
+__global__ void __launch_bounds__(256)
+    k_window_reduce(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ buckets,
+                    const uint32_t* __restrict__ pieces, uint32_t K, uint32_t nb, uint32_t M, uint32_t J,
+                    uint32_t* __restrict__ out) {
   constexpr int PW = 4 * FieldWords<F>::value;
   extern __shared__ uint32_t sm[];
   const uint32_t RT = blockDim.x;
@@ -791,11 +732,6 @@ __global__ void k_window_reduce_sm(const uint32_t* __restrict__ offsets, const u
   }
 }
 
-// which form reduces a field's windows (G1's register-resident form does not spill: 200
-// registers)
-template <class F>
-constexpr bool kReduceInSmem = FieldWords<F>::value == 16;
-
 // Shape of the window reduction: RT threads x M buckets per thread x J parts per window, picked
 // by a latency model.  A thread's dependent chain is M (2 + e / K) additions (each bucket
 // costs its pieces, about 1 + e / K for e entries per bucket, plus the running-sum addition),
@@ -815,12 +751,7 @@ int reduce_blocks_per_sm(uint32_t RT) {
   while ((1u << lrt) < RT) lrt++;
   if (!cache[lrt]) {
     int n = 0;
-    if constexpr (kReduceInSmem<F>)
-      BG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_window_reduce_sm<F>, (int)RT,
-                                                            reduce_sm_bytes<F>(RT)));
-    else
-      BG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_window_reduce<F>, (int)RT,
-                                                            RT * 4 * FieldWords<F>::value * sizeof(uint32_t)));
+    BG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_window_reduce<F>, (int)RT, reduce_sm_bytes<F>(RT)));
     cache[lrt] = n > 0 ? n : 1;
   }
   return cache[lrt];
@@ -1158,12 +1089,9 @@ void msm_accumulate(Ctx& ctx, cudaStream_t st, const std::string& tag, const uin
     if (rsh.coop)
       k_window_reduce_coop<F><<<so.sets * J, RT * kCoopLanes, RT * coop_group_words<F>() * sizeof(uint32_t), rs>>>(
           acc_offsets, buckets, bs.parts, bs.K, so.nb, M, J, parts);
-    else if constexpr (kReduceInSmem<F>)
-      k_window_reduce_sm<F><<<so.sets * J, RT, reduce_sm_bytes<F>(RT), rs>>>(acc_offsets, buckets, bs.parts, bs.K,
-                                                                             so.nb, M, J, parts);
     else
-      k_window_reduce<F><<<so.sets * J, RT, RT * PW * sizeof(uint32_t), rs>>>(acc_offsets, buckets, bs.parts, bs.K,
-                                                                               so.nb, M, J, parts);
+      k_window_reduce<F><<<so.sets * J, RT, reduce_sm_bytes<F>(RT), rs>>>(acc_offsets, buckets, bs.parts, bs.K, so.nb, M,
+                                                                          J, parts);
     BG_CHECK_LAUNCH();
   }
   plan.fetch_stream = rs;
@@ -1342,12 +1270,10 @@ void msm_finish(const MsmPlan& plan, uint32_t* out_affine_words32) {
 constexpr int kInitMaxDevices = 64;
 void msm_init_kernels() {
   static std::once_flag once[kInitMaxDevices];
-  static_assert(!kReduceInSmem<Fq> && kReduceInSmem<Fq2>, "reduction forms: G1 in registers, G2 in shared memory");
   int dev = 0;
   BG_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= kInitMaxDevices) throw Error(BG_E_ARG, "msm: device index out of range");
   std::call_once(once[dev], [] {
-    BG_CUDA(cudaFuncSetAttribute(k_window_reduce<Fq>, cudaFuncAttributeMaxDynamicSharedMemorySize, 256 * 32 * 4));
     auto smem = [](auto* k, size_t bytes) {
       BG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     };
@@ -1355,8 +1281,8 @@ void msm_init_kernels() {
     smem(k_pair_round<Fq, false>, pair_smem_bytes<Fq>());
     smem(k_pair_round<Fq2, true>, pair_smem_bytes<Fq2>());
     smem(k_pair_round<Fq2, false>, pair_smem_bytes<Fq2>());
-    BG_CUDA(cudaFuncSetAttribute(k_window_reduce_sm<Fq2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)reduce_sm_bytes<Fq2>(256)));
+    smem(k_window_reduce<Fq>, reduce_sm_bytes<Fq>(256));
+    smem(k_window_reduce<Fq2>, reduce_sm_bytes<Fq2>(256));
   });
 }
 
@@ -1492,8 +1418,7 @@ void msm_g1_noalloc(const uint32_t* d_points, const uint32_t* d_scalars, size_t 
   BG_CHECK_LAUNCH();
   bucket_accumulate<Fq>(nullptr, st, d_points, offsets, sorted, (uint32_t)nkeys, max_entries, buckets, bs);
   bucket_heavy<Fq>(nullptr, st, offsets, buckets, bs);
-  k_window_reduce<Fq><<<W * J, RT, RT * PW * sizeof(uint32_t), st>>>(offsets, buckets, bs.parts, bs.K, nb, M, J,
-                                                                     parts);
+  k_window_reduce<Fq><<<W * J, RT, reduce_sm_bytes<Fq>(RT), st>>>(offsets, buckets, bs.parts, bs.K, nb, M, J, parts);
   BG_CHECK_LAUNCH();
   BG_CUDA(cudaMemcpyAsync(g_noalloc_host_parts, parts, host_words * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   BG_CUDA(cudaMemcpyAsync(&g_noalloc_host_status, status, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
