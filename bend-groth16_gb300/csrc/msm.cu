@@ -15,10 +15,11 @@
 //                     (mixed add); a bucket cut by slice boundaries leaves pieces, joined
 //                     where the reduction reads it (k_bucket_heavy first joins the rare
 //                     buckets of very many pieces)
-//   5. k_window_reduce one CTA per window part: running sums over M buckets per thread, an
-//                     in-CTA suffix scan and tree sum give sum_b (b+1) B_b for the part
-//   6. host: parts -> window sums -> Horner (a window's width of doublings per window) ->
-//      affine.  Windows have balanced widths of at most c bits (window_width).
+//   5. k_window_reduce one CTA per window part: running sums over M buckets per thread and a tree
+//                     that leaves sum_b (b+1) B_b as one sum per bit of the thread's index;
+//                     k_window_join sums the parts of a window
+//   6. host: one Horner over those bit positions -> affine.  Windows have balanced widths of at
+//      most c bits (window_width).
 // Window sums and the final point are exact group elements, so the affine result equals the
 // reference's for the same inputs regardless of bucket order inside a window.
 #include "common.cuh"
@@ -602,18 +603,24 @@ void bucket_heavy(Ctx* prof, cudaStream_t st, const uint32_t* offsets, uint32_t*
 // Window reduction, one CTA per (window, part).  Part j of window w covers buckets
 // [j RT M, (j+1) RT M); thread t folds M consecutive buckets into R_t = sum B and
 // T_t = sum_k (k+1) B_{tM+k} (running sums).  The part's weighted sum
-//   S_j = sum_{local b} (b+1) B_b = sum_t T_t + M sum_{t>=1} Suf_t,   Suf_t = sum_{t'>=t} R_t'
-// comes from an in-CTA suffix scan of R and a tree sum; the part also reports R_j = Suf_0.
-// The host finishes window w as sum_j S_j + (RT M) sum_j j R_j.
+//   S_j = sum_{local b} (b+1) B_b = sum_t T_t + M sum_t t R_t
+// is left split by the bits of t: sum_t t R_t = sum_b 2^b U_b with U_b the sum of the R_t whose t
+// has bit b.  Halving R over t and t + d leaves in the columns [d, 2d) just the terms of U_log2(d),
+// so one tree of log2(RT) levels sums R, T and, in the columns that it frees, every U_b; no level
+// has more than RT additions and the host's Horner, which doubles through all those bit positions
+// anyway, adds each U_b at its own.  k_window_join sums the parts of a window the same way.
 //
-// The points a thread owns lie in shared memory (word i of thread t's point at base[i * RT + t]): R,
-// T and a staging column for the scan.  One out-of-line body adds a point into another (and one
-// doubles in place), so no point is live in registers across a call.  Bound by the latency of that
-// chain of additions, with one CTA per SM in use.  The register-resident form this replaced spilled
-// in G2 (2.4 KB per thread; G2 MSM 2^18 5.59 -> 5.33 ms then); in G1 it did not, but its fourteen
-// calls per addition cost more than the one call here with the products inlined: reductions of
-// 16000 points 207 -> 185 us, 2^18 points 448 -> 410 us.  Bounded to two CTAs per SM (128
-// registers, spills) G1 measured no gain and SquareChain(2^14) 10% slower.
+// The points a thread owns lie in shared memory (word i of thread t's point at base[i * RT + t]): R
+// and T.  One out-of-line body adds a point into another, its products inlined, so no point is live
+// in registers across a call: fourteen calls per addition, registers across all of them, measured
+// 207 us for the reductions of 16000 G1 points where this took 185.
+//
+// Bound by the latency of the chain of additions, two warps per scheduler at most.  The suffix scan
+// of R that this tree replaced (all threads in each of log2(RT) steps, then M Suf_t by doublings and
+// a second tree) was half of that chain: reductions of G1 MSMs of 16000 / 2^18 / 2^20 points 185 /
+// 410 / 404 -> 94 / 334 / 326 us, of G2 MSMs of 65000 / 2^18 points 687 / 1172 -> 395 / 903 us;
+// proofs SquareChain(2^10) 0.555 -> 0.525 ms, 2^14 1.15 -> 1.08, 2^15 1.63 -> 1.48, 2^17 3.98 ->
+// 3.74, 2^20 20.5 -> 20.3 (a mixed batch of 16: 16.5 -> 16.7).
 BG_DEV void elem_load(Fq& e, const uint32_t* src, uint32_t stride) {
 #pragma unroll
   for (int l = 0; l < 8; l++) e.v[l] = src[l * stride];
@@ -657,18 +664,26 @@ static __device__ __noinline__ void pt_add_into(uint32_t* dst, uint32_t stride, 
   else pt_load(q, src, sstride);
   pt_store(dst, stride, xyzz_add_inline(p, q));
 }
+// shared memory of k_window_reduce: R and T (one bucket per thread: T_t = R_t)
 template <class F>
-static __device__ __noinline__ void pt_dbl_in(uint32_t* dst, uint32_t stride) {
-  XYZZ<F> p;
-  pt_load(p, dst, stride);
-  pt_store(dst, stride, xyzz_dbl(p));
+constexpr size_t reduce_sm_bytes(uint32_t RT, uint32_t M) {
+  return (M == 1 ? 1 : 2) * (size_t)RT * 4 * FieldWords<F>::value * sizeof(uint32_t);
 }
-// shared memory of k_window_reduce: R, T and the scan's staging column
-template <class F>
-constexpr size_t reduce_sm_bytes(uint32_t RT) {
-  return 3 * (size_t)RT * 4 * FieldWords<F>::value * sizeof(uint32_t);
+// The tree's level d: additions col += col + d for the first d columns of R, of T (with_t) and of
+// each U_b split off so far (offset o).  Index i of them -> column of R, or of T (from RT up).
+BG_DEV uint32_t tree_column(uint32_t i, uint32_t d, uint32_t RT, bool with_t) {
+  const uint32_t q = i / d, k = i % d;
+  if (q == 0) return k;
+  if (with_t && q == 1) return RT + k;
+  return ((2 * d) << (q - 1 - (with_t ? 1 : 0))) + k;
+}
+BG_DEV uint32_t tree_count(uint32_t d, uint32_t RT, bool with_t) {
+  uint32_t arrays = with_t ? 2 : 1;
+  for (uint32_t e = 2 * d; e < RT; e <<= 1) arrays++;
+  return arrays * d;
 }
 
+// A part's points in `out`: T, U_0 .. U_(log2 RT - 1), and with several parts R last.
 template <class F>
 __global__ void __launch_bounds__(256)
     k_window_reduce(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ buckets,
@@ -679,11 +694,13 @@ __global__ void __launch_bounds__(256)
   const uint32_t RT = blockDim.x;
   const uint32_t w = blockIdx.x / J, j = blockIdx.x % J, t = threadIdx.x;
   const size_t key0 = (size_t)w * nb + ((size_t)j * RT + t) * M;
-  uint32_t* R = sm + t;                        // running sum R_t
-  uint32_t* T = sm + (size_t)PW * RT + t;      // weighted sum T_t
-  uint32_t* S = sm + (size_t)2 * PW * RT + t;  // staging for the scan
+  const bool with_t = M > 1;
+  // point of column c: R below RT, T from RT up
+  auto col = [&](uint32_t c) { return sm + (c < RT ? c : (size_t)PW * RT + (c - RT)); };
+  uint32_t* R = sm + t;                     // running sum R_t
+  uint32_t* T = sm + (size_t)PW * RT + t;   // weighted sum T_t
   pt_store(R, RT, xyzz_inf<F>());
-  pt_store(T, RT, xyzz_inf<F>());
+  if (with_t) pt_store(T, RT, xyzz_inf<F>());
   for (int k = (int)M - 1; k >= 0; k--) {
     const size_t key = key0 + k;
     const uint32_t o0 = offsets[key], o1 = offsets[key + 1];
@@ -696,96 +713,103 @@ __global__ void __launch_bounds__(256)
         for (uint32_t u = t0 + 1; u <= t1; u++) pt_add_into<F>(R, RT, pieces + 2 * (size_t)u * PW, 1);
       }
     }
-    pt_add_into<F>(T, RT, R, RT);
-  }
-  __syncthreads();
-  // inclusive suffix scan of R over the CTA (Hillis-Steele), through the staging column
-  for (uint32_t d = 1; d < RT; d <<= 1) {
-    if (t + d < RT) {
-#pragma unroll 8
-      for (int i = 0; i < PW; i++) S[i * RT] = R[i * RT + d];
-    } else {
-      pt_store(S, RT, xyzz_inf<F>());
-    }
-    __syncthreads();
-    pt_add_into<F>(R, RT, S, RT);
-    __syncthreads();
-  }
-  // R_j = Suf_0
-  if (t == 0) {
-#pragma unroll 8
-    for (int i = 0; i < PW; i++) out[((size_t)blockIdx.x * 2 + 1) * PW + i] = R[i * RT];
-  }
-  // Y_t = T_t + M Suf_t (t >= 1), Y_0 = T_0
-  if (t >= 1) {
-    for (uint32_t m = M; m > 1; m >>= 1) pt_dbl_in<F>(R, RT);
-    pt_add_into<F>(T, RT, R, RT);
+    if (with_t) pt_add_into<F>(T, RT, R, RT);
   }
   __syncthreads();
   for (uint32_t d = RT >> 1; d >= 1; d >>= 1) {
-    if (t < d) pt_add_into<F>(T, RT, T + d, RT);
+    if (t < tree_count(d, RT, with_t)) {
+      const uint32_t c = tree_column(t, d, RT, with_t);
+      pt_add_into<F>(col(c), RT, col(c + d), RT);
+    }
     __syncthreads();
   }
-  if (t == 0) {
-#pragma unroll 8
-    for (int i = 0; i < PW; i++) out[(size_t)blockIdx.x * 2 * PW + i] = T[i * RT];
+  uint32_t lrt = 0;
+  while ((1u << lrt) < RT) lrt++;
+  const uint32_t np = lrt + 1 + (J > 1 ? 1 : 0);
+  uint32_t* o = out + (size_t)blockIdx.x * np * PW;
+  for (uint32_t i = t; i < np * PW; i += RT) {
+    const uint32_t q = i / PW;
+    const uint32_t c = q == 0 ? (with_t ? RT : 0u) : q <= lrt ? 1u << (q - 1) : 0u;
+    o[i] = col(c)[(size_t)(i % PW) * RT];
   }
 }
 
 // Shape of the window reduction: RT threads x M buckets per thread x J parts per window, picked
 // by a latency model.  A thread's dependent chain is M (2 + e / K) additions (each bucket
-// costs its pieces, about 1 + e / K for e entries per bucket, plus the running-sum addition),
-// two log2(RT) trees and log2(M) doublings, times the number of waves the sets x J CTAs need
-// at the kernel's occupancy; the host then adds 3 J points per bucket set, at about 1/16 of a
-// device addition's latency each (a single dependent chain is ~20x faster on a CPU core than
-// on one GPU thread).
+// costs its pieces, about 1 + e / K for e entries per bucket, plus the running-sum addition that
+// a single bucket does without) and the tree's log2(RT), times the number of waves the sets x J
+// CTAs need at the kernel's occupancy; the join of several parts adds a launch and its own levels.
+constexpr double kCoopAddCost = 0.45, kCoopWarpCost = 0.1;
 struct ReduceShape {
   uint32_t RT, M, J;
   double cost = 0;     // the model's latency, in dependent additions
   bool coop = false;   // k_window_reduce_coop: RT groups of 8 lanes
+  bool scan = false;   // which weighs its one part's sums itself
 };
+inline int log2_of(uint32_t x) {
+  int l = 0;
+  while ((1u << l) < x) l++;
+  return l;
+}
 template <class F>
 int reduce_blocks_per_sm(uint32_t RT) {
   static int cache[9] = {};
-  int lrt = 0;
-  while ((1u << lrt) < RT) lrt++;
+  const int lrt = log2_of(RT);
   if (!cache[lrt]) {
     int n = 0;
-    BG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_window_reduce<F>, (int)RT, reduce_sm_bytes<F>(RT)));
+    BG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_window_reduce<F>, (int)RT, reduce_sm_bytes<F>(RT, 2)));
     cache[lrt] = n > 0 ? n : 1;
   }
   return cache[lrt];
 }
-// The host's part of a reduction, in device additions: J parts per bucket set, 3 host additions
-// each at about 1/16 of a device addition's latency.  With `pooled`, a single bucket set of a
-// power-of-two J >= 32 (window tables) counts as msm_finish sums it: in chunks on the host pool,
-// so its latency is a chunk's parts plus the chunks' join.
-inline double host_parts_cost(uint32_t J, int sets, bool pooled) {
-  if (pooled && sets == 1 && J >= 32 && (J & (J - 1)) == 0) {
-    const uint32_t chunks = std::min<uint32_t>(16, J / 8), C = J / chunks;
-    return 3.0 * (C + chunks) / 16.0;
-  }
-  return 3.0 * J * sets / 16.0;
+// dependent additions over a thread's own buckets
+inline double reduce_chain(uint32_t M, double entries_per_slice) {
+  return M * (1.0 + entries_per_slice) + (M > 1 ? M : 0);
+}
+// the join of J parts, in additions of the reduction's threads
+constexpr double kJoinLaunchCost = 0.5;
+// A set's points beside T cost the host an addition each.  From 64 additions on they go to the
+// host pool, whose wake-up (about 45 us) is worth four additions here: for the small sets of a small
+// MSM more than the levels saved, so that a part that covers its set weighs its sums itself (a
+// suffix scan, log2(RT) levels more; MSMs of 1000 points G1 / G2 269 / 493 us, 305 / 556 by bits).
+constexpr int kHostPoolPoints = 64;
+constexpr double kHostPoolCost = 4.0;
+inline bool reduce_scan(uint32_t RT, uint32_t M, uint32_t J, int sets) {
+  return J == 1 && M == 1 && sets * log2_of(RT) >= kHostPoolPoints;
+}
+inline double host_cost(bool scan, uint32_t span, int sets) {
+  return !scan && sets >= 4 && sets * log2_of(span) >= kHostPoolPoints ? kHostPoolCost : 0.0;
+}
+constexpr uint32_t kCoopMaxParts = 4096;  // of all sets: bounds the parts buffer (8 MB in G2)
+// (k_window_join: 32 groups at most, the last point's tree the longest)
+inline double join_cost(uint32_t J) {
+  if (J == 1) return 0.0;
+  double adds = 0;
+  for (uint32_t d = J >> 1, arrays = 1; d >= 1; d >>= 1, arrays++) adds += (arrays * d + 31) / 32;
+  return kJoinLaunchCost + kCoopAddCost * adds;
+}
+// Waves of CTAs times how far warps that share a scheduler slow each other's additions, two of them
+// being the unit; small CTAs follow one another without a last empty wave.
+inline double thread_waves(double ctas, int bps, uint32_t RT, int sm_count) {
+  const double waves = ctas / ((double)sm_count * bps);
+  const double resident = std::min<double>(bps, std::ceil(ctas / sm_count)) * RT / 128.0;
+  return std::max(1.0, bps >= 4 ? waves : std::ceil(waves)) * (1.0 + 0.35 * std::max(0.0, resident - 2.0));
 }
 
 template <class F>
-ReduceShape reduce_shape(uint32_t nb, int sets, size_t entries, uint32_t K, int sm_count, uint32_t max_rt,
-                         bool pooled_host = false) {
+ReduceShape reduce_shape(uint32_t nb, int sets, size_t entries, uint32_t K, int sm_count, uint32_t min_rt,
+                         uint32_t max_rt) {
   const double e = (double)entries / ((double)nb * sets);
-  const double per_bucket = 2.0 + e / K;
   ReduceShape best{nb < 32 ? nb : 32, 1, 1};
   best.J = nb / best.RT;
   double best_cost = 1e300;
-  for (uint32_t RT = 32; RT <= max_rt; RT <<= 1) {
+  for (uint32_t RT = nb < min_rt ? 32 : min_rt; RT <= max_rt; RT <<= 1) {
     for (uint32_t M = 1; M <= 16; M <<= 1) {
       if ((uint64_t)RT * M > nb) continue;
       const uint32_t J = nb / (RT * M);
-      int lrt = 0, lm = 0;
-      while ((1u << lrt) < RT) lrt++;
-      while ((1u << lm) < M) lm++;
-      const double slots = (double)sm_count * reduce_blocks_per_sm<F>(RT);
-      const double waves = std::ceil((double)J * sets / slots);
-      const double cost = waves * (M * per_bucket + 2.0 * lrt + lm) + host_parts_cost(J, sets, pooled_host);
+      const double waves = thread_waves((double)J * sets, reduce_blocks_per_sm<F>(RT), RT, sm_count);
+      const double cost = waves * (reduce_chain(M, e / K) + log2_of(RT)) + join_cost(J) +
+                          host_cost(false, nb / M, sets);
       if (cost < best_cost) {
         best_cost = cost;
         best = {RT, M, J, cost, false};
@@ -797,32 +821,26 @@ ReduceShape reduce_shape(uint32_t nb, int sets, size_t entries, uint32_t K, int 
 }
 
 // A hidden reduction's shape by work instead of latency: the one with the fewest warp-additions
-// per bucket (the running sums, plus the scan, doublings and tree that a CTA of RT threads adds
-// on top, counted per warp as a warp issues them) whose latency by reduce_shape's model stays
+// per bucket (the running sums, plus the tree that a CTA of RT threads adds on top, counted per
+// warp as a warp issues them) whose latency by reduce_shape's model stays
 // within `max_cost` dependent additions; {0, 0, 0} when none does.
 template <class F>
 ReduceShape reduce_shape_work(uint32_t nb, int sets, size_t entries, uint32_t K, int sm_count, uint32_t max_rt,
                               double max_cost) {
   const double e = (double)entries / ((double)nb * sets);
-  const double per_bucket = 2.0 + e / K;
   ReduceShape best{0, 0, 0, 1e300, false};
   double best_work = 1e300;
   for (uint32_t RT = 32; RT <= max_rt; RT <<= 1) {
     for (uint32_t M = 1; M <= 16; M <<= 1) {
       if ((uint64_t)RT * M > nb) continue;
       const uint32_t J = nb / (RT * M);
-      int lrt = 0, lm = 0;
-      while ((1u << lrt) < RT) lrt++;
-      while ((1u << lm) < M) lm++;
-      const double slots = (double)sm_count * reduce_blocks_per_sm<F>(RT);
-      const double waves = std::ceil((double)J * sets / slots);
-      const double cost = waves * (M * per_bucket + 2.0 * lrt + lm) + host_parts_cost(J, sets, false);
+      const double waves = thread_waves((double)J * sets, reduce_blocks_per_sm<F>(RT), RT, sm_count);
+      const double cost = waves * (reduce_chain(M, e / K) + log2_of(RT)) + join_cost(J);
       if (cost > max_cost) continue;
-      const double warps = RT / 32.0;
-      double scan = 0, tree = 0;
-      for (uint32_t d = 1; d < RT; d <<= 1) scan += std::ceil((RT - d) / 32.0);
-      for (uint32_t d = RT >> 1; d >= 1; d >>= 1) tree += std::ceil(d / 32.0);
-      const double work = (warps * M * per_bucket + scan + warps * (lm + 1) + tree) / ((double)RT * M);
+      double tree = 0;
+      for (uint32_t d = RT >> 1; d >= 1; d >>= 1)
+        tree += std::ceil(d * (log2_of(RT / d) + (M > 1 ? 1 : 0)) / 32.0);
+      const double work = (RT / 32.0 * reduce_chain(M, e / K) + tree) / ((double)RT * M);
       if (work < best_work - 1e-12) {
         best_work = work;
         best = {RT, M, J, cost, false};
@@ -836,13 +854,11 @@ ReduceShape reduce_shape_work(uint32_t nb, int sets, size_t entries, uint32_t K,
 
 // The cooperative form's shape by the same model: RT groups (of 8 lanes) per CTA, each addition
 // about kCoopAddCost of a thread's addition (dependency depth 4.6 of 14 products, plus the
-// group's exchanges), the log2 M doublings on one lane at full cost.
-constexpr double kCoopAddCost = 0.45;
+// group's exchanges) with one warp per scheduler and kCoopWarpCost more for each further one.
 template <class F>
 int reduce_coop_blocks_per_sm(uint32_t RT) {
   static int cache[6] = {};
-  int lrt = 0;
-  while ((1u << lrt) < RT) lrt++;
+  const int lrt = log2_of(RT);
   if (!cache[lrt]) {
     int n = 0;
     BG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_window_reduce_coop<F>, (int)RT * kCoopLanes,
@@ -852,25 +868,55 @@ int reduce_coop_blocks_per_sm(uint32_t RT) {
   return cache[lrt];
 }
 template <class F>
-ReduceShape reduce_shape_coop(uint32_t nb, int sets, size_t entries, uint32_t K, int sm_count, bool pooled_host) {
+ReduceShape reduce_shape_coop(uint32_t nb, int sets, size_t entries, uint32_t K, int sm_count) {
   const double e = (double)entries / ((double)nb * sets);
-  const double per_bucket = 2.0 + e / K;
   ReduceShape best{0, 0, 0, 1e300, true};
   for (uint32_t RT = 4; RT <= 32; RT <<= 1) {
     for (uint32_t M = 1; M <= 16; M <<= 1) {
       if ((uint64_t)RT * M > nb) continue;
       const uint32_t J = nb / (RT * M);
-      int lrt = 0, lm = 0;
-      while ((1u << lrt) < RT) lrt++;
-      while ((1u << lm) < M) lm++;
-      const double slots = (double)sm_count * reduce_coop_blocks_per_sm<F>(RT);
-      const double waves = std::ceil((double)J * sets / slots);
-      const double cost =
-          waves * (kCoopAddCost * (M * per_bucket + 2.0 * lrt) + lm) + host_parts_cost(J, sets, pooled_host);
-      if (cost < best.cost) best = {RT, M, J, cost, true};
+      if (J > 1 && J * (uint32_t)sets > kCoopMaxParts) continue;
+      const int bps = reduce_coop_blocks_per_sm<F>(RT);
+      const double ctas = (double)J * sets;
+      const double resident = std::min<double>(bps, std::ceil(ctas / sm_count)) * RT * kCoopLanes / 128.0;
+      const double add = kCoopAddCost + kCoopWarpCost * std::max(0.0, resident - 1.0);
+      const bool scan = reduce_scan(RT, M, J, sets);
+      const double cost = std::max(1.0, ctas / ((double)sm_count * bps)) * add *
+                              (reduce_chain(M, e / K) + log2_of(RT) * (scan ? 2 : 1)) +
+                          join_cost(J) + host_cost(scan, nb / M, sets);
+      if (cost < best.cost) best = {RT, M, J, cost, true, scan};
     }
   }
   return best;
+}
+
+// Points a bucket set leaves: T and a sum per bit above a thread's buckets.
+inline size_t reduce_points(const ReduceShape& r) { return r.scan ? 1 : 1 + log2_of(r.RT) + log2_of(r.J); }
+// Points of the parts buffer per bucket set: with several parts theirs (one more each) and the
+// joined ones.
+inline size_t reduce_part_points(const ReduceShape& r) {
+  return r.J > 1 ? r.J * (size_t)(2 + log2_of(r.RT)) + reduce_points(r) : reduce_points(r);
+}
+// The reduction and, for several parts per window, their join; returns where the sets' points are.
+template <class F>
+uint32_t* window_reduce(cudaStream_t st, const ReduceShape& r, const uint32_t* offsets, const uint32_t* buckets,
+                        const BucketScratch& bs, uint32_t nb, int sets, uint32_t* parts) {
+  constexpr int PW = 4 * FieldWords<F>::value;
+  if (r.coop)
+    k_window_reduce_coop<F><<<sets * r.J, r.RT * kCoopLanes, r.RT * coop_group_words<F>() * sizeof(uint32_t), st>>>(
+        offsets, buckets, bs.parts, bs.K, nb, r.M, r.J, r.scan, parts);
+  else
+    k_window_reduce<F><<<sets * r.J, r.RT, reduce_sm_bytes<F>(r.RT, r.M), st>>>(offsets, buckets, bs.parts, bs.K, nb,
+                                                                               r.M, r.J, parts);
+  BG_CHECK_LAUNCH();
+  if (r.J == 1) return parts;
+  const int np = 2 + log2_of(r.RT);
+  uint32_t* joined = parts + (size_t)sets * r.J * np * PW;
+  const uint32_t groups = std::min<uint32_t>(32, r.J / 2);
+  k_window_join<F><<<sets * np, groups * kCoopLanes, groups * (size_t)kCoopTmp * FieldWords<F>::value * sizeof(uint32_t),
+                     st>>>(parts, r.J, np, joined);
+  BG_CHECK_LAUNCH();
+  return joined;
 }
 
 // ---------------------------------------------------------------- host driver
@@ -1041,64 +1087,47 @@ void msm_accumulate(Ctx& ctx, cudaStream_t st, const std::string& tag, const uin
   }
   bucket_heavy<F>(prof, rs, acc_offsets, buckets, bs);
 
-  // A reduction hidden under a later accumulation keeps its CTAs at 128 threads: a 256-thread
-  // CTA of ~210 registers leaves no room for an accumulation CTA on its SM for its whole
-  // (latency-bound) life (K = 18 proof: caps 64 / 128 / 256 measured 11.0 / 10.8 / 10.8 ms
-  // with the reductions' streams first, 10.12 / 9.87 / 9.94 ms with the accumulations first).
+  // A reduction hidden under a later accumulation runs in CTAs of 128 threads: 256 leave no room for
+  // an accumulation CTA on their SM for their whole (latency-bound) life, and smaller ones spread
+  // over more SMs (a mixed batch of 16 proofs 17.0 ms with 32 and 64 allowed, 16.7 without).
   ReduceShape rsh =
-      reduce_shape<F>(so.nb, so.sets, acc_entries, bs.K, ctx.sm_count, plan.latency_critical ? 256u : 128u);
-  // A reduction meant to run under later accumulations that the latency model says outlasts
-  // them (a mid-size proof's G2 MSM: SquareChain(2^14)'s took 1.02 ms after 0.39 ms of
-  // remaining accumulations) is critical after all.  Latency of one dependent addition at a
-  // reduction's occupancy: about 11 us (G1), 29 us (G2), measured on GB300.
-  // It takes the critical shapes only when it would outlast its budget twice over (by one time,
-  // SquareChain(2^15) and 2^16 proofs measured 1-4% slower: reductions near their budget are
-  // hidden well enough; by four times, 2^14 measured 1.59 -> 1.95 ms).  A critical reduction that ends while the host pool is otherwise idle
-  // (not one of a small proof's reductions, which end together and share the pool with the
-  // combine's products) has its host part sums priced as the pool runs them.  Interleaved on
-  // one GB300 against the fixed rule (only the last MSM critical): SquareChain(2^13) 2.12 ->
-  // 1.24 ms, 2^14 2.09 -> 1.68 ms, 2^16 3.75 -> 3.70 ms, 2^10 / 2^12 / 2^18 level.
+      reduce_shape<F>(so.nb, so.sets, acc_entries, bs.K, ctx.sm_count, plan.latency_critical ? 32u : 128u,
+                      plan.latency_critical ? 256u : 128u);
+  // A reduction meant to run under later accumulations that the latency model says outlasts them
+  // (SquareChain(2^14)'s G2 MSM: 0.53 ms, 0.29 ms of accumulations left) is critical after all and
+  // takes the critical shapes: 2^14 proofs 1.28 ms where it had to outlast them twice over, 1.09 ms
+  // so and with half the time, other sizes level.  Latency of one dependent addition at a
+  // reduction's occupancy: about 11 us (G1), 29 us (G2).
   bool critical = plan.latency_critical;
   const double add_us = FW == 16 ? 29.0 : 11.0;
-  if (!critical && plan.hidden_us > 0 && rsh.cost * add_us > 2.0 * plan.hidden_us) critical = true;
-  // A hidden G1 reduction takes the shape with the least work per bucket (longer chains, fewer
-  // scan, doubling and tree additions per bucket) whose modelled latency stays within a quarter
-  // of its budget (the model underestimates a reduction running beside accumulations by 1.3-2x).
-  // Interleaved against the shortest-chain shapes on one GB300: SquareChain(2^16) 3.69 ->
-  // 3.46 ms, 2^17 6.14 -> 5.96 ms, 2^18 10.55 -> 10.48 ms, 2^14 and 2^20 level; with the
-  // accumulations first, half or all of the budget instead of a quarter measured level to 6%
-  // slower (2^16 3.46 -> 3.51 / 3.69 ms).  For G2 it
-  // measured level to 1% slower at 2^20 (the G2 reduction stretched 2.9 -> 5.1 ms and crowded
-  // the last accumulations), so G2 keeps the shortest chain.
+  if (!critical && plan.hidden_us > 0 && rsh.cost * add_us > plan.hidden_us) critical = true;
+  // A hidden G1 reduction takes the shape with the least work per bucket (longer chains, fewer tree
+  // additions per bucket) whose modelled latency stays within a small part of its budget, which the
+  // accumulations beside it stretch: a quarter / 6% / 3% of it measured 2^17 3.78 / 3.74 / 3.73 ms,
+  // 2^18 6.60 / 6.55 / 6.53, 2^20 20.27 / 20.25 / 20.29.  G2 keeps the shortest chain (at 2^20 the
+  // least work crowded the last accumulations).
   if (!critical && plan.hidden_us > 0 && FW == 8) {
     const ReduceShape wsh =
-        reduce_shape_work<F>(so.nb, so.sets, acc_entries, bs.K, ctx.sm_count, 128u, 0.25 * plan.hidden_us / add_us);
+        reduce_shape_work<F>(so.nb, so.sets, acc_entries, bs.K, ctx.sm_count, 128u, 0.06 * plan.hidden_us / add_us);
     if (wsh.RT) rsh = wsh;
   }
-  const bool pooled = critical && plan.host_pool_free;
-  if (pooled) rsh = reduce_shape<F>(so.nb, so.sets, acc_entries, bs.K, ctx.sm_count, 256u, true);
+  if (critical && !plan.latency_critical)
+    rsh = reduce_shape<F>(so.nb, so.sets, acc_entries, bs.K, ctx.sm_count, 32u, 256u);
   // a reduction that ends a critical path may take the cooperative form (8 lanes per addition)
   if (critical && ctx.coop_reduce != 0) {
-    const ReduceShape csh = reduce_shape_coop<F>(so.nb, so.sets, acc_entries, bs.K, ctx.sm_count, pooled);
-    if (ctx.coop_reduce > 0 || csh.cost < rsh.cost) rsh = csh;
+    const ReduceShape csh = reduce_shape_coop<F>(so.nb, so.sets, acc_entries, bs.K, ctx.sm_count);
+    if (csh.RT && (ctx.coop_reduce > 0 || csh.cost < rsh.cost)) rsh = csh;
   }
-  const uint32_t RT = rsh.RT, M = rsh.M, J = rsh.J;
-  uint32_t* parts = ws.get_t<uint32_t>(tag + ".parts", (size_t)so.sets * J * 2 * PW);
+  uint32_t* parts = ws.get_t<uint32_t>(tag + ".parts", so.sets * reduce_part_points(rsh) * PW);
+  const size_t points = reduce_points(rsh);  // per bucket set
   {
     KernelTimer kt(ctx, FW == 8 ? "msm_reduce_g1" : "msm_reduce_g2", rs);
-    if (rsh.coop)
-      k_window_reduce_coop<F><<<so.sets * J, RT * kCoopLanes, RT * coop_group_words<F>() * sizeof(uint32_t), rs>>>(
-          acc_offsets, buckets, bs.parts, bs.K, so.nb, M, J, parts);
-    else
-      k_window_reduce<F><<<so.sets * J, RT, reduce_sm_bytes<F>(RT), rs>>>(acc_offsets, buckets, bs.parts, bs.K, so.nb, M,
-                                                                          J, parts);
-    BG_CHECK_LAUNCH();
+    plan.d_window_sums = window_reduce<F>(rs, rsh, acc_offsets, buckets, bs, so.nb, so.sets, parts);
   }
   plan.fetch_stream = rs;
-  plan.J = J;
-  plan.part_span = RT * M;
-  plan.d_window_sums = parts;
-  plan.host_window_sums = ctx.host_cache.get_t<uint32_t>(tag + ".window_sums", (size_t)so.sets * J * 2 * PW);
+  plan.bits = (int)points - 1;
+  plan.shift = log2_of(rsh.M);
+  plan.host_window_sums = ctx.host_cache.get_t<uint32_t>(tag + ".window_sums", so.sets * points * PW);
 }
 
 int msm_rounds(const Ctx& ctx, size_t n, int c, bool shared_set, bool g2) {
@@ -1175,85 +1204,42 @@ void msm_fetch(Ctx& ctx, cudaStream_t st, MsmPlan& plan) {
   if (plan.W == 0) return;
   if (plan.fetch_stream) st = plan.fetch_stream;
   BG_CUDA(cudaMemcpyAsync(plan.host_window_sums, plan.d_window_sums,
-                          (size_t)plan.W * plan.J * 2 * PW * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-  ctx.d2h_bytes += (uint64_t)plan.W * plan.J * 2 * PW * sizeof(uint32_t);
+                          (size_t)plan.W * (plan.bits + 1) * PW * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+  ctx.d2h_bytes += (uint64_t)plan.W * (plan.bits + 1) * PW * sizeof(uint32_t);
 }
 
-// Window w = s_w + span u_w with s_w = sum_j S_j and u_w = sum_j j R_j; total = sum_w 2^(o_w)
-// window_w (Horner, span a power of two below the window's: u_w joins log2(span) doublings above
-// s_w, so no window doubles by itself).
+// Window w = T + 2^shift sum_b 2^b U_b, total = sum_w 2^(o_w) window_w: one Horner over the bit
+// positions.  Positions from the window's width up hold no digit (a last bucket set of narrower
+// windows leaves them at infinity).
 template <class H>
 bgh::Xyzz<H> msm_sum(const MsmPlan& plan) {
   constexpr int PW = 4 * H::WORDS;
-  int span_log = 0;
-  while ((1u << span_log) < plan.part_span) span_log++;
-  // s_w and u_w from window w's J parts (independent per window)
-  std::vector<bgh::Xyzz<H>> wsum(plan.W), wjr(plan.W, bgh::xyzz_inf<H>());
-  auto window_sum = [&](int w) {
-    const uint32_t* pw = plan.host_window_sums + (size_t)w * plan.J * 2 * PW;
-    bgh::Xyzz<H> s = bgh::xyzz_inf<H>(), run = bgh::xyzz_inf<H>(), jr = bgh::xyzz_inf<H>();
-    for (int j = (int)plan.J - 1; j >= 0; j--) {
-      s = bgh::xyzz_add(s, bgh::xyzz_from_words32<H>(pw + (size_t)(2 * j) * PW));
-      if (j >= 1) {
-        run = bgh::xyzz_add(run, bgh::xyzz_from_words32<H>(pw + (size_t)(2 * j + 1) * PW));
-        jr = bgh::xyzz_add(jr, run);  // sum_{j>=1} j R_j
-      }
-    }
-    wsum[w] = s;
-    wjr[w] = jr;
+  auto point = [&](int w, int i) {
+    return bgh::xyzz_from_words32<H>(plan.host_window_sums + ((size_t)w * (plan.bits + 1) + i) * PW);
   };
-  // One window of many parts (the shared bucket set of a key's window tables, e.g. J = 128 for
-  // msm_h of a SquareChain(2^18) proof: ~390 host additions after the proof's last kernel) is
-  // split into power-of-two chunks of parts on the host pool.  Chunk c covers parts [lo, lo + C)
-  // with lo = c C and gives s_c = sum S_j, t_c = sum R_j, u_c = sum (j - lo) R_j; then
-  // sum_j j R_j = sum_c u_c + C sum_{c>=1} c t_c, the last sum by a running sum over chunks.
-  auto single_window_chunked = [&]() {
-    const uint32_t J = plan.J;
-    const uint32_t chunks = std::min<uint32_t>(16, J / 8), C = J / chunks;
-    const uint32_t* pw = plan.host_window_sums;
-    std::vector<bgh::Xyzz<H>> cs(chunks), ct(chunks), cu(chunks);
-    HostPool::get().parallel_for((int)chunks, [&](int c) {
-      const uint32_t lo = (uint32_t)c * C;
-      bgh::Xyzz<H> s = bgh::xyzz_inf<H>(), run = bgh::xyzz_inf<H>(), u = bgh::xyzz_inf<H>();
-      for (int j = (int)(lo + C) - 1; j >= (int)lo; j--) {
-        s = bgh::xyzz_add(s, bgh::xyzz_from_words32<H>(pw + (size_t)(2 * j) * PW));
-        run = bgh::xyzz_add(run, bgh::xyzz_from_words32<H>(pw + (size_t)(2 * j + 1) * PW));
-        if (j > (int)lo) u = bgh::xyzz_add(u, run);
-      }
-      cs[c] = s;
-      ct[c] = run;
-      cu[c] = u;
-    });
-    bgh::Xyzz<H> s = bgh::xyzz_inf<H>(), jr = bgh::xyzz_inf<H>(), run = bgh::xyzz_inf<H>(),
-                 ctop = bgh::xyzz_inf<H>();
-    for (int c = (int)chunks - 1; c >= 0; c--) {
-      s = bgh::xyzz_add(s, cs[c]);
-      jr = bgh::xyzz_add(jr, cu[c]);
-      if (c >= 1) {
-        run = bgh::xyzz_add(run, ct[c]);
-        ctop = bgh::xyzz_add(ctop, run);  // sum_{c>=1} c t_c
-      }
+  // acc 2^(positions) + the window's points below its `positions` lowest bits
+  auto horner = [&](bgh::Jac<H> acc, int w, int positions) {
+    for (int d = positions - 1; d >= 0; d--) {
+      acc = bgh::jac_dbl(acc);
+      if (d >= plan.shift && d < plan.shift + plan.bits) acc = bgh::jac_add(acc, point(w, 1 + d - plan.shift));
     }
-    for (uint32_t m = C; m > 1; m >>= 1) ctop = bgh::xyzz_dbl(ctop);
-    wsum[0] = s;
-    wjr[0] = bgh::xyzz_add(jr, ctop);  // sum_{j>=1} j R_j
+    return bgh::jac_add(acc, point(w, 0));
   };
-  // The window sums of a bucket-set-per-window MSM are about two thirds of its host work
-  // (17 windows x 8 parts: ~550 of ~850 point operations); they run on the host pool, the
-  // Horner chain after them stays serial.  SquareChain(2^18) one-shot proof: the G2 finish is
-  // the tail of the proof.
-  const bool pow2_parts = plan.J >= 32 && (plan.J & (plan.J - 1)) == 0;
-  if (plan.W == 1 && pow2_parts && HostPool::get().workers() > 0) single_window_chunked();
-  else if (plan.W >= 4 && (size_t)plan.W * (plan.J - 1) >= 64)  // fewer additions take less than the pool's wake-up
-    HostPool::get().parallel_for(plan.W, window_sum);
-  else
-    for (int w = 0; w < plan.W; w++) window_sum(w);
+  const int top = plan.shift + plan.bits;
   bgh::Jac<H> acc = bgh::jac_inf<H>();
-  for (int w = plan.W - 1; w >= 0; w--) {
-    for (int d = window_width(w, plan.W); d > span_log; d--) acc = bgh::jac_dbl(acc);
-    acc = bgh::jac_add(acc, wjr[w]);
-    for (int d = 0; d < span_log; d++) acc = bgh::jac_dbl(acc);
-    acc = bgh::jac_add(acc, wsum[w]);
+  // The windows' own sums run on the host pool where they take longer than its wake-up.
+  if (plan.W >= 4 && plan.W * plan.bits >= kHostPoolPoints) {
+    std::vector<bgh::Xyzz<H>> win(plan.W);
+    HostPool::get().parallel_for(plan.W, [&](int w) {
+      win[w] = bgh::xyzz_from_jac(horner(bgh::jac_inf<H>(), w, std::min(top, window_width(w, plan.W))));
+    });
+    for (int w = plan.W - 1; w >= 0; w--) {
+      for (int d = window_width(w, plan.W); d > 0; d--) acc = bgh::jac_dbl(acc);
+      acc = bgh::jac_add(acc, win[w]);
+    }
+  } else {
+    for (int w = plan.W - 1; w >= 0; w--)
+      acc = horner(acc, w, w == plan.W - 1 ? std::min(top, window_width(w, plan.W)) : window_width(w, plan.W));
   }
   return bgh::xyzz_from_jac(acc);
 }
@@ -1281,8 +1267,8 @@ void msm_init_kernels() {
     smem(k_pair_round<Fq, false>, pair_smem_bytes<Fq>());
     smem(k_pair_round<Fq2, true>, pair_smem_bytes<Fq2>());
     smem(k_pair_round<Fq2, false>, pair_smem_bytes<Fq2>());
-    smem(k_window_reduce<Fq>, reduce_sm_bytes<Fq>(256));
-    smem(k_window_reduce<Fq2>, reduce_sm_bytes<Fq2>(256));
+    smem(k_window_reduce<Fq>, reduce_sm_bytes<Fq>(256, 2));
+    smem(k_window_reduce<Fq2>, reduce_sm_bytes<Fq2>(256, 2));
   });
 }
 
@@ -1327,7 +1313,7 @@ namespace {
 
 constexpr size_t kNoAllocMaxPoints = size_t(1) << 14;
 constexpr size_t kNoAllocScratchBytes = size_t(9) << 20;  // the worst case up to 2^14 points needs 6.6 MiB
-constexpr size_t kNoAllocHostWords = 8192;                // window parts copied back for the Horner
+constexpr size_t kNoAllocHostWords = 16384;               // window points copied back for the Horner
 constexpr int kNoAllocMaxDevices = 64;
 
 static __device__ __align__(256) uint8_t g_noalloc_scratch[kNoAllocScratchBytes];
@@ -1371,8 +1357,7 @@ void msm_g1_noalloc(const uint32_t* d_points, const uint32_t* d_scalars, size_t 
   BG_CUDA(cudaGetDevice(&dev));
   BG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   msm_init_kernels();
-  const ReduceShape rsh = reduce_shape<Fq>(nb, W, max_entries, 32, sms, 256u);
-  const uint32_t RT = rsh.RT, M = rsh.M, J = rsh.J;
+  const ReduceShape rsh = reduce_shape<Fq>(nb, W, max_entries, 32, sms, 32u, 256u);
   const unsigned tiles = ceil_div(nkeys + 1, kScanTile);
 
   size_t off = 0;
@@ -1392,8 +1377,8 @@ void msm_g1_noalloc(const uint32_t* d_points, const uint32_t* d_scalars, size_t 
   // 32-entry slices: the fixed array is sized for them
   const BucketScratch bs =
       bucket_scratch<Fq>(max_entries, nkeys, [&](const char*, size_t words) { return carve(words); }, 32);
-  uint32_t* parts = carve((size_t)W * J * 2 * PW);
-  const size_t host_words = (size_t)W * J * 2 * PW;
+  uint32_t* parts = carve(W * reduce_part_points(rsh) * PW);
+  const size_t host_words = W * reduce_points(rsh) * PW;
   if (off > kNoAllocScratchBytes || host_words > kNoAllocHostWords || tiles > (unsigned)kScanTile)
     throw Error(BG_E_ARG, "bg_msm_g1_noalloc: scratch layout exceeds the fixed array");
 
@@ -1418,9 +1403,8 @@ void msm_g1_noalloc(const uint32_t* d_points, const uint32_t* d_scalars, size_t 
   BG_CHECK_LAUNCH();
   bucket_accumulate<Fq>(nullptr, st, d_points, offsets, sorted, (uint32_t)nkeys, max_entries, buckets, bs);
   bucket_heavy<Fq>(nullptr, st, offsets, buckets, bs);
-  k_window_reduce<Fq><<<W * J, RT, reduce_sm_bytes<Fq>(RT), st>>>(offsets, buckets, bs.parts, bs.K, nb, M, J, parts);
-  BG_CHECK_LAUNCH();
-  BG_CUDA(cudaMemcpyAsync(g_noalloc_host_parts, parts, host_words * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+  const uint32_t* sums = window_reduce<Fq>(st, rsh, offsets, buckets, bs, nb, W, parts);
+  BG_CUDA(cudaMemcpyAsync(g_noalloc_host_parts, sums, host_words * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   BG_CUDA(cudaMemcpyAsync(&g_noalloc_host_status, status, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   BG_CUDA(cudaStreamSynchronize(st));
   if (g_noalloc_host_status & BG_DSTATUS_SCALAR_RANGE)
@@ -1428,8 +1412,8 @@ void msm_g1_noalloc(const uint32_t* d_points, const uint32_t* d_scalars, size_t 
   MsmPlan plan;
   plan.c = c;
   plan.W = W;
-  plan.J = J;
-  plan.part_span = RT * M;
+  plan.bits = (int)reduce_points(rsh) - 1;
+  plan.shift = log2_of(rsh.M);
   plan.host_window_sums = g_noalloc_host_parts;
   msm_finish<Fq>(plan, out_aff32);
 }

@@ -12,11 +12,11 @@ struct MsmPlan {
   int c = 0;                              // window bits (0: pick from n)
   int W = 0;                              // windows
   size_t entries = 0;                     // bucket entries (n * W upper bound)
-  uint32_t J = 1;                         // reduction parts per window
-  uint32_t part_span = 1;                 // buckets per part
-  const uint32_t* d_window_sums = nullptr;  // W x J x 2 XYZZ points on the device
+  int bits = 0;                           // sums per window besides T: one per bit of a thread's index
+  int shift = 0;                          // log2 of the buckets per thread, the first such bit's position
+  const uint32_t* d_window_sums = nullptr;  // W x (1 + bits) XYZZ points on the device
   cudaStream_t fetch_stream = nullptr;      // stream the reduction (and the copy) run on
-  // W XYZZ points after msm_fetch, in the context's pinned cache (a pageable destination
+  // those points after msm_fetch, in the context's pinned cache (a pageable destination
   // would make the copy block the host and serialise the streams of a proof)
   uint32_t* host_window_sums = nullptr;
   // false: the reduction runs underneath later work (another MSM's accumulation) and takes
@@ -29,9 +29,6 @@ struct MsmPlan {
   double hidden_us = 0;
   // the accumulation has a stream to itself: its level buffers are not shared with other MSMs'
   bool own_stream = false;
-  // the host pool is otherwise idle when this reduction ends (not one of a small proof's
-  // reductions that end together), so its part sums are priced as the pool runs them
-  bool host_pool_free = false;
 };
 
 // Window table of a fixed point set: row w (w < W) holds 2^(o_w) P_i for all i (o_w the bit

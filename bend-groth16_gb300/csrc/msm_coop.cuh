@@ -2,7 +2,7 @@
 //
 // A window reduction that ends a critical path (a small proof's MSMs, the last MSM of a large
 // one) is a chain of dependent point additions per thread: a bucket's slice pieces, the
-// running sums, the scan and the tree.  One add-2008-s addition is 14 field products, but its
+// running sums and the tree.  One add-2008-s addition is 14 field products, but its
 // dependency depth is about 4.6: six independent products (u1, u2, s1, s2, zz1 zz2,
 // zzz1 zzz2), two squares, three products (ppp, qq, zz3), and zzz3 beside
 // y3 = r (qq - x3) - s1 ppp.  Here the 8 lanes of a group share one addition: each level's
@@ -112,13 +112,14 @@ constexpr size_t coop_group_words() {
 }
 
 // k_window_reduce with one group of 8 lanes in place of each thread (RT groups per CTA, M
-// buckets per group, J parts per bucket set): the same running sums, suffix scan and tree, on
-// cooperative additions; the part's two points out as k_window_reduce writes them.
+// buckets per group, J parts per bucket set): the same running sums and tree, on cooperative
+// additions; the part's points out as k_window_reduce writes them.  With `scan` (M = J = 1) the
+// weighted sum alone.
 template <class F>
 __global__ void __launch_bounds__(256) k_window_reduce_coop(const uint32_t* __restrict__ offsets,
                                                             const uint32_t* __restrict__ buckets,
                                                             const uint32_t* __restrict__ pieces, uint32_t K,
-                                                            uint32_t nb, uint32_t M, uint32_t J,
+                                                            uint32_t nb, uint32_t M, uint32_t J, bool scan,
                                                             uint32_t* __restrict__ out) {
   constexpr int FW = FieldWords<F>::value;
   constexpr int PW = 4 * FW;
@@ -133,8 +134,9 @@ __global__ void __launch_bounds__(256) k_window_reduce_coop(const uint32_t* __re
   uint32_t* const tmp = R + 3 * PW;
   const uint32_t w = blockIdx.x / J, j = blockIdx.x % J;
   const size_t key0 = (size_t)w * nb + ((size_t)j * RT + g) * M;
+  const bool with_t = M > 1;
   coop_set_inf<F>(R, gl, gmask);
-  coop_set_inf<F>(T, gl, gmask);
+  if (with_t) coop_set_inf<F>(T, gl, gmask);
   for (int k = (int)M - 1; k >= 0; k--) {
     const size_t key = key0 + k;
     const uint32_t o0 = offsets[key], o1 = offsets[key + 1];
@@ -152,33 +154,77 @@ __global__ void __launch_bounds__(256) k_window_reduce_coop(const uint32_t* __re
         }
       }
     }
-    coop_add<F>(T, R, tmp, gl, gmask);
+    if (with_t) coop_add<F>(T, R, tmp, gl, gmask);
   }
   __syncthreads();
-  // inclusive suffix scan of R over the groups (Hillis-Steele), through S
-  for (uint32_t dd = 1; dd < RT; dd <<= 1) {
-    if (g + dd < RT) coop_copy<F>(S, R + (size_t)dd * coop_group_words<F>(), gl, gmask);
-    else coop_set_inf<F>(S, gl, gmask);
-    __syncthreads();
-    coop_add<F>(R, S, tmp, gl, gmask);
-    __syncthreads();
-  }
-  // R_j = Suf_0
-  if (g == 0 && gl < 4) store_elem(out + ((size_t)blockIdx.x * 2 + 1) * PW + gl * FW, coop_ld<F>(R + gl * FW));
-  // Y_g = T_g + M Suf_g (g >= 1), Y_0 = T_0; the log2 M doublings on one lane
-  if (g >= 1) {
-    __syncwarp(gmask);
-    if (gl == 0 && M > 1) {
-      XYZZ<F> r = load_xyzz<F>(R);
-      for (uint32_t m = M; m > 1; m >>= 1) r = xyzz_dbl(r);
-      store_xyzz(R, r);
+  // point of column c: R below RT, T from RT up
+  auto col = [&](uint32_t c) {
+    return c < RT ? sm + (size_t)c * coop_group_words<F>() : sm + (size_t)(c - RT) * coop_group_words<F>() + PW;
+  };
+  if (scan) {  // M = J = 1: sum_t (t + 1) R_t, the sum of R's suffix sums
+    for (uint32_t d = 1; d < RT; d <<= 1) {
+      if (g + d < RT) coop_copy<F>(S, col(g + d), gl, gmask);
+      __syncthreads();
+      if (g + d < RT) coop_add<F>(R, S, tmp, gl, gmask);
+      __syncthreads();
     }
-    coop_add<F>(T, R, tmp, gl, gmask);
+    for (uint32_t d = RT >> 1; d >= 1; d >>= 1) {
+      if (g < d) coop_add<F>(R, col(g + d), tmp, gl, gmask);
+      __syncthreads();
+    }
+    for (uint32_t i = threadIdx.x; i < PW; i += blockDim.x) out[(size_t)blockIdx.x * PW + i] = sm[i];
+    return;
   }
-  __syncthreads();
-  for (uint32_t dd = RT >> 1; dd >= 1; dd >>= 1) {
-    if (g < dd) coop_add<F>(T, T + (size_t)dd * coop_group_words<F>(), tmp, gl, gmask);
+  for (uint32_t d = RT >> 1; d >= 1; d >>= 1) {
+    if (g < tree_count(d, RT, with_t)) {
+      const uint32_t c = tree_column(g, d, RT, with_t);
+      coop_add<F>(col(c), col(c + d), tmp, gl, gmask);
+    }
     __syncthreads();
   }
-  if (g == 0 && gl < 4) store_elem(out + (size_t)blockIdx.x * 2 * PW + gl * FW, coop_ld<F>(T + gl * FW));
+  uint32_t lrt = 0;
+  while ((1u << lrt) < RT) lrt++;
+  const uint32_t np = lrt + 1 + (J > 1 ? 1 : 0);
+  uint32_t* o = out + (size_t)blockIdx.x * np * PW;
+  for (uint32_t i = threadIdx.x; i < np * PW; i += blockDim.x) {
+    const uint32_t q = i / PW;
+    const uint32_t c = q == 0 ? (with_t ? RT : 0u) : q <= lrt ? 1u << (q - 1) : 0u;
+    o[i] = col(c)[i % PW];
+  }
+}
+
+// Join of a window's J parts (np points each: T, the U_b, R): one CTA per window and point sums it
+// over the parts in place, on cooperative additions; R by the same tree of sums as inside a part,
+// which leaves a U for each bit of the part's index.  `out`: the window's T, U_b and those.
+template <class F>
+__global__ void __launch_bounds__(256) k_window_join(uint32_t* parts, uint32_t J, uint32_t np, uint32_t* out) {
+  constexpr int FW = FieldWords<F>::value;
+  constexpr int PW = 4 * FW;
+  extern __shared__ __align__(16) uint32_t sm[];
+  const uint32_t groups = blockDim.x / kCoopLanes;
+  const uint32_t g = threadIdx.x / kCoopLanes;
+  const int gl = (int)(threadIdx.x % kCoopLanes);
+  const unsigned gmask = 0xffu << (kCoopLanes * (g & 3u));
+  uint32_t* const tmp = sm + (size_t)g * kCoopTmp * FW;
+  const uint32_t w = blockIdx.x / np, q = blockIdx.x % np;
+  const bool split = q == np - 1;
+  uint32_t* const p0 = parts + ((size_t)w * J * np + q) * PW;
+  auto col = [&](uint32_t j) { return p0 + (size_t)j * np * PW; };
+  for (uint32_t d = J >> 1; d >= 1; d >>= 1) {
+    const uint32_t n = split ? tree_count(d, J, false) : d;
+    for (uint32_t i = g; i < n; i += groups) {
+      const uint32_t c = split ? tree_column(i, d, J, false) : i;
+      coop_add<F>(col(c), col(c + d), tmp, gl, gmask);
+    }
+    __syncthreads();
+  }
+  uint32_t lj = 0;
+  while ((1u << lj) < J) lj++;
+  uint32_t* o = out + (size_t)w * (np - 1 + lj) * PW;
+  if (!split) {
+    for (uint32_t i = threadIdx.x; i < PW; i += blockDim.x) o[q * PW + i] = p0[i];
+  } else {
+    for (uint32_t i = threadIdx.x; i < lj * PW; i += blockDim.x)
+      o[(np - 1) * PW + i] = col(1u << (i / PW))[i % PW];
+  }
 }

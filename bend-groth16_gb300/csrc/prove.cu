@@ -536,7 +536,6 @@ void prove_resident(Ctx& ctx, PkDev& pk, const uint32_t* witness16, const uint32
     // 0.9 ns for G2 inside a proof), which the reduction should not outlast.
     p.latency_critical = overlap || j == 4;
     p.own_stream = overlap;
-    p.host_pool_free = !overlap && !ctx.shared_gpu;
     // (Batch and server lanes keep the fixed rule: other proofs fill the GPU there.)
     p.hidden_us = 0;
     if (!ctx.shared_gpu)
@@ -683,7 +682,7 @@ static size_t msm_footprint_c(size_t n, bool g2, int c) {
   // shortest slices: 3/4 of 32 after whole-wave rounding, 4 in the latency regime
   const size_t K = entries >= (size_t(1) << 21) ? 24 : 4;
   const size_t threads = (entries + K - 1) / K;
-  const size_t J = nb < 32 ? 1 : nb / 32;  // most parts a reduction shape can have (RT >= 32)
+  const size_t J = nb < 32 ? 1 : nb / 32;  // window parts, two points each (more on the few that small sets have)
   // counters, offsets, cursors, entry list, buckets, slice pieces + heavy list, window parts,
   // scan sums
   // batch-affine pair rounds where the model takes them: levels 1 and 2 (affine points, half
