@@ -10,16 +10,16 @@ constexpr int kTuneMinLog2 = 10;
 constexpr int kTuneMaxLog2 = 22;
 // one bucket set per window (standalone MSMs)
 constexpr signed char kTuneSets[2][kTuneMaxLog2 - kTuneMinLog2 + 1] = {
-    {5, 5, 6, 9, 9, 10, 10, 15, 15, 15, 15, 15, 17},
-    {6, 6, 6, 7, 9, 9, 12, 15, 15, 15, 15, 0, 0}};
+    {5, 5, 9, 9, 9, 10, 11, 15, 15, 15, 15, 15, 17},
+    {6, 8, 8, 9, 11, 11, 11, 15, 15, 15, 15, 0, 0}};
 // window tables of resident keys (one shared bucket set)
 constexpr signed char kTuneTables[2][kTuneMaxLog2 - kTuneMinLog2 + 1] = {
-    {10, 11, 11, 13, 13, 15, 15, 15, 18, 18, 17, 0, 0},
-    {11, 11, 13, 12, 12, 15, 15, 15, 18, 18, 17, 0, 0}};
+    {12, 11, 13, 13, 13, 15, 15, 15, 17, 17, 17, 0, 0},
+    {12, 11, 12, 12, 12, 15, 15, 15, 18, 18, 17, 0, 0}};
 // one bucket set per window inside a proof (one-shot proofs): the MSMs share the GPU with
 // each other's reductions and the QAP, which moves the best width from the standalone one
 constexpr signed char kTuneProofSets[2][kTuneMaxLog2 - kTuneMinLog2 + 1] = {
-    {6, 6, 7, 9, 10, 10, 12, 12, 13, 0, 15, 0, 0},
-    {6, 6, 6, 9, 9, 9, 12, 12, 13, 0, 15, 0, 0}};
+    {6, 6, 8, 9, 10, 11, 12, 12, 13, 0, 15, 0, 0},
+    {6, 6, 8, 9, 10, 11, 12, 12, 13, 0, 15, 0, 0}};
 
 }  // namespace bg
