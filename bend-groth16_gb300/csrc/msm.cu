@@ -312,10 +312,9 @@ __global__ void __launch_bounds__(128) k_build_table(const uint32_t* __restrict_
 constexpr uint32_t kPieceLimit = 24;
 // G2's accumulation stages the next entry's point in shared memory (cp.async) instead of
 // registers, where a prefetched Fq2 point held 32 registers across the whole addition: 222
-// registers instead of 242, the G2 accumulation of a 2^18 MSM 2.96 -> 2.93 ms,
-// SquareChain(2^18) 9.88 -> 9.75-9.79 ms, 2^20 34.8 -> 34.4-34.5 ms.  The registers saved do
-// not buy more warps: capped at 200 (10 warps per SM in 64-thread CTAs, a few spills) or 216
-// (9 warps in 32-thread CTAs) the same kernel measured 3.14 / 3.12 ms.  G1 keeps its register
+// registers instead of 242 and 1% of the G2 accumulation.  The registers saved do
+// not buy more warps: with 9, 10 or 12 per SM instead of 8 the accumulation of a 2^18 MSM measured
+// 2.25-2.29 ms against 1.89.  G1 keeps its register
 // prefetch (126 registers, four 128-thread CTAs per SM either way).
 template <class F>
 constexpr bool kAccStaged = FieldWords<F>::value == 16;
@@ -381,8 +380,8 @@ __global__ void __launch_bounds__(kAccThreads<F>) k_bucket_acc(const uint32_t* _
   uint32_t bstart = offsets[b], bend = offsets[b + 1];
   XYZZ<F> acc = xyzz_inf<F>();
   // The next entry's point is gathered before this entry's addition, so the gather's latency
-  // hides behind the arithmetic (G1 accumulation 2^20 3.88 -> 3.82 ms; 126 registers, still
-  // four CTAs per SM): into registers for G1, into one of two shared-memory slots for G2 (the
+  // hides behind the arithmetic (1.5% of a G1 accumulation; four 128-thread CTAs per SM either
+  // way): into registers for G1, into one of two shared-memory slots for G2 (the
   // slot read in this iteration is refilled two iterations later, after the addition that
   // consumed it).
   // sorted == nullptr: the entries are the points themselves (the output of the pair rounds)
@@ -479,22 +478,29 @@ constexpr uint32_t kHeavyGrid = 152;
 
 #include "msm_pairs.cuh"
 
-// Entries per accumulation thread, from a latency model with constants measured on GB300 (G1;
-// G2 scales them alike): a thread's K mixed additions take K x 6.6 us at low occupancy, the
-// whole accumulation cannot beat its throughput (4.58 entries per ns), and a bucket of e
-// entries leaves about e / K + 1 pieces for the reduction (4.5 us each: a 9 us addition, of
-// which half is hidden under other work, fitted to SquareChain(2^12..2^16) proofs).  Large MSMs
-// get 32-entry slices (throughput-bound, fewest pieces); small ones 8 (SquareChain(2^12) proof
-// 2.06 -> 1.69 ms, 2^14 2.44 -> 2.34 ms).
-inline uint32_t slice_entries(size_t max_entries, size_t nkeys, double piece_us = 4.5) {
+// Entries per accumulation thread, from a latency model in dependent mixed additions: a thread's K, or
+// the whole accumulation at its throughput when that is longer, and the e / K pieces that a bucket of e
+// entries leaves for the reduction.  A piece costs more the more buckets there are: one addition where
+// they fit a warp per scheduler, a few where the reduction's additions share the multiplier, fewer in a
+// proof, whose reductions run beside other accumulations.  Against one price per piece and K of 4, 8,
+// 16 or 32: G1 MSMs of 1000 / 12000 / 50000 points 267 / 398 / 625 -> 245 / 370 / 586 us, G2 of 2500 /
+// 10000 601 / 740 -> 566 / 724 us, SquareChain(2^15) 1.44 -> 1.37 ms, 2^16 2.28 -> 2.19.  In a proof K stays a power of
+// two (12 and 24: one-shot 2^11 0.79 -> 0.86 ms, 2^13 1.14 -> 1.21).
+template <class F>
+uint32_t slice_entries(size_t max_entries, size_t nkeys, bool in_proof) {
+  constexpr bool g2 = FieldWords<F>::value == 16;
   const double e = (double)max_entries / (double)(nkeys ? nkeys : 1);
-  const double floor_us = (double)max_entries / 4580.0;
+  const double least = (double)max_entries / (g2 ? 26000.0 : 47000.0);
+  const double per_key = g2 ? 1 / 1000.0 : in_proof ? 1 / 2700.0 : 1 / 600.0;
+  const double most = g2 ? (in_proof ? 1.4 : 13.0) : 3.0;
+  const double piece = std::min(most, std::max(1.0, (double)nkeys * per_key));
   uint32_t best = 32;
-  double best_us = 1e300;
-  for (uint32_t k = 4; k <= 32; k <<= 1) {
-    const double t = std::max(k * 6.6, floor_us) + (e / k + 2.0) * piece_us;
-    if (t < best_us - 1e-9 || (t <= best_us + 1e-9 && k > best)) {
-      best_us = t;
+  double best_t = 1e300;
+  for (uint32_t k : {4u, 6u, 8u, 12u, 16u, 24u, 32u}) {
+    if (in_proof && (k & (k - 1))) continue;
+    const double t = std::max((double)k, least) + e / k * piece;
+    if (t < best_t) {
+      best_t = t;
       best = k;
     }
   }
@@ -546,8 +552,8 @@ double acc_slots() {
 
 // Every slice costs the same K additions, so an accumulation grid of 1.6 waves takes as long
 // as 2.  When the model's slices need more than one wave, K is rounded so that the grid is a
-// whole number of waves (the nearest, at least one): SquareChain(2^18) proof 11.05 -> 10.7 ms,
-// G2 accumulation 2^18 3.25 -> 2.95 ms.  Slices then hold at least 3/4 of the model's K
+// whole number of waves (the nearest, at least one): 9% of the G2 accumulation of a 2^18
+// MSM, whose slices fill 1.6 waves.  Slices then hold at least 3/4 of the model's K
 // (rounding 1.5 waves up to 2 at worst); the model picks K = 32 for every MSM that needs more
 // than a wave and at least 2^21 entries.
 template <class F>
@@ -560,13 +566,10 @@ uint32_t whole_wave_slices(size_t max_entries, uint32_t K) {
 }
 
 template <class F, class Get>
-BucketScratch bucket_scratch(size_t max_entries, size_t nkeys, Get get, uint32_t K = 0) {
+BucketScratch bucket_scratch(size_t max_entries, size_t nkeys, bool in_proof, Get get, uint32_t K = 0) {
   constexpr int PW = 4 * FieldWords<F>::value;
   BucketScratch b;
-  // a G2 piece costs a G2 addition in the reduction: about twice a G1 one relative to the
-  // accumulation's mixed additions (SquareChain(2^12): G2 slices of 16 instead of 8)
-  const double piece_us = FieldWords<F>::value == 16 ? 9.0 : 4.5;
-  b.K = K ? K : whole_wave_slices<F>(max_entries, slice_entries(max_entries, nkeys, piece_us));
+  b.K = K ? K : whole_wave_slices<F>(max_entries, slice_entries<F>(max_entries, nkeys, in_proof));
   const size_t s = bucket_slices(max_entries, b.K);
   b.parts = get("parts", 2 * s * PW);
   b.heavy = get("heavy", s / kPieceLimit + 2);
@@ -1071,7 +1074,7 @@ void msm_accumulate(Ctx& ctx, cudaStream_t st, const std::string& tag, const uin
   }
   plan.entries = acc_entries;
   uint32_t* buckets = ws.get_t<uint32_t>(tag + ".buckets", so.nkeys * PW);
-  const BucketScratch bs = bucket_scratch<F>(acc_entries, so.nkeys, [&](const char* name, size_t words) {
+  const BucketScratch bs = bucket_scratch<F>(acc_entries, so.nkeys, plan.in_proof, [&](const char* name, size_t words) {
     return ws.get_t<uint32_t>(tag + ".slice_" + name, words);
   });
   bucket_accumulate<F>(prof, st, acc_points, acc_offsets, acc_sorted, (uint32_t)so.nkeys, acc_entries, buckets, bs);
@@ -1376,7 +1379,7 @@ void msm_g1_noalloc(const uint32_t* d_points, const uint32_t* d_scalars, size_t 
   uint32_t* buckets = carve(nkeys * PW);
   // 32-entry slices: the fixed array is sized for them
   const BucketScratch bs =
-      bucket_scratch<Fq>(max_entries, nkeys, [&](const char*, size_t words) { return carve(words); }, 32);
+      bucket_scratch<Fq>(max_entries, nkeys, false, [&](const char*, size_t words) { return carve(words); }, 32);
   uint32_t* parts = carve(W * reduce_part_points(rsh) * PW);
   const size_t host_words = W * reduce_points(rsh) * PW;
   if (off > kNoAllocScratchBytes || host_words > kNoAllocHostWords || tiles > (unsigned)kScanTile)

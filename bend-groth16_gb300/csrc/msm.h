@@ -29,6 +29,8 @@ struct MsmPlan {
   double hidden_us = 0;
   // the accumulation has a stream to itself: its level buffers are not shared with other MSMs'
   bool own_stream = false;
+  // one of a proof's MSMs, whose reduction runs beside the others' accumulations
+  bool in_proof = false;
 };
 
 // Window table of a fixed point set: row w (w < W) holds 2^(o_w) P_i for all i (o_w the bit

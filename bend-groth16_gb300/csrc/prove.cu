@@ -536,6 +536,7 @@ void prove_resident(Ctx& ctx, PkDev& pk, const uint32_t* witness16, const uint32
     // 0.9 ns for G2 inside a proof), which the reduction should not outlast.
     p.latency_critical = overlap || j == 4;
     p.own_stream = overlap;
+    p.in_proof = true;
     // (Batch and server lanes keep the fixed rule: other proofs fill the GPU there.)
     p.hidden_us = 0;
     if (!ctx.shared_gpu)
