@@ -967,10 +967,13 @@ void msm_sort(Ctx& ctx, cudaStream_t st, const std::string& tag, const uint32_t*
   const uint32_t idx_stride = shared_set ? (uint32_t)n : 0u;
   size_t max_entries = n * (size_t)W;
   if (max_entries >= 0x80000000ull) throw Error(BG_E_ARG, "msm: n x windows must be below 2^31");
-  // buckets padded for the pair rounds, as many as the padding allows
-  while (rounds > 0 && (nkeys << rounds) > std::max(8 * max_entries, size_t(1) << 20)) rounds--;
-  const size_t padded = max_entries + nkeys * ((size_t(1) << rounds) - 1);
-  if (padded >= 0x80000000ull) throw Error(BG_E_ARG, "msm: n x windows must be below 2^31");
+  // buckets padded for the pair rounds, as many as the padding allows: a few empty slots per entry,
+  // and positions that fit 31 bits
+  auto padded_to = [&](int r) { return max_entries + nkeys * ((size_t(1) << r) - 1); };
+  while (rounds > 0 && ((nkeys << rounds) > std::max(8 * max_entries, size_t(1) << 20) ||
+                        padded_to(rounds) >= 0x80000000ull))
+    rounds--;
+  const size_t padded = padded_to(rounds);
   out.rounds = rounds;
   out.c = c;
   out.W = W;
