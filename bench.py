@@ -13,7 +13,7 @@ runs (bend2/bench/prover_results.md:59).
   e2e    ms/proof through bg_prove_host with every .bin file in pinned host memory: the whole
          upload (all files), the proof and the result reads are inside the timed region.
   roofline  the dominant kernel's algorithmic 32-bit multiply-adds per launch over its
-         CUDA-event duration, against the IMAD rate measured by the library's probe.
+         CUDA-event duration, against the IMAD issue rate (64 per clock and SM).
   cpu_baseline  the C restatement in oracle/ (the reference's Bend/Rust CPU paths cannot
          run here), all host threads, one proof of the same instance, rank 0 at N=1.
 
@@ -39,12 +39,14 @@ UNIT = "ms/proof"
 # the reference's own GPU path (Bend 2 CUDA, RTX 5090) at K=18, T total
 # (bend2/bench/prover_results.md:63, README.md:57)
 REF_GPU_K18_MS = 56083.0
-# 32-bit multiply-adds (mad.lo + mad.hi) the accumulation kernel executes per mixed addition
-# (madd-2008-s), from the products of fp_wide.cuh: a 512-bit Karatsuba product 3 x 32 = 96,
-# a 512-bit square 72, a Montgomery reduction 8 x 17 = 136.  Fq product 232, square 208,
+# The unit of work: 32-bit multiply-adds (a low or a high half each) of a mixed addition
+# (madd-2008-s), counted on the product with the fewest of them: a 512-bit Karatsuba product 3 x 32 =
+# 96, a 512-bit square 72, a Montgomery reduction 8 x 17 = 136.  Fq product 232, square 208,
 # u v - w z 2 x 96 + 136 = 328.  G1: 6 products + 2 squares + Y3 = 2136.  G2 (Fq2 product 3 x 96
 # + 2 x 136 = 560, square = 2 Fq products, u v - w z 6 x 96 + 2 x 136 = 848): 6 x 560 +
-# 2 x 464 + 848 = 5136.
+# 2 x 464 + 848 = 5136.  The kernels execute a few more (schoolbook, 264 per Fq product, in 128
+# two-half instructions and 8 low ones), which take 528 cycles of a scheduler against 928 for 232
+# separate halves: the unit understates what they do, never the reverse.
 MADD_G1_IMAD = 6 * (96 + 136) + 2 * (72 + 136) + (2 * 96 + 136)
 MADD_G2_IMAD = 6 * (3 * 96 + 2 * 136) + 2 * 2 * (96 + 136) + (6 * 96 + 2 * 136)
 # per affine pair addition of the batch-affine rounds (msm_pairs.cuh): three products of the
@@ -52,6 +54,8 @@ MADD_G2_IMAD = 6 * (3 * 96 + 2 * 136) + 2 * 2 * (96 + 136) + (6 * 96 + 2 * 136)
 # and y3: 5 products + 1 square.  G1: 5 x 232 + 208 = 1368; G2: 5 x 560 + 464 = 3264.
 PAIR_G1_IMAD = 5 * (96 + 136) + (72 + 136)
 PAIR_G2_IMAD = 5 * (3 * 96 + 2 * 136) + 2 * (96 + 136)
+IMAD_PEAK_SOURCE = ("64 multiply-adds per clock and SM at the maximum SM clock, the rate of the fused 64-bit form; "
+                    "separate mad.lo / mad.hi chains (bg_probe_imad) reach about 0.65 of it")
 KERNEL_FAMILIES = ["msm_pair_g1", "msm_pair_g2", "msm_bucket_acc_g1", "msm_bucket_acc_g2", "msm_heavy_g1",
                    "msm_heavy_g2", "msm_reduce_g1", "msm_reduce_g2", "msm_digits", "msm_scatter", "ntt_pass"]
 
@@ -242,10 +246,10 @@ def run_ours(args, dist: Dist):
             if i >= max(3, args.warmup):
                 out.append(e0.elapsed_time(e1))
         ms = statistics.median(out)
-        ops, pms = ctx.probe_imad(0, 4096)
+        peak = imad_rate(ctx)
         ctx.close()
         return {"metric": "NTT 2^20 forward ms", "value": round(ms, 4), "unit": "ms", "higher_is_better": False,
-                "roofline": ntt_roofline(20, round(ms, 4), ops / (pms * 1e-3))}
+                "roofline": ntt_roofline(20, round(ms, 4), peak)}
     path = ensure_instance(args, dist, lambda k, s, p: ctx.synth_square_chain(k, s, p))
     files = bendg.HostFiles(path, pinned=True)
     hdr = files.words("header")
@@ -255,9 +259,8 @@ def run_ours(args, dist: Dist):
         import torch
         flush = torch.empty(512 << 20, dtype=torch.uint8, device="cuda")
         ext = torch.cuda.ExternalStream(ctx.stream)
-        ops, ms = ctx.probe_imad(0, 4096)
         ctx.pair_rounds_override(args.pair_rounds)
-        prims = primitives(ctx, files, nh, nb, args, ext, flush, ops / (ms * 1e-3), only_g1=True)
+        prims = primitives(ctx, files, nh, nb, args, ext, flush, imad_rate(ctx), only_g1=True)
         ctx.close()
         key = "g1_msm_2^%d_ms" % args.msm_log2n
         return {"metric": "G1 MSM 2^%d ms" % args.msm_log2n, "value": prims[key], "unit": "ms",
@@ -276,9 +279,8 @@ def run_ours(args, dist: Dist):
 
     for _ in range(max(3, args.warmup)):
         step_resident()
-    # IMAD peak of this GPU, measured before the timed region
-    ops, ms = ctx.probe_imad(0, 4096)
-    imad_peak = ops / (ms * 1e-3)
+    # IMAD peak of this GPU, before the timed region
+    imad_peak = imad_rate(ctx)
     ops_f, ms_f = ctx.probe_imad(1, 256)
     fqmul_rate = ops_f / (ms_f * 1e-3)
 
@@ -322,13 +324,14 @@ def run_ours(args, dist: Dist):
     fams = KERNEL_FAMILIES
     stats = {f: ctx.kernel_stats(f) for f in fams}
     ctx.profile(False)
-    dom = "msm_bucket_acc_g1"
+    # the G1 accumulations: batch-affine pair rounds where the library takes them inside the proof
+    # (two rounds: three quarters of the entries in pair additions, the rest mixed additions)
     g1_sizes = [na, nb, nh, nl]
     # the timed proofs run against the resident key: window tables, W = floor(254 / c_table) + 1
     entries_g1 = sum(n * table_window_counts(L, n)[1] for n in g1_sizes)
-    entries_g2 = nb * table_window_counts(L, nb, 1)[1]
-    work = {"msm_bucket_acc_g1": entries_g1 * MADD_G1_IMAD,
-            "msm_bucket_acc_g2": entries_g2 * MADD_G2_IMAD}
+    paired = stats["msm_pair_g1"][0] > 0
+    dom = "msm_pair_g1" if paired else "msm_bucket_acc_g1"
+    work = {"msm_pair_g1": entries_g1 * 3 // 4 * PAIR_G1_IMAD, "msm_bucket_acc_g1": entries_g1 * MADD_G1_IMAD}
     roof = None
     if dom in work:
         nl_, tms = stats[dom]
@@ -343,8 +346,9 @@ def run_ours(args, dist: Dist):
                 "bound": "imad", "achieved": round(achieved, 1), "peak": round(imad_peak / 1e9, 1),
                 "unit": "Gimad/s", "frac": round(achieved / (imad_peak / 1e9), 4), "traffic": traffic,
                 "work_per_launch": per_launch_work, "avg_launch_ms": round(avg_ms, 4),
-                "peak_source": "bg_probe_imad on this GPU (32-bit mad.lo/mad.hi chains)",
-                "work_model": "entries x %d IMAD per G1 mixed add (G2: %d)" % (MADD_G1_IMAD, MADD_G2_IMAD)}
+                "peak_source": IMAD_PEAK_SOURCE,
+                "work_model": ("entries x 3/4 x %d IMAD per G1 pair addition" % PAIR_G1_IMAD if paired else
+                               "entries x %d IMAD per G1 mixed addition" % MADD_G1_IMAD)}
     kernel_ms = {f: {"launches": v[0], "ms_per_proof": round(v[1] / args.steps, 3)} for f, v in stats.items()}
 
     # e2e: all .bin files from pinned host memory through bg_prove_host, every step (after the
@@ -461,6 +465,20 @@ def shifted_witness(z_words, m: int):
     return np.concatenate([w[0:1], head, w[2 + m:], tail]).reshape(-1)
 
 
+def imad_rate(ctx) -> float:
+    """multiply-adds per second at the nominal issue rate and maximum SM clock, or the library's
+    probe of separate halves where that measures more or the clock cannot be read"""
+    import torch
+    ops, ms = ctx.probe_imad(0, 4096)
+    probe = ops / (ms * 1e-3)
+    try:
+        mhz = float(subprocess.run(["nvidia-smi", "--query-gpu=clocks.max.sm", "--format=csv,noheader,nounits"],
+                                   capture_output=True, text=True, timeout=20).stdout.split()[0])
+    except (OSError, IndexError, ValueError, subprocess.SubprocessError):
+        return probe
+    return max(probe, 64.0 * torch.cuda.get_device_properties(0).multi_processor_count * mhz * 1e6)
+
+
 def proof_imad(L, hdr) -> int:
     """algorithmic 32-bit multiply-adds of one resident-key proof: every MSM entry one mixed
     addition (n W per MSM with W the window-table rows: G1 2136, G2 5136 IMAD) and the 7 NTTs of
@@ -544,7 +562,7 @@ def batched(ctx, args, flush, ext, imad_peak=None):
                 "frac_needed_for_2x_plain": round(2 * work / (t_plain * 1e-3) / imad_peak, 4),
                 "model": "per proof: MSM entries (n W with the window-table W) x 2136 (G1) / 5136 (G2) IMAD + "
                          "7 NTTs x (d/2) log2 d x 232; reductions left out (a lower bound)",
-                "best_kernel_frac_alone": "the XYZZ accumulation reaches 0.76 of the probe running alone "
+                "best_kernel_frac_alone": "the XYZZ accumulation reaches 0.77 of the peak running alone "
                                           "(G1 MSM 2^20, one bucket set per window)"}
     return {"workload": "64 SquareChain proofs, K drawn from %s with weights %s (seed %d), resident keys"
                         % (list(BATCH_KS), list(BATCH_WEIGHTS), args.seed + 3),
@@ -832,7 +850,7 @@ def primitives(ctx, files, nh, nb, args, ext, flush, imad_peak, only_g1=False):
                        "bound": "imad", "achieved": round(achieved, 1), "peak": round(imad_peak / 1e9, 1),
                        "unit": "Gimad/s", "frac": round(achieved / (imad_peak / 1e9), 4), "traffic": traffic,
                        "work_per_launch": work, "avg_launch_ms": round(avg, 4), "launches": launches,
-                       "peak_source": "bg_probe_imad on this GPU (32-bit mad.lo/mad.hi chains)",
+                       "peak_source": IMAD_PEAK_SOURCE,
                        "work_model": model,
                        "accumulation_after_rounds_ms": round(stats["msm_bucket_acc_g1"][1] /
                                                              max(1, stats["msm_bucket_acc_g1"][0]), 4),
@@ -885,7 +903,7 @@ def ntt_roofline(lg, ms, imad_peak):
     bound = "imad" if t_hbm is None or t_imad >= t_hbm else "hbm"
     return {"n": n, "ms": ms, "bound": bound,
             "imad": {"work": work, "bound_ms": round(t_imad, 4), "achieved_gimad_s": round(work / (ms * 1e-3) / 1e9, 1),
-                     "frac": round(t_imad / ms, 4), "peak_source": "bg_probe_imad"},
+                     "frac": round(t_imad / ms, 4), "peak_source": IMAD_PEAK_SOURCE},
             "hbm": {"min_bytes": min_bytes, "bound_ms": round(t_hbm, 4) if t_hbm else None,
                     "moved_bytes_2_pass_plan": 2 * min_bytes,
                     "achieved_gbs": round(2 * min_bytes / (ms * 1e-3) / 1e9, 1),
