@@ -1175,8 +1175,9 @@ int msm_pick_c_table(size_t n, bool g2) {
   if (const int t = tuned(kTuneTables, n, g2)) return t;
   const int lg = floor_log2(n);
   // the smallest proofs are bound by the chains of their reductions, whose length is the entries per
-  // bucket: SquareChain(2^8) 0.54 ms at 7 bits, 0.44 at 10; 2^9 0.53 ms at 8, 0.46 at 10 and 11
-  if (lg == 8 || lg == 9) return g2 ? lg + 2 : 10;
+  // bucket: SquareChain(2^5) 0.388 ms at 6 bits, 0.330 at 8; 2^6 0.427 at 6, 0.344 at 9; 2^7 0.520 at 6,
+  // 0.358 at 10 and 11; 2^8 0.377 at 10, 0.367 at 11; 2^9 0.424 at 10, 0.397 at 11; below 2^5 level
+  if (lg <= 9) return std::min(11, std::max(7, lg + 3));
   return std::min(18, std::max(6, lg - 1));
 }
 
