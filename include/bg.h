@@ -240,13 +240,13 @@ int bg_msm_window_override(bg_ctx* ctx, int layout, int curve, int c);
 int bg_msm_pair_rounds(size_t n, int curve);
 /* Tuning hook: the number of batch-affine pair rounds before each later MSM's bucket
  * accumulation on this context and its batch lanes (each round adds the points of every bucket
- * in pairs, in affine coordinates, sharing one field inversion per CTA); -1 restores the
+ * in pairs, in affine coordinates, sharing field inversions in a CTA); -1 restores the
  * library's cost model, 0 turns the rounds off, at most 12.  Results do not depend on it. */
 int bg_msm_pair_rounds_override(bg_ctx* ctx, int rounds);
 /* Tuning hook: the window reductions that end a critical path (standalone MSMs, a proof's last
  * MSM, every MSM of a small proof) may run each point addition on a group of 8 cooperating
  * lanes; mode -1 lets the library's latency model choose (the default), 0 never, 1 always
- * (for those reductions).  Results do not depend on it. */
+ * (for those reductions, up to 4096 parts in all).  Results do not depend on it. */
 int bg_msm_coop_reduce_override(bg_ctx* ctx, int mode);
 
 /* ---- measurement (no counterpart in the reference, which prints only T lines) ------- */
