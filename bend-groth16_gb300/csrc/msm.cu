@@ -565,10 +565,39 @@ uint32_t whole_wave_slices(size_t max_entries, uint32_t K) {
   return (uint32_t)std::ceil((double)max_entries / (rounded * slots));
 }
 
+// A standalone MSM's K where its slices do not fill the GPU.  The accumulation lasts as long as the SM
+// with the most CTAs, K additions each at a price that depends on how many share it, so the good K are
+// those whose grid just fits 1, 2, ... CTAs on every SM (G1 44236 points, 281 / 321 / 375 / 450 CTAs on
+// 152 SMs: 532 / 602 / 571 / 554 us; G2 32768 points 256 / 307 CTAs: 1028 / 1162 us); the pieces priced
+// as in slice_entries.  With K of 4, 6, 8, 12, 16, 24 or 32 whatever the grid: G2 32768 points 1140 us.
+template <class F>
+uint32_t level_slices(size_t max_entries, size_t nkeys) {
+  constexpr bool g2 = FieldWords<F>::value == 16;
+  constexpr int kResident = g2 ? 2 : 4;  // CTAs per SM
+  // an addition with 1 .. kResident CTAs on the SM, in those of one alone
+  const double price[4] = {1.0, g2 ? 1.28 : 1.2, 1.7, 2.26};
+  const double piece = std::min(g2 ? 8.0 : 4.5, std::max(1.0, (double)nkeys / (g2 ? 3300.0 : 600.0)));
+  const double e = (double)max_entries / (double)(nkeys ? nkeys : 1);
+  const double sms = std::max(1.0, acc_slots<F>() / (kResident * kAccThreads<F>));
+  uint32_t best = 32;
+  double best_t = 1e300;
+  for (uint32_t k = 4; k <= 48; k++) {
+    const double ctas = std::ceil(std::ceil((double)max_entries / k) / kAccThreads<F>);
+    const double level = std::ceil(ctas / sms), waves = std::ceil(level / kResident);
+    const double t = k * waves * price[(int)std::min<double>(level, kResident) - 1] + e / k * piece;
+    if (t < best_t) {
+      best_t = t;
+      best = k;
+    }
+  }
+  return best;
+}
+
 template <class F, class Get>
 BucketScratch bucket_scratch(size_t max_entries, size_t nkeys, bool in_proof, Get get, uint32_t K = 0) {
   constexpr int PW = 4 * FieldWords<F>::value;
   BucketScratch b;
+  if (!K && !in_proof && max_entries < (size_t(1) << 21)) K = level_slices<F>(max_entries, nkeys);
   b.K = K ? K : whole_wave_slices<F>(max_entries, slice_entries<F>(max_entries, nkeys, in_proof));
   const size_t s = bucket_slices(max_entries, b.K);
   b.parts = get("parts", 2 * s * PW);
