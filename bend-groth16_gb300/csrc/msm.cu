@@ -478,26 +478,22 @@ constexpr uint32_t kHeavyGrid = 152;
 
 #include "msm_pairs.cuh"
 
-// Entries per accumulation thread, from a latency model in dependent mixed additions: a thread's K, or
-// the whole accumulation at its throughput when that is longer, and the e / K pieces that a bucket of e
-// entries leaves for the reduction.  A piece costs more the more buckets there are: one addition where
-// they fit a warp per scheduler, a few where the reduction's additions share the multiplier, fewer in a
-// proof, whose reductions run beside other accumulations.  Against one price per piece and K of 4, 8,
-// 16 or 32: G1 MSMs of 1000 / 12000 / 50000 points 267 / 398 / 625 -> 245 / 370 / 586 us, G2 of 2500 /
-// 10000 601 / 740 -> 566 / 724 us, SquareChain(2^15) 1.44 -> 1.37 ms, 2^16 2.28 -> 2.19.  In a proof K stays a power of
-// two (12 and 24: one-shot 2^11 0.79 -> 0.86 ms, 2^13 1.14 -> 1.21).
+// Entries per accumulation thread in a proof and for MSMs that fill the GPU, from a latency model in
+// dependent mixed additions: a thread's K, or the whole accumulation at its throughput when that is
+// longer (then 32, the fewest pieces), and the e / K pieces that a bucket of e entries leaves for the
+// reduction.  A piece costs more the more buckets share the multiplier, and little in all, since the
+// reductions run beside other accumulations.  Against one price per piece: SquareChain(2^12) 0.622 ->
+// 0.608 ms, 2^15 1.44 -> 1.37, 2^16 2.28 -> 2.19.  K stays a power of two (12 and 24 too: one-shot 2^11
+// 0.79 -> 0.86 ms, 2^13 1.14 -> 1.21).
 template <class F>
-uint32_t slice_entries(size_t max_entries, size_t nkeys, bool in_proof) {
+uint32_t slice_entries(size_t max_entries, size_t nkeys) {
   constexpr bool g2 = FieldWords<F>::value == 16;
   const double e = (double)max_entries / (double)(nkeys ? nkeys : 1);
   const double least = (double)max_entries / (g2 ? 26000.0 : 47000.0);
-  const double per_key = g2 ? 1 / 1000.0 : in_proof ? 1 / 2700.0 : 1 / 600.0;
-  const double most = g2 ? (in_proof ? 1.4 : 13.0) : 3.0;
-  const double piece = std::min(most, std::max(1.0, (double)nkeys * per_key));
+  const double piece = std::min(g2 ? 1.4 : 3.0, std::max(1.0, (double)nkeys / (g2 ? 1000.0 : 2700.0)));
   uint32_t best = 32;
   double best_t = 1e300;
-  for (uint32_t k : {4u, 6u, 8u, 12u, 16u, 24u, 32u}) {
-    if (in_proof && (k & (k - 1))) continue;
+  for (uint32_t k = 4; k <= 32; k <<= 1) {
     const double t = std::max((double)k, least) + e / k * piece;
     if (t < best_t) {
       best_t = t;
@@ -568,8 +564,10 @@ uint32_t whole_wave_slices(size_t max_entries, uint32_t K) {
 // A standalone MSM's K where its slices do not fill the GPU.  The accumulation lasts as long as the SM
 // with the most CTAs, K additions each at a price that depends on how many share it, so the good K are
 // those whose grid just fits 1, 2, ... CTAs on every SM (G1 44236 points, 281 / 321 / 375 / 450 CTAs on
-// 152 SMs: 532 / 602 / 571 / 554 us; G2 32768 points 256 / 307 CTAs: 1028 / 1162 us); the pieces priced
-// as in slice_entries.  With K of 4, 6, 8, 12, 16, 24 or 32 whatever the grid: G2 32768 points 1140 us.
+// 152 SMs: 532 / 602 / 571 / 554 us; G2 32768 points 256 / 307 CTAs: 1028 / 1162 us); a piece
+// costs one addition where the buckets fit a warp per scheduler, several where many share the multiplier.
+// With K of 4, 6, 8, 12, 16, 24 or 32 whatever the grid G2 32768 points measured 1140 us, here 989; G1
+// 1000 points 241 and 240, where one price per piece and K of 4, 8, 16 or 32 measured 267.
 template <class F>
 uint32_t level_slices(size_t max_entries, size_t nkeys) {
   constexpr bool g2 = FieldWords<F>::value == 16;
@@ -598,7 +596,7 @@ BucketScratch bucket_scratch(size_t max_entries, size_t nkeys, bool in_proof, Ge
   constexpr int PW = 4 * FieldWords<F>::value;
   BucketScratch b;
   if (!K && !in_proof && max_entries < (size_t(1) << 21)) K = level_slices<F>(max_entries, nkeys);
-  b.K = K ? K : whole_wave_slices<F>(max_entries, slice_entries<F>(max_entries, nkeys, in_proof));
+  b.K = K ? K : whole_wave_slices<F>(max_entries, slice_entries<F>(max_entries, nkeys));
   const size_t s = bucket_slices(max_entries, b.K);
   b.parts = get("parts", 2 * s * PW);
   b.heavy = get("heavy", s / kPieceLimit + 2);
