@@ -174,10 +174,17 @@ inline __attribute__((always_inline)) Fe fe_wide_redc(const Mod& m, const uint64
   return fe_cond_sub(m, r);
 }
 inline Fe fe_sqr(const Mod& m, const Fe& a) { return fe_mul(m, a, a); }
+// (any 256-bit a)
 inline Fe fe_to_mont(const Mod& m, const Fe& a) {
-  return fe_mul(m, a, Fe{{m.r2[0], m.r2[1], m.r2[2], m.r2[3]}});
+  return fe_mul(m, Fe{{m.r2[0], m.r2[1], m.r2[2], m.r2[3]}}, a);
 }
-inline Fe fe_from_mont(const Mod& m, const Fe& a) { return fe_mul(m, a, fe_raw(1)); }
+inline Fe fe_from_mont(const Mod& m, const Fe& a) { return fe_mul(m, fe_raw(1), a); }
+// a mod p for any 256-bit a: what a caller's words become before the arithmetic here, whose first
+// factors have to be below p
+inline Fe fe_reduce(const Mod& m, Fe a) {
+  while (geq(a.v, m.p)) sub4(a.v, a.v, m.p);  // at most five times
+  return a;
+}
 
 inline Fe fe_pow(const Mod& m, const Fe& a, const uint64_t e[4]) {
   Fe r = fe_one(m);
@@ -567,6 +574,28 @@ Aff<F> aff_from_words32(const uint32_t* w) {
   elem_from_words32<F>(a.y, w + F::WORDS);
   a.inf = F::is_zero(a.x) && F::is_zero(a.y);
   return a;
+}
+// the same from a caller's words, whose coordinates may lie at or above p
+inline void elem_reduce(Fe& a) { a = fe_reduce(FQ, a); }
+inline void elem_reduce(Fe2& a) { a = {fe_reduce(FQ, a.c0), fe_reduce(FQ, a.c1)}; }
+template <class F>
+Aff<F> aff_from_input32(const uint32_t* w) {
+  Aff<F> a = aff_from_words32<F>(w);
+  elem_reduce(a.x);
+  elem_reduce(a.y);
+  return a;
+}
+// A proof's blinding scalars r, s and r s, canonical, from their 16-word Montgomery form (rs.bin: r,
+// then s; words at or above the modulus are taken modulo it)
+inline void blinding_scalars(const uint32_t* rs16, uint64_t r[4], uint64_t s[4], uint64_t rs[4]) {
+  const Fe rm = fe_from_words16(rs16), sm = fe_from_words16(rs16 + 16);
+  const Fe rc = fe_from_mont(FR, rm), sc = fe_from_mont(FR, sm);
+  const Fe prod = fe_mul(FR, rc, sm);
+  for (int i = 0; i < 4; i++) {
+    r[i] = rc.v[i];
+    s[i] = sc.v[i];
+    rs[i] = prod.v[i];
+  }
 }
 template <class F>
 void aff_to_words32(uint32_t* w, const Aff<F>& a) {

@@ -156,7 +156,7 @@ static Aff<H> host_affine_from_wire(const uint32_t* w16) {
   for (int i = 0; i < 2 * H::WORDS; i++) {
     packed[i] = (w16[2 * i] & 0xffffu) | (w16[2 * i + 1] << 16);
   }
-  return bgh::aff_from_words32<H>(packed);
+  return bgh::aff_from_input32<H>(packed);
 }
 
 static void* dmalloc(size_t bytes) {
@@ -380,12 +380,6 @@ void pk_free(PkDev* pk) {
 }
 
 // ---------------------------------------------------------------- combine (host)
-static void scalar_from_mont_wire(const uint32_t* w16, uint64_t out[4]) {
-  const Fe m = bgh::fe_from_words16(w16);
-  const Fe c = bgh::fe_from_mont(bgh::FR, m);
-  for (int i = 0; i < 4; i++) out[i] = c.v[i];
-}
-
 template <class H>
 static void wire_from_affine(uint32_t* w16, const Aff<H>& a) {
   uint32_t packed[2 * H::WORDS];
@@ -429,13 +423,7 @@ void prove_resident(Ctx& ctx, PkDev& pk, const uint32_t* witness16, const uint32
   // operations; with a resident key each splits into four 64-bit pieces over precomputed
   // 2^(64 j) delta.
   uint64_t r[4], s[4], rs[4];
-  scalar_from_mont_wire(rs16, r);
-  scalar_from_mont_wire(rs16 + 16, s);
-  {
-    const Fe rm = bgh::fe_from_words16(rs16), sm = bgh::fe_from_words16(rs16 + 16);
-    const Fe prod = bgh::fe_from_mont(bgh::FR, bgh::fe_mul(bgh::FR, rm, sm));
-    for (int i = 0; i < 4; i++) rs[i] = prod.v[i];
-  }
+  bgh::blinding_scalars(rs16, r, s, rs);
   const uint64_t* const ks[3] = {r, s, rs};
   const int pieces = pk.delta_pow_ready ? 4 : 1;
   Xyzz<FqOps> piece[3][4];
