@@ -306,10 +306,9 @@ __global__ void __launch_bounds__(128) k_build_table(const uint32_t* __restrict_
 // entries [o, o') cut into slices t0 = o / K .. t1 = (o' - 1) / K has its pieces at 2 t0 + 1
 // and 2 u for t0 < u <= t1; the window reduction adds them where it reads the
 // bucket, which costs the same additions as a separate join pass without its launch
-// and its mostly idle lanes.  A bucket of more than kPieceLimit + 1 pieces (a scalar value
+// and its mostly idle lanes.  A bucket of more than `limit` + 1 pieces (piece_limit; a scalar value
 // repeated thousands of times) is joined beforehand by k_bucket_heavy: the thread that owns its
 // first piece lists it in heavy[1 + i] (heavy[0] counts, cleared before the accumulation).
-constexpr uint32_t kPieceLimit = 24;
 // G2's accumulation stages the next entry's point in shared memory (cp.async) instead of
 // registers, where a prefetched Fq2 point held 32 registers across the whole addition: 222
 // registers instead of 242 and 1% of the G2 accumulation.  The registers saved do
@@ -357,7 +356,8 @@ template <class F>
 __global__ void __launch_bounds__(kAccThreads<F>) k_bucket_acc(const uint32_t* __restrict__ points,
                                                                const uint32_t* __restrict__ offsets,
                                                                const uint32_t* __restrict__ sorted, uint32_t nbuckets,
-                                                               uint32_t K, uint32_t* __restrict__ buckets,
+                                                               uint32_t K, uint32_t limit,
+                                                               uint32_t* __restrict__ buckets,
                                                                uint32_t* __restrict__ parts, uint32_t* __restrict__ heavy) {
   constexpr int FW = FieldWords<F>::value;
   constexpr int PW = 4 * FW;
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(kAccThreads<F>) k_bucket_acc(const uint32_t* _
       if (bstart < beg || bend > end) {
         const size_t slot = 2 * (size_t)t + (bstart < beg ? 0 : 1);
         store_xyzz(parts + slot * PW, acc);
-        if (bstart >= beg && (bend - 1) / K - t > kPieceLimit) heavy[1 + atomicAdd(heavy, 1u)] = b;
+        if (bstart >= beg && (bend - 1) / K - t > limit) heavy[1 + atomicAdd(heavy, 1u)] = b;
       } else {
         store_xyzz(buckets + (size_t)b * PW, acc);
       }
@@ -524,11 +524,23 @@ double pair_slots() {
   return s;
 }
 
+// Pieces after the first from which a bucket goes to k_bucket_heavy, whose tree costs its eight
+// additions whatever the count.  The reduction adds a bucket's pieces one after another, M buckets
+// per thread, and its shape counts on the e / K that a bucket of e = max_entries / nkeys entries
+// leaves: three times that and four more are what evenly spread scalars never reach, 24 the most.
+// With 24 alone, scalars of 8 bits put up to 20 pieces into each of the 255 lowest buckets where the
+// shape counts on one: MSMs of 131072 such scalars took 1.29 ms in G1 and 3.39 in G2, 0.50 and 1.01 now.
+inline uint32_t piece_limit(size_t max_entries, size_t nkeys, uint32_t K) {
+  const size_t mean = max_entries / ((nkeys ? nkeys : 1) * K);
+  return (uint32_t)std::min<size_t>(24, 4 + 3 * mean);
+}
+
 // Scratch of the bucket phase for at most max_entries entries (words): pieces and the heavy list.
 struct BucketScratch {
   uint32_t K = 32;            // entries per accumulation thread
+  uint32_t limit = 24;        // piece_limit
   uint32_t* parts = nullptr;  // 2 x slices XYZZ points
-  uint32_t* heavy = nullptr;  // 1 + slices / kPieceLimit + 1
+  uint32_t* heavy = nullptr;  // 1 + slices / limit + 1
 };
 inline size_t bucket_slices(size_t max_entries, uint32_t K) { return (max_entries + K - 1) / K; }
 
@@ -598,8 +610,9 @@ BucketScratch bucket_scratch(size_t max_entries, size_t nkeys, bool in_proof, Ge
   if (!K && !in_proof && max_entries < (size_t(1) << 21)) K = level_slices<F>(max_entries, nkeys);
   b.K = K ? K : whole_wave_slices<F>(max_entries, slice_entries<F>(max_entries, nkeys));
   const size_t s = bucket_slices(max_entries, b.K);
+  b.limit = piece_limit(max_entries, nkeys, b.K);
   b.parts = get("parts", 2 * s * PW);
-  b.heavy = get("heavy", s / kPieceLimit + 2);
+  b.heavy = get("heavy", s / b.limit + 2);
   return b;
 }
 
@@ -613,7 +626,7 @@ void bucket_accumulate(Ctx* prof, cudaStream_t st, const uint32_t* points, const
   BG_CUDA(cudaMemsetAsync(s.heavy, 0, sizeof(uint32_t), st));
   std::unique_ptr<KernelTimer> kt(prof ? new KernelTimer(*prof, FW == 8 ? "msm_bucket_acc_g1" : "msm_bucket_acc_g2", st)
                                        : nullptr);
-  k_bucket_acc<F><<<ceil_div(slices, kAccThreads<F>), kAccThreads<F>, 0, st>>>(points, offsets, sorted, nkeys, s.K, buckets, s.parts,
+  k_bucket_acc<F><<<ceil_div(slices, kAccThreads<F>), kAccThreads<F>, 0, st>>>(points, offsets, sorted, nkeys, s.K, s.limit, buckets, s.parts,
                                                          s.heavy);
   BG_CHECK_LAUNCH();
 }
@@ -717,8 +730,8 @@ BG_DEV uint32_t tree_count(uint32_t d, uint32_t RT, bool with_t) {
 template <class F>
 __global__ void __launch_bounds__(256)
     k_window_reduce(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ buckets,
-                    const uint32_t* __restrict__ pieces, uint32_t K, uint32_t nb, uint32_t M, uint32_t J,
-                    uint32_t* __restrict__ out) {
+                    const uint32_t* __restrict__ pieces, uint32_t K, uint32_t limit, uint32_t nb, uint32_t M,
+                    uint32_t J, uint32_t* __restrict__ out) {
   constexpr int PW = 4 * FieldWords<F>::value;
   extern __shared__ uint32_t sm[];
   const uint32_t RT = blockDim.x;
@@ -736,7 +749,7 @@ __global__ void __launch_bounds__(256)
     const uint32_t o0 = offsets[key], o1 = offsets[key + 1];
     if (o1 != o0) {
       const uint32_t t0 = o0 / K, t1 = (o1 - 1) / K;
-      if (t0 == t1 || t1 - t0 > kPieceLimit) {
+      if (t0 == t1 || t1 - t0 > limit) {
         pt_add_into<F>(R, RT, buckets + key * PW, 1);
       } else {
         pt_add_into<F>(R, RT, pieces + (2 * (size_t)t0 + 1) * PW, 1);
@@ -934,10 +947,10 @@ uint32_t* window_reduce(cudaStream_t st, const ReduceShape& r, const uint32_t* o
   constexpr int PW = 4 * FieldWords<F>::value;
   if (r.coop)
     k_window_reduce_coop<F><<<sets * r.J, r.RT * kCoopLanes, r.RT * coop_group_words<F>() * sizeof(uint32_t), st>>>(
-        offsets, buckets, bs.parts, bs.K, nb, r.M, r.J, r.scan, parts);
+        offsets, buckets, bs.parts, bs.K, bs.limit, nb, r.M, r.J, r.scan, parts);
   else
-    k_window_reduce<F><<<sets * r.J, r.RT, reduce_sm_bytes<F>(r.RT, r.M), st>>>(offsets, buckets, bs.parts, bs.K, nb,
-                                                                               r.M, r.J, parts);
+    k_window_reduce<F><<<sets * r.J, r.RT, reduce_sm_bytes<F>(r.RT, r.M), st>>>(offsets, buckets, bs.parts, bs.K,
+                                                                               bs.limit, nb, r.M, r.J, parts);
   BG_CHECK_LAUNCH();
   if (r.J == 1) return parts;
   const int np = 2 + log2_of(r.RT);

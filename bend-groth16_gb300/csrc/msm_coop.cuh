@@ -118,7 +118,7 @@ constexpr size_t coop_group_words() {
 template <class F>
 __global__ void __launch_bounds__(256) k_window_reduce_coop(const uint32_t* __restrict__ offsets,
                                                             const uint32_t* __restrict__ buckets,
-                                                            const uint32_t* __restrict__ pieces, uint32_t K,
+                                                            const uint32_t* __restrict__ pieces, uint32_t K, uint32_t limit,
                                                             uint32_t nb, uint32_t M, uint32_t J, bool scan,
                                                             uint32_t* __restrict__ out) {
   constexpr int FW = FieldWords<F>::value;
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(256) k_window_reduce_coop(const uint32_t* __re
     const uint32_t o0 = offsets[key], o1 = offsets[key + 1];
     if (o1 != o0) {
       const uint32_t t0 = o0 / K, t1 = (o1 - 1) / K;
-      if (t0 == t1 || t1 - t0 > kPieceLimit) {
+      if (t0 == t1 || t1 - t0 > limit) {
         coop_copy<F>(S, buckets + key * PW, gl, gmask);
         coop_add<F>(R, S, tmp, gl, gmask);
       } else {
