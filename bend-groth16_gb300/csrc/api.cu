@@ -49,10 +49,12 @@ namespace {
 
 thread_local std::string g_err_noctx;
 
+// `gpu`: the body queues work on the context, and one that fails is waited for
 template <class Fn>
-int guard(bg_ctx* ctx, Fn&& fn) {
+int guard(bg_ctx* ctx, Fn&& fn, bool gpu = true) {
   try {
-    fn();
+    if (ctx && gpu) drained(ctx->c, fn);
+    else fn();
     if (ctx) ctx->c.last_error.clear();
     return BG_OK;
   } catch (const Error& e) {
@@ -544,7 +546,9 @@ int bg_prove_batch(bg_ctx* ctx, bg_pk* const* pks, const uint32_t* const* witnes
         if (k >= count) return;
         const size_t i = order[k];
         try {
-          prove_resident(*lane, *pks[i]->pk, witnesses[i], rs[i], &out[i], times ? &times[i] : nullptr, 0.0);
+          drained(*lane, [&] {
+            prove_resident(*lane, *pks[i]->pk, witnesses[i], rs[i], &out[i], times ? &times[i] : nullptr, 0.0);
+          });
           statuses[i] = BG_OK;
         } catch (const Error& e) {
           statuses[i] = e.status;
@@ -573,7 +577,7 @@ int bg_server_create(bg_ctx* ctx, int lanes, size_t hbm_budget_bytes, bg_server*
 
 int bg_server_submit(bg_server* s, bg_pk* pk, const uint32_t* witness16, const uint32_t* rs16, uint64_t tag) {
   BG_ARG_CHECK(s ? s->owner : nullptr, !s || !pk || !witness16 || !rs16 || pk->owner != s->owner);
-  return guard(s->owner, [&] { server_submit(s->s, pk->pk, witness16, rs16, tag); });
+  return guard(s->owner, [&] { server_submit(s->s, pk->pk, witness16, rs16, tag); }, false);
 }
 
 int bg_server_wait(bg_server* s, int timeout_ms, uint64_t* tag, bg_proof* out, bg_phase_ms* times,

@@ -189,6 +189,29 @@ struct Ctx {
   }
 };
 
+// Waits for whatever a context has queued on any of its streams and clears its error word.
+inline void ctx_drain(Ctx& c) {
+  if (c.stream) cudaStreamSynchronize(c.stream);
+  if (c.copy) cudaStreamSynchronize(c.copy);
+  for (cudaStream_t s : c.side)
+    if (s) cudaStreamSynchronize(s);
+  if (c.d_status) *static_cast<volatile uint32_t*>(c.d_status) = 0;
+}
+// Runs a call's body; one that throws (an allocation that failed between two launches) leaves nothing
+// behind on the GPU.  The next call may order its work otherwise and take over buffers that the
+// failed one's kernels still write through (the sorts of a context share their ranks, the pair
+// rounds their levels), its caller may free what the failed one's copies still read, and a late
+// error flag would fail it.
+template <class Fn>
+void drained(Ctx& c, Fn&& fn) {
+  try {
+    fn();
+  } catch (...) {
+    ctx_drain(c);
+    throw;
+  }
+}
+
 // Brackets one kernel launch with events when the context profiles (see bg_ctx_profile).
 class KernelTimer {
  public:

@@ -123,7 +123,7 @@ class Server {
       d.tag = r.tag;
       const auto t_start = Clock::now();
       try {
-        prove_resident(lane, *r.pk, r.witness16, r.rs16, &d.proof, &d.times, 0.0);
+        drained(lane, [&] { prove_resident(lane, *r.pk, r.witness16, r.rs16, &d.proof, &d.times, 0.0); });
         d.status = BG_OK;
       } catch (const Error& e) {
         d.status = e.status;
