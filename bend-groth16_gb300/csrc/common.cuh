@@ -189,6 +189,18 @@ struct Ctx {
   }
 };
 
+// Whether a stream has drained.  A runtime may keep "not ready" as the thread's last error, which the
+// check after the next launch would take for that launch's.
+inline bool stream_drained(cudaStream_t s) {
+  const cudaError_t e = cudaStreamQuery(s);
+  if (e == cudaErrorNotReady) {
+    cudaGetLastError();
+    return false;
+  }
+  BG_CUDA(e);
+  return true;
+}
+
 // Waits for whatever a context has queued on any of its streams and clears its error word.
 inline void ctx_drain(Ctx& c) {
   if (c.stream) cudaStreamSynchronize(c.stream);

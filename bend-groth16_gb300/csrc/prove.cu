@@ -624,11 +624,7 @@ void prove_resident(Ctx& ctx, PkDev& pk, const uint32_t* witness16, const uint32
       const int before = left;
       for (int k : {0, 1, 2, 4, 3}) {
         if (taken[k]) continue;
-        if (plan[k].fetch_stream) {
-          const cudaError_t e = cudaStreamQuery(plan[k].fetch_stream);
-          if (e == cudaErrorNotReady) continue;
-          BG_CUDA(e);
-        }
+        if (plan[k].fetch_stream && !stream_drained(plan[k].fetch_stream)) continue;
         taken[k] = true;
         left--;
         if (k == 3) finish(3);

@@ -68,6 +68,17 @@ extern "C" int t_drained(int fail, int* synced, unsigned* status) {
   for (int i = 0; i < 2 + kStreams; i++) *synced += std::count(g_synced.begin(), g_synced.end(), st(i)) > 0;
   return seen;
 }
+// what stream_drained says of a query's result (2: it throws), and the last error it leaves
+extern "C" int t_stream_drained(int query, int* last) {
+  g_query = (cudaError_t)query;
+  int r = 2;
+  try {
+    r = stream_drained(st(0)) ? 1 : 0;
+  } catch (const Error&) {
+  }
+  *last = cudaGetLastError();
+  return r;
+}
 """
 
 
@@ -98,3 +109,9 @@ def test_a_failed_call_leaves_nothing_in_flight(lib):
     assert lib.t_drained(0, ctypes.byref(synced), ctypes.byref(status)) == 0
     assert synced.value == 0
 
+
+def test_a_stream_still_running_is_no_error(lib):
+    last = ctypes.c_int()
+    assert (lib.t_stream_drained(600, ctypes.byref(last)), last.value) == (0, 0)
+    assert (lib.t_stream_drained(0, ctypes.byref(last)), last.value) == (1, 0)
+    assert lib.t_stream_drained(999, ctypes.byref(last)) == 2
