@@ -580,9 +580,10 @@ void prove_resident(Ctx& ctx, PkDev& pk, const uint32_t* witness16, const uint32
   // ---- finish each MSM on the host when its reduction stream drains.  Combine
   // (groth16.bend:298-308): A = alpha + mA + r delta; B1 = beta + mB1 + s delta; B2 = beta2 + mB2 +
   // s delta2; C = s A + r B1 - r s delta + (mL + mH).  s A and r B1 are chains of 90 us, mB2's sum up
-  // to 140: a proof that has the GPU to itself hands each MSM's part to the pool as it drains, in
-  // whatever order, and this thread takes msm_h; one after another they were the longer half of a
-  // small proof (SquareChain(2^10): 430 of 600 us).  A lane of a batch or a server shares the pool
+  // to 140: a proof that has the GPU to itself hands each MSM's part to the pool as it drains and this
+  // thread takes msm_h; one after another they were the longer half of a small proof
+  // (SquareChain(2^10): 430 of 600 us).  Small proofs, whose MSMs run side by side, are polled for
+  // whichever is next; the others are waited for in order.  A lane of a batch or a server shares the pool
   // with others and takes them in turn.
   products.wait();
   auto total = [&](auto* q) {
@@ -619,18 +620,28 @@ void prove_resident(Ctx& ctx, PkDev& pk, const uint32_t* witness16, const uint32
     }
   } else {
     HostPool::Task tasks[5];
-    bool taken[5] = {};
-    for (int left = 5; left;) {
-      const int before = left;
+    auto hand_over = [&](int k) {
+      if (k == 3) finish(3);
+      else tasks[k] = HostPool::get().start(1, [&finish, k](int) { finish(k); });
+    };
+    if (!overlap) {
+      // one accumulation stream: the MSMs drain in about this order, milliseconds apart
       for (int k : {0, 1, 2, 4, 3}) {
-        if (taken[k]) continue;
-        if (plan[k].fetch_stream && !stream_drained(plan[k].fetch_stream)) continue;
-        taken[k] = true;
-        left--;
-        if (k == 3) finish(3);
-        else tasks[k] = HostPool::get().start(1, [&finish, k](int) { finish(k); });
+        if (plan[k].fetch_stream) BG_CUDA(cudaStreamSynchronize(plan[k].fetch_stream));
+        hand_over(k);
       }
-      if (left == before) std::this_thread::yield();
+    } else {
+      bool taken[5] = {};
+      for (int left = 5; left;) {
+        const int before = left;
+        for (int k : {0, 1, 2, 4, 3}) {
+          if (taken[k] || (plan[k].fetch_stream && !stream_drained(plan[k].fetch_stream))) continue;
+          taken[k] = true;
+          left--;
+          hand_over(k);
+        }
+        if (left == before) std::this_thread::yield();
+      }
     }
     for (HostPool::Task& t : tasks) t.wait();
   }
