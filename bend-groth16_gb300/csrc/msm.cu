@@ -992,6 +992,29 @@ struct HostField<Fq2> {
   typedef bgh::Fq2Ops T;
 };
 
+// Sizes of a sort: windows, bucket keys, and entries as padded for as many of `rounds` pair rounds as the
+// padding allows (a few empty slots per entry, and positions that fit 31 bits).
+struct SortSizes {
+  int W, sets, rounds;
+  size_t nkeys, entries, padded;
+};
+static SortSizes sort_sizes(size_t n, int c, bool shared_set, int rounds) {
+  SortSizes z;
+  z.W = 254 / c + 1;
+  z.sets = shared_set ? 1 : z.W;
+  z.nkeys = (size_t)z.sets << (c - 1);
+  z.entries = n * (size_t)z.W;
+  auto padded_to = [&](int r) { return z.entries + z.nkeys * ((size_t(1) << r) - 1); };
+  while (rounds > 0 && ((z.nkeys << rounds) > std::max(8 * z.entries, size_t(1) << 20) ||
+                        padded_to(rounds) >= 0x80000000ull))
+    rounds--;
+  z.rounds = rounds;
+  z.padded = padded_to(rounds);
+  return z;
+}
+// one rank buffer for a context's sorts below 2^kRankLog2 scalars, else cursors by key
+static bool sort_by_rank(size_t n) { return n < (size_t(1) << kRankLog2); }
+
 void msm_sort(Ctx& ctx, cudaStream_t st, const std::string& tag, const uint32_t* d_scalars, size_t n, int c,
               bool shared_set, int rounds, MsmSort& out) {
   out = MsmSort();
@@ -999,32 +1022,25 @@ void msm_sort(Ctx& ctx, cudaStream_t st, const std::string& tag, const uint32_t*
   if (n == 0) return;
   if (n >= 0x80000000ull) throw Error(BG_E_ARG, "msm: n must be below 2^31");
   if (c < 2 || c > 24) throw Error(BG_E_ARG, "msm: window width out of range");
-  const int W = 254 / c + 1;
+  const SortSizes z = sort_sizes(n, c, shared_set, rounds);
+  if (z.entries >= 0x80000000ull) throw Error(BG_E_ARG, "msm: n x windows must be below 2^31");
+  const int W = z.W;
   const uint32_t nb = 1u << (c - 1);
-  const int sets = shared_set ? 1 : W;
-  const size_t nkeys = (size_t)sets * nb;
+  const size_t nkeys = z.nkeys, padded = z.padded;
   const uint32_t key_stride = shared_set ? 0u : nb;
   const uint32_t idx_stride = shared_set ? (uint32_t)n : 0u;
-  size_t max_entries = n * (size_t)W;
-  if (max_entries >= 0x80000000ull) throw Error(BG_E_ARG, "msm: n x windows must be below 2^31");
-  // buckets padded for the pair rounds, as many as the padding allows: a few empty slots per entry,
-  // and positions that fit 31 bits
-  auto padded_to = [&](int r) { return max_entries + nkeys * ((size_t(1) << r) - 1); };
-  while (rounds > 0 && ((nkeys << rounds) > std::max(8 * max_entries, size_t(1) << 20) ||
-                        padded_to(rounds) >= 0x80000000ull))
-    rounds--;
-  const size_t padded = padded_to(rounds);
+  rounds = z.rounds;
   out.rounds = rounds;
   out.c = c;
   out.W = W;
-  out.sets = sets;
+  out.sets = z.sets;
   out.nb = nb;
   out.nkeys = nkeys;
   out.max_entries = padded;
 
   Workspace& ws = ctx.ws;
   uint32_t* counts = ws.get_t<uint32_t>(tag + ".counts", nkeys + 1);
-  const bool by_rank = n < (size_t(1) << kRankLog2);
+  const bool by_rank = sort_by_rank(n);
   // one rank buffer: the context's sorts are ordered
   uint32_t* cursor = by_rank ? ws.get_t<uint32_t>("sort.ranks", n * (size_t)W)
                              : ws.get_t<uint32_t>(tag + ".cursor", nkeys + 1);
@@ -1176,10 +1192,44 @@ void msm_accumulate(Ctx& ctx, cudaStream_t st, const std::string& tag, const uin
   plan.host_window_sums = ctx.host_cache.get_t<uint32_t>(tag + ".window_sums", so.sets * points * PW);
 }
 
-int msm_rounds(const Ctx& ctx, size_t n, int c, bool shared_set, bool g2) {
-  if (ctx.pair_rounds_override >= 0) return ctx.pair_rounds_override;
+int msm_rounds_model(size_t n, int c, bool shared_set, bool g2) {
   const size_t W = 254 / c + 1;
   return pair_rounds_model(n, n * W, (shared_set ? 1 : W) << (c - 1), g2, shared_set);
+}
+int msm_rounds(const Ctx& ctx, size_t n, int c, bool shared_set, bool g2) {
+  return ctx.pair_rounds_override >= 0 ? ctx.pair_rounds_override : msm_rounds_model(n, c, shared_set, g2);
+}
+
+// ---- the device bytes of the buffers above, for a proof's reservation.  Bounds where a choice depends on
+// the GPU: slices at three quarters of the model's K (whole_wave_slices), the most parts a reduction's
+// shape can have.
+size_t msm_sort_bytes(size_t n, int c, bool shared_set, int rounds) {
+  const SortSizes z = sort_sizes(n, c, shared_set, rounds);
+  const size_t tiles = (z.nkeys + 1) / kScanTile + 1;
+  const size_t keyed = (sort_by_rank(n) ? 2 : 3) * (z.nkeys + 1);  // counts, offsets, cursors
+  return 4 * (keyed + z.padded + 2 * tiles + 2 * (tiles / kScanTile + 1));
+}
+size_t msm_rank_bytes(size_t n, int c) { return sort_by_rank(n) ? 4 * n * (size_t)(254 / c + 1) : 0; }
+void msm_level_bytes(size_t n, int c, bool shared_set, int rounds, bool g2, size_t out[2]) {
+  const SortSizes z = sort_sizes(n, c, shared_set, rounds);
+  const size_t point = g2 ? 128 : 64;
+  out[0] = z.rounds > 0 ? (z.padded >> 1) * point : 0;
+  out[1] = z.rounds > 1 ? (z.padded >> 2) * point : 0;
+}
+size_t msm_bucket_bytes(size_t n, int c, bool shared_set, int rounds, bool g2) {
+  const SortSizes z = sort_sizes(n, c, shared_set, rounds);
+  const size_t entries = z.padded >> z.rounds, nb = size_t(1) << (c - 1), point = g2 ? 256 : 128;
+  const uint32_t K = g2 ? slice_entries<Fq2>(entries, z.nkeys) : slice_entries<Fq>(entries, z.nkeys);
+  const size_t slices = 4 * entries / (3 * K) + 1;
+  size_t parts = 0;  // points per bucket set
+  for (uint32_t RT = 4; RT <= 256 && RT <= std::max<size_t>(nb, 4); RT <<= 1) {
+    ReduceShape r{RT, 1, (uint32_t)std::max<size_t>(1, nb / RT)};
+    // fewer than 32 threads, or a scan, in the cooperative form alone
+    if (RT < 32 && r.J > 1) r.J = std::min<uint32_t>(r.J, kCoopMaxParts / z.sets + 1);
+    parts = std::max(parts, reduce_part_points(r));
+  }
+  return point * (z.nkeys + 2 * slices + z.sets * parts) + 4 * (slices / 4 + 2) +
+         (z.rounds ? 4 * (z.nkeys + 1) : 0);
 }
 
 template <class F>

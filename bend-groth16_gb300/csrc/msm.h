@@ -88,7 +88,14 @@ void msm_sort(Ctx& ctx, cudaStream_t st, const std::string& tag, const uint32_t*
               bool shared_set, int rounds, MsmSort& out);
 // Batch-affine pair rounds of an MSM of n points with c-bit windows (the context's override, else
 // the cost model); MSMs that share a sort take the most of theirs
+int msm_rounds_model(size_t n, int c, bool shared_set, bool g2);
 int msm_rounds(const Ctx& ctx, size_t n, int c, bool shared_set, bool g2);
+// Device bytes that a sort, an accumulation and reduction (both upper bounds), the rank buffer that a
+// context's sorts share and the two level buffers that its pair rounds share take.
+size_t msm_sort_bytes(size_t n, int c, bool shared_set, int rounds);
+size_t msm_bucket_bytes(size_t n, int c, bool shared_set, int rounds, bool g2);
+size_t msm_rank_bytes(size_t n, int c);
+void msm_level_bytes(size_t n, int c, bool shared_set, int rounds, bool g2, size_t out[2]);
 template <class F>
 void msm_accumulate(Ctx& ctx, cudaStream_t st, const std::string& tag, const uint32_t* d_points, const MsmSort& so,
                     MsmPlan& plan, cudaStream_t st_reduce = nullptr, const MsmTable* table = nullptr);

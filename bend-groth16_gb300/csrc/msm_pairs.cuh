@@ -300,11 +300,11 @@ __global__ void __launch_bounds__(kPairThreads<F>, FieldWords<F>::value == 8 ? 4
 // MSM 2^20 (17.8 M entries, 64 per bucket) 2.42 ms of mixed additions -> 1.57 + 0.65 ms, the MSM
 // 3.49 -> 3.19 ms (one round 3.33, three 3.3); SquareChain(2^20) 23.2 -> 20.75 ms, 2^19 12.2 ->
 // 11.15 ms, 16 mixed proofs in a batch 17.2 -> 16.5 ms; SquareChain(2^18) level (6.65-6.77 ms either
-// way), with tables of 2 M entries too 2^17 and the batch 2% slower.  Window tables of 2^18 points
-// and up, whose levels fit the scratch a proof reserves (SquareChain(2^17)'s msm_h, 262143 points,
-// would need 3% more).  The bucket sets of standalone MSMs hold fewer entries per bucket
-// (G2 MSM 2^18: 17) and their accumulation is not what its reduction waits behind, so only the
-// largest G1 ones take rounds.
+// way), with tables of 2 M entries too 2^17 and the batch 2% slower: window tables of 2^18 points and
+// up, of which a proof takes as many rounds as its reservation has room for (prove_round_cap).  The
+// bucket sets of standalone MSMs hold fewer entries per bucket; of those only the largest G1 ones
+// take rounds (G2: one round measured 3.20 -> 3.04 ms at 2^18 points and 4.33 -> 3.98 at 400,000;
+// bg_msm_pair_rounds is documented to take none there).
 inline int pair_rounds_model(size_t n, size_t max_entries, size_t nkeys, bool g2, bool shared_set) {
   if (shared_set) return n >= (size_t(1) << 18) && max_entries >= 3000000 && max_entries >= 24 * nkeys ? 2 : 0;
   if (g2 || max_entries < (size_t(1) << 23) || max_entries < 32 * nkeys) return 0;

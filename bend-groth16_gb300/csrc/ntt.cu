@@ -338,6 +338,12 @@ static std::vector<Fe> powers(const Fe& base, size_t n, const Fe& first) {
   return out;
 }
 
+size_t ntt_table_bytes(int L) {
+  const size_t half = L > 0 ? size_t(1) << (L - 1) : 1, lo = size_t(1) << ((L + 1) / 2), hi = (size_t(1) << L) / lo;
+  const size_t nlo = std::min(half, size_t(1) << 10), nhi = (half + nlo - 1) / nlo;
+  return 32 * (2 * half + nlo + nhi + 2 * lo + 4 * hi + 2);
+}
+
 NttTables& ntt_tables(Ctx& ctx, int L) {
   NttTables& slot = ctx.ntt_tabs[L];
   if (slot.ready) return slot;

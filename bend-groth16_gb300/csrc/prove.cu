@@ -482,6 +482,13 @@ void prove_resident(Ctx& ctx, PkDev& pk, const uint32_t* witness16, const uint32
   // assignment) and, with equal lengths, the same window layout, so they share one sort; l's
   // follows; h's is made on the main stream once the QAP is done.  The accumulation stream then
   // runs the five accumulations back to back, each waiting only for its own sort.
+  // Pair rounds over window tables are the one part that can outgrow what the key's proofs reserve
+  // (bg_prove_footprint): a key of many wires in a small domain, or the reverse, takes fewer.
+  int round_cap = 12;
+  if (pk.tables && ctx.pair_rounds_override < 0) {
+    const int c[5] = {pk.tab[0].c, pk.tab[1].c, pk.tab[2].c, pk.tab[3].c, pk.tab[4].c};
+    round_cap = prove_round_cap(h, c);
+  }
   cudaStream_t acc_st = ctx.side[0];
   cudaStream_t sort_st = ctx.side[kSortStream];
   BG_CUDA(cudaStreamWaitEvent(sort_st, ev_scalars, 0));
@@ -501,7 +508,7 @@ void prove_resident(Ctx& ctx, PkDev& pk, const uint32_t* witness16, const uint32
     int rounds = 0;
     for (const Job& o : jobs)
       if (o.sc == k.sc && o.n == k.n && width(o) == k.c && (o.tab != nullptr) == k.shared)
-        rounds = std::max(rounds, msm_rounds(ctx, o.n, k.c, k.shared, o.g2));
+        rounds = std::max(rounds, std::min(round_cap, msm_rounds(ctx, o.n, k.c, k.shared, o.g2)));
     msm_sort(ctx, s, std::string(jb.tag) + ".sort", jb.sc, jb.n, k.c, k.shared, rounds, sorts.back().second);
     return sorts.back().second;
   };
@@ -692,8 +699,10 @@ static size_t msm_footprint_c(size_t n, bool g2, int c) {
 }
 // Window widths the reservation is made for, per floor(log2 n) from 10, G1 and G2: a standalone MSM's
 // and a one-shot proof's.  They are wider than the tuned ones in places and stay as they are when
-// those change, so that a budget admits what it admitted; a proof's scratch lies below the
-// reservation (SquareChain(2^10): 6 of 30 MB, 2^18: 0.8 of 1.5 GB, 2^20: 2.6 of 7.7 GB).
+// those change, so that a budget admits what it admitted.  A proof's scratch lies below the
+// reservation (SquareChain(2^10): 15 of 30 MB, 2^18: 0.8 of 1.5 GB, 2^20: 2.6 of 7.7 GB): without
+// pair rounds at most three quarters of it for any header, and prove_round_cap allows only the
+// rounds that fit.
 static int reserved_c(size_t n, bool g2, bool in_proof) {
   static const signed char sets[2][13] = {{8, 8, 9, 9, 9, 10, 11, 12, 15, 15, 15, 15, 17},
                                           {8, 9, 9, 9, 9, 10, 11, 12, 15, 15, 15, 0, 0}};
@@ -721,6 +730,40 @@ size_t prove_footprint(const Header& h) {
   b += msm_footprint(h.na, false) + msm_footprint(h.nb, false) + msm_footprint(h.nb, true) +
        msm_footprint(h.nh, false) + msm_footprint(h.nl, false);
   return b + b / 10 + (4u << 20);
+}
+
+size_t prove_scratch(const Header& h, const int* c, int cap) {
+  const size_t d = size_t(1) << h.lg, nz = (size_t)h.ni + h.nw;
+  const size_t n[5] = {h.na, h.nb, h.nb, h.nh, h.nl};
+  const int set[5] = {0, h.na == h.nb ? 0 : 1, h.na == h.nb ? 0 : 1, 2, 3};  // MSMs of equal scalars
+  auto rounds_of = [&](int i) {  // of the sort, which MSMs of equal scalars and widths share
+    int r = 0;
+    for (int j = 0; j < 5; j++)
+      if (n[j] && set[j] == set[i] && c[j] == c[i])
+        r = std::max(r, msm_rounds_model(n[j], c[j], true, j == 2));
+    return std::min(r, cap);
+  };
+  size_t b = nz * 128 + 4 * d * 32 + ntt_table_bytes((int)h.lg);
+  size_t rank = 0, level[2] = {0, 0};
+  for (int i = 0; i < 5; i++) {
+    if (!n[i]) continue;
+    const int r = rounds_of(i);
+    bool sorted = false;
+    for (int j = 0; j < i; j++) sorted = sorted || (n[j] && set[j] == set[i] && c[j] == c[i]);
+    if (!sorted) b += msm_sort_bytes(n[i], c[i], true, r);
+    b += msm_bucket_bytes(n[i], c[i], true, r, i == 2);
+    rank = std::max(rank, msm_rank_bytes(n[i], c[i]));
+    size_t l[2];
+    msm_level_bytes(n[i], c[i], true, r, i == 2, l);
+    for (int k = 0; k < 2; k++) level[k] = std::max(level[k], l[k]);
+  }
+  return b + rank + level[0] + level[1];
+}
+int prove_round_cap(const Header& h, const int* c) {
+  const size_t reserved = prove_footprint(h);
+  int cap = 2;  // the most that the model takes
+  while (cap > 0 && prove_scratch(h, c, cap) > reserved) cap--;
+  return cap;
 }
 
 // ---------------------------------------------------------------- proof text

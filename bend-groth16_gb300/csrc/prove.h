@@ -57,6 +57,11 @@ void prove_resident(Ctx& ctx, PkDev& pk, const uint32_t* witness16, const uint32
 int format_proof(const bg_proof* p, char* buf, size_t cap);
 // device bytes of scratch one proof against a key with this header needs
 size_t prove_footprint(const Header& h);
+// the device bytes a proof with window tables of these widths (a, b1, b2, h, l) takes, an upper bound,
+// if its MSMs take at most `cap` pair rounds; and the most rounds with which that stays within the
+// footprint
+size_t prove_scratch(const Header& h, const int* c, int cap);
+int prove_round_cap(const Header& h, const int* c);
 
 // serving loop (server.cu)
 class Server;

@@ -236,7 +236,7 @@ int bg_msm_proof_window_bits(size_t n, int curve);
 int bg_msm_window_override(bg_ctx* ctx, int layout, int curve, int c);
 /* Batch-affine pair rounds the library's cost model takes for a standalone MSM of n points of
  * `curve` (bg_msm_g1/g2 and their _dev forms): 2 for G1 MSMs of at least 2^23 entries with at
- * least 32 per bucket, else 0 (measured slower there on GB300). */
+ * least 32 per bucket, else 0. */
 int bg_msm_pair_rounds(size_t n, int curve);
 /* Tuning hook: the number of batch-affine pair rounds before each later MSM's bucket
  * accumulation on this context and its batch lanes (each round adds the points of every bucket
