@@ -223,49 +223,92 @@ BG_DEV XYZZ<F> xyzz_add_inline(const XYZZ<F>& p, const XYZZ<F>& q) {
 }
 
 // ---------------------------------------------------------------- affine pair additions
-// P + Q for affine P and Q where the caller supplies 1/d for the denominator d: the
-// batch-affine accumulation inverts the denominators of many additions at once (Montgomery's
-// simultaneous inversion), so an addition costs the chord slope and the new coordinates
-// (two products and a square) plus its three products of the shared inversion, against
-// madd-2008-s's eight products and two squares.  pair_kind picks the case and its denominator:
-// the chord (x_Q - x_P), the tangent (2 y_P) when P = Q, or none (a result of infinity, or one
-// input at infinity).  The affine infinity is (0, 0) as everywhere on the device.
-enum : uint32_t { kPairChord = 0, kPairTangent = 1, kPairInf = 2, kPairFirst = 3, kPairSecond = 4 };
+// P + Q for affine P and Q whose denominator is inverted together with those of many other additions
+// (Montgomery's simultaneous inversion): the chord slope and the new coordinates (two products and a
+// square) plus three products of the shared inversion, against madd-2008-s's eight products and
+// two squares.  The affine infinity is (0, 0) as everywhere on the device, and a missing point.
+// a - b as some representative below 2^256 (a, b < p): for the second factor of a product
+BG_DEV Fq sub_loose(const Fq& a, const Fq& b) {
+  Fq r;
+  asm("add.cc.u32  %0, %8,  %16;\n\t"
+      "addc.cc.u32 %1, %9,  %17;\n\t"
+      "addc.cc.u32 %2, %10, %18;\n\t"
+      "addc.cc.u32 %3, %11, %19;\n\t"
+      "addc.cc.u32 %4, %12, %20;\n\t"
+      "addc.cc.u32 %5, %13, %21;\n\t"
+      "addc.cc.u32 %6, %14, %22;\n\t"
+      "addc.u32    %7, %15, %23;"
+      : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]), "=r"(r.v[7])
+      : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7]),
+        "n"(FqParams::P0), "n"(FqParams::P1), "n"(FqParams::P2), "n"(FqParams::P3), "n"(FqParams::P4),
+        "n"(FqParams::P5), "n"(FqParams::P6), "n"(FqParams::P7));
+  asm("sub.cc.u32  %0, %0, %8;\n\t"
+      "subc.cc.u32 %1, %1, %9;\n\t"
+      "subc.cc.u32 %2, %2, %10;\n\t"
+      "subc.cc.u32 %3, %3, %11;\n\t"
+      "subc.cc.u32 %4, %4, %12;\n\t"
+      "subc.cc.u32 %5, %5, %13;\n\t"
+      "subc.cc.u32 %6, %6, %14;\n\t"
+      "subc.u32    %7, %7, %15;"
+      : "+r"(r.v[0]), "+r"(r.v[1]), "+r"(r.v[2]), "+r"(r.v[3]), "+r"(r.v[4]), "+r"(r.v[5]), "+r"(r.v[6]), "+r"(r.v[7])
+      : "r"(b.v[0]), "r"(b.v[1]), "r"(b.v[2]), "r"(b.v[3]), "r"(b.v[4]), "r"(b.v[5]), "r"(b.v[6]), "r"(b.v[7]));
+  return r;
+}
+// (an Fq2 product adds its factors' halves, which leaves no room)
+BG_DEV Fq2 sub_loose(const Fq2& a, const Fq2& b) { return sub(a, b); }
 
+BG_DEV Fq select(bool c, const Fq& a, const Fq& b) {
+  Fq r;
+#pragma unroll
+  for (int i = 0; i < 8; i++) r.v[i] = c ? a.v[i] : b.v[i];
+  return r;
+}
+BG_DEV Fq2 select(bool c, const Fq2& a, const Fq2& b) { return {select(c, a.c0, b.c0), select(c, a.c1, b.c1)}; }
+
+// The denominator's last step, for points of equal x (x_Q - x_P = 0, which cannot be a factor of the
+// running product): 2 y for the tangent (P = Q), 1 where no addition is due -- Q = -P, two missing
+// points, or one and a point of x = 0.  A missing point beside one of x != 0 gives that point's +-x,
+// as good a factor as any.
 template <class F>
-BG_DEV uint32_t pair_kind(const Affine<F>& p, const Affine<F>& q, F& d) {
-  if (is_inf(p)) return kPairSecond;
-  if (is_inf(q)) return kPairFirst;
-  d = sub(q.x, p.x);
-  if (!is_zero(d)) return kPairChord;
-  if (eq(p.y, q.y) && !is_zero(p.y)) {
-    d = dbl(p.y);
-    return kPairTangent;
-  }
-  return kPairInf;  // Q = -P (or a point of order two, which the prime-order groups lack)
+BG_DEV F pair_equal_x(const F& yp, const F& yq) {
+  return eq(yp, yq) && !is_zero(yp) ? dbl(yp) : field_one<F>();
 }
 
-// the sum for the case pair_kind chose; dinv = 1 / d for the chord and tangent cases
+// The denominator of P + Q as the forward pass took it, with the slope's numerator, and whether the
+// sum is (0, 0); mp, mq: P or Q is missing.
 template <class F>
-BG_DEV Affine<F> pair_finish(const Affine<F>& p, const Affine<F>& q, uint32_t kind, const F& dinv) {
-  if (kind == kPairFirst) return p;
-  if (kind == kPairSecond) return q;
+BG_DEV bool pair_terms(const Affine<F>& p, const Affine<F>& q, bool mp, bool mq, F& d, F& num) {
+  d = sub(q.x, p.x);
+  num = sub_loose(q.y, p.y);
+  bool none = mp && mq;  // no sum, or a sum at infinity
+  if (is_zero(d)) {
+    if (!none && eq(p.y, q.y) && !is_zero(p.y)) {
+      d = dbl(p.y);
+      const F x2 = fsqr(p.x);
+      num = add(dbl(x2), x2);
+    } else {
+      d = field_one<F>();
+      none = none || (!mp && !mq);
+    }
+  }
+  return none;
+}
+
+// the sum, from pair_terms' numerator and the inverse of its denominator
+template <class F>
+BG_DEV Affine<F> pair_sum(const Affine<F>& p, const Affine<F>& q, bool mp, bool mq, bool none, const F& num,
+                          const F& dinv) {
+  const F l = imul(dinv, num);
   Affine<F> r;
-  if (kind == kPairInf) {
-    r.x = field_zero<F>();
-    r.y = field_zero<F>();
-    return r;
-  }
-  F num;
-  if (kind == kPairChord) {
-    num = sub(q.y, p.y);
-  } else {
-    const F x2 = fsqr(p.x);
-    num = add(dbl(x2), x2);
-  }
-  const F l = imul(num, dinv);
   r.x = sub(sub(isqr(l), p.x), q.x);  // the tangent case has q.x = p.x
-  r.y = sub(imul(l, sub(p.x, r.x)), p.y);
+  r.y = sub(imul(l, sub_loose(p.x, r.x)), p.y);
+  if (mp || mq || none) {
+    r = mp ? q : p;
+    if (none) {
+      r.x = field_zero<F>();
+      r.y = field_zero<F>();
+    }
+  }
   return r;
 }
 

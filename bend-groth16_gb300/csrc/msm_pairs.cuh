@@ -50,13 +50,6 @@ constexpr size_t pair_smem_bytes() {
   return pair_ring_chunks<F>() * 16 > tree ? pair_ring_chunks<F>() * 16 : tree;
 }
 
-BG_DEV Fq select(bool c, const Fq& a, const Fq& b) {
-  Fq r;
-#pragma unroll
-  for (int i = 0; i < 8; i++) r.v[i] = c ? a.v[i] : b.v[i];
-  return r;
-}
-BG_DEV Fq2 select(bool c, const Fq2& a, const Fq2& b) { return {select(c, a.c0, b.c0), select(c, a.c1, b.c1)}; }
 template <class F>
 BG_DEV F elem_of_chunks(const uint4* c, int stride) {
   if constexpr (FieldWords<F>::value == 16) {
@@ -75,36 +68,6 @@ template <int N>
 BG_DEV void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
-
-// a - b as some representative below 2^256 (a, b < p): for the second factor of a product
-BG_DEV Fq sub_loose(const Fq& a, const Fq& b) {
-  Fq r;
-  asm("add.cc.u32  %0, %8,  %16;\n\t"
-      "addc.cc.u32 %1, %9,  %17;\n\t"
-      "addc.cc.u32 %2, %10, %18;\n\t"
-      "addc.cc.u32 %3, %11, %19;\n\t"
-      "addc.cc.u32 %4, %12, %20;\n\t"
-      "addc.cc.u32 %5, %13, %21;\n\t"
-      "addc.cc.u32 %6, %14, %22;\n\t"
-      "addc.u32    %7, %15, %23;"
-      : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]), "=r"(r.v[7])
-      : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7]),
-        "n"(FqParams::P0), "n"(FqParams::P1), "n"(FqParams::P2), "n"(FqParams::P3), "n"(FqParams::P4),
-        "n"(FqParams::P5), "n"(FqParams::P6), "n"(FqParams::P7));
-  asm("sub.cc.u32  %0, %0, %8;\n\t"
-      "subc.cc.u32 %1, %1, %9;\n\t"
-      "subc.cc.u32 %2, %2, %10;\n\t"
-      "subc.cc.u32 %3, %3, %11;\n\t"
-      "subc.cc.u32 %4, %4, %12;\n\t"
-      "subc.cc.u32 %5, %5, %13;\n\t"
-      "subc.cc.u32 %6, %6, %14;\n\t"
-      "subc.u32    %7, %7, %15;"
-      : "+r"(r.v[0]), "+r"(r.v[1]), "+r"(r.v[2]), "+r"(r.v[3]), "+r"(r.v[4]), "+r"(r.v[5]), "+r"(r.v[6]), "+r"(r.v[7])
-      : "r"(b.v[0]), "r"(b.v[1]), "r"(b.v[2]), "r"(b.v[3]), "r"(b.v[4]), "r"(b.v[5]), "r"(b.v[6]), "r"(b.v[7]));
-  return r;
-}
-// (an Fq2 product adds its factors' halves, which leaves no room)
-BG_DEV Fq2 sub_loose(const Fq2& a, const Fq2& b) { return sub(a, b); }
 
 // One round: `per_thread` positions per thread.  dst's x field of each position first holds the
 // thread's running product up to it (read back by the backward pass) and is then overwritten by
@@ -172,8 +135,6 @@ __global__ void __launch_bounds__(kPairThreads<F>, FieldWords<F>::value == 8 ? 4
       cp_async_wait<FD - 1>();
       const uint4* s = ring + (size_t)(t & (FD - 1)) * 2 * CH * NT;
       const F xp = elem_of_chunks<F>(s, NT), xq = elem_of_chunks<F>(s + CH * NT, NT);
-      // A missing point has x = 0 and gives the other's +-x, as good a factor as any: the backward
-      // pass takes it out again.  Only a zero needs care: equal x or two missing points.
       F d = sub(xq, xp);
       if (is_zero(d)) {
         const uint2 en = entries(t);
@@ -182,7 +143,7 @@ __global__ void __launch_bounds__(kPairThreads<F>, FieldWords<F>::value == 8 ? 4
         if (!kFirst || en.y != kNullEntry) load_elem(yq, point(t, en, 1) + FW);
         if (kFirst && (en.x >> 31)) yp = neg(yp);
         if (kFirst && (en.y >> 31)) yq = neg(yq);
-        d = eq(yp, yq) && !is_zero(yp) ? dbl(yp) : field_one<F>();  // the tangent's, or no addition
+        d = pair_equal_x(yp, yq);
       }
       acc = imul(acc, d);
       store_elem(dst + (base + (uint64_t)t * NT) * PW, acc);
@@ -264,33 +225,12 @@ __global__ void __launch_bounds__(kPairThreads<F>, FieldWords<F>::value == 8 ? 4
       p.y = select(ec.x >> 31, neg(p.y), p.y);
       q.y = select(ec.y >> 31, neg(q.y), q.y);
     }
-    F d = sub(q.x, p.x), num = sub_loose(q.y, p.y);
-    bool none = mp && mq;  // no sum, or a sum at infinity
-    if (is_zero(d)) {
-      if (!none && eq(p.y, q.y) && !is_zero(p.y)) {
-        d = dbl(p.y);
-        const F x2 = fsqr(p.x);
-        num = add(dbl(x2), x2);
-      } else {
-        d = field_one<F>();
-        none = none || (!mp && !mq);
-      }
-    }
+    F d, num;
+    const bool none = pair_terms(p, q, mp, mq, d, num);
     F dinv = inv;
     if (t > 0) dinv = imul(inv, elem_of_chunks<F>(s + 4 * CH * NT, NT));
     inv = imul(inv, d);
-    const F l = imul(dinv, num);
-    Affine<F> r;
-    r.x = sub(sub(isqr(l), p.x), q.x);  // the tangent case has q.x = p.x
-    r.y = sub(imul(l, sub_loose(p.x, r.x)), p.y);
-    if (mp || mq || none) {
-      r = mp ? q : p;
-      if (none) {
-        r.x = field_zero<F>();
-        r.y = field_zero<F>();
-      }
-    }
-    store_affine(dst + j * PW, r);
+    store_affine(dst + j * PW, pair_sum(p, q, mp, mq, none, num, dinv));
   }
 }
 

@@ -1,7 +1,7 @@
 """The device field and curve arithmetic, executed on the host for CPU tests.
 
-`bend-groth16_gb300/csrc/fp.cuh`, `fp_wide.cuh` and `ec.cuh` compute every Fr/Fq/Fq2 product
-and every G1/G2 addition with PTX carry chains written as inline `asm` statements.  This
+`bend-groth16_gb300/csrc/fp.cuh`, `fp_wide.cuh`, `ec.cuh` and `ntt_butterfly.cuh` compute every
+Fr/Fq/Fq2 product, every G1/G2 addition and the NTT butterflies with PTX carry chains written as inline `asm` statements.  This
 module checks those chains without a GPU: it runs the C preprocessor over the headers,
 rewrites each `asm(...)` statement into C++ that executes the same PTX instructions on 32-bit
 integers with an explicit carry flag, compiles the result with g++ into a shared library and
@@ -28,7 +28,7 @@ import tempfile
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(HERE), "bend-groth16_gb300", "csrc")
-HEADERS = ("fp.cuh", "fp_wide.cuh", "ec.cuh")
+HEADERS = ("fp.cuh", "fp_wide.cuh", "ec.cuh", "ntt_butterfly.cuh")
 
 _ASM = re.compile(r"\basm\s*(?:volatile\s*)?\(")
 _OPCODE = re.compile(r"^(add|addc|sub|subc|mul|mad|madc)((?:\.lo|\.hi)?)((?:\.cc)?)\.u32$")
@@ -256,14 +256,24 @@ template <class F> static Affine<F> lda(const uint32_t* s) {
 template <class F> static void sta(uint32_t* d, const Affine<F>& p) {
   constexpr int W = FieldWords<F>::value; stf(d, p.x); stf(d + W, p.y);
 }
-/* one affine pair addition as the batch-affine rounds make it, with a one-element batch: the
- * denominator pair_kind picks, inverted by the binary-Euclid inverse, into pair_finish */
+/* one affine pair addition as k_pair_round makes it, with a one-element batch: the forward pass's
+ * denominator inverted, then the backward pass's terms and sum; kind: 0 chord, 1 tangent, 2 the sum is
+ * infinity, 3 Q missing, 4 P missing.  The two passes' denominators have to agree. */
 template <class F> static void pair_add_impl(const uint32_t* p, const uint32_t* q, uint32_t* r, uint32_t* kind) {
   const Affine<F> P = lda<F>(p), Q = lda<F>(q);
-  F d = field_zero<F>();
-  *kind = pair_kind(P, Q, d);
-  const F dinv = *kind <= kPairTangent ? field_inv_fast(d) : field_zero<F>();
-  sta(r, pair_finish(P, Q, *kind, dinv));
+  F fwd = sub(Q.x, P.x);
+  if (is_zero(fwd)) fwd = pair_equal_x(P.y, Q.y);
+  const bool mp = is_inf(P), mq = is_inf(Q);
+  F d, num;
+  const bool none = pair_terms(P, Q, mp, mq, d, num);
+  if (!eq(d, fwd)) { *kind = 99; return; }
+  sta(r, pair_sum(P, Q, mp, mq, none, num, field_inv_fast(d)));
+  *kind = mp ? 4 : mq ? 3 : none ? 2 : is_zero(sub(Q.x, P.x)) ? 1 : 0;
+}
+template <bool DIT> static void butterfly_impl(uint32_t* x0, uint32_t* x1, const uint32_t* w, int unit) {
+  Fr a = ld<FrParams>(x0), b = ld<FrParams>(x1);
+  butterfly<DIT>(a, b, w, 0, unit != 0);
+  st(x0, a); st(x1, b);
 }
 
 #define FIELD_OPS(PFX, PARAMS)                                                                  \
@@ -301,9 +311,20 @@ void fq2_inv_fast(const uint32_t* a, uint32_t* r) { st2(r, field_inv_fast(ld2(a)
 void g1_pair_add(const uint32_t* p, const uint32_t* q, uint32_t* kind, uint32_t* r) { pair_add_impl<Fq>(p, q, r, kind); }
 void g2_pair_add(const uint32_t* p, const uint32_t* q, uint32_t* kind, uint32_t* r) { pair_add_impl<Fq2>(p, q, r, kind); }
 
+void fq_mul_loose(const uint32_t* a, const uint32_t* b, uint32_t* r) { st(r, mul_loose(ld<FqParams>(a), ld<FqParams>(b))); }
+void fr_mul_loose(const uint32_t* a, const uint32_t* b, uint32_t* r) { st(r, mul_loose(ld<FrParams>(a), ld<FrParams>(b))); }
+void fq_sub_loose(const uint32_t* a, const uint32_t* b, uint32_t* r) { st(r, sub_loose(ld<FqParams>(a), ld<FqParams>(b))); }
+void fr_add_raw(const uint32_t* a, const uint32_t* b, uint32_t* r) { st(r, add_raw(ld<FrParams>(a), ld<FrParams>(b))); }
+void fr_sub_plus2(const uint32_t* a, const uint32_t* b, uint32_t* r) { st(r, sub_plus2(ld<FrParams>(a), ld<FrParams>(b))); }
+void fr_reduce2(const uint32_t* a, uint32_t* r) { st(r, reduce2(ld<FrParams>(a))); }
+void fr_reduce1(const uint32_t* a, uint32_t* r) { st(r, reduce1(ld<FrParams>(a))); }
+void butterfly_dit(uint32_t* x0, uint32_t* x1, const uint32_t* w, int unit) { butterfly_impl<true>(x0, x1, w, unit); }
+void butterfly_dif(uint32_t* x0, uint32_t* x1, const uint32_t* w, int unit) { butterfly_impl<false>(x0, x1, w, unit); }
+
 #define CURVE_OPS(PFX, F)                                                                       \
   void PFX##_madd(const uint32_t* p, const uint32_t* q, uint32_t* r) { stx(r, xyzz_madd(ldx<F>(p), lda<F>(q))); } \
   void PFX##_add(const uint32_t* p, const uint32_t* q, uint32_t* r) { stx(r, xyzz_add(ldx<F>(p), ldx<F>(q))); } \
+  void PFX##_add_inline(const uint32_t* p, const uint32_t* q, uint32_t* r) { stx(r, xyzz_add_inline(ldx<F>(p), ldx<F>(q))); } \
   void PFX##_dbl(const uint32_t* p, uint32_t* r) { stx(r, xyzz_dbl(ldx<F>(p))); }               \
   void PFX##_dbl_affine(const uint32_t* q, uint32_t* r) { stx(r, xyzz_dbl_affine(lda<F>(q))); } \
   void PFX##_from_affine(const uint32_t* q, uint32_t* r) { stx(r, xyzz_from_affine(lda<F>(q))); }
@@ -322,7 +343,7 @@ def build(out_dir: str | None = None) -> str:
         open(os.path.join(fake, h), "w").close()
     top = os.path.join(out_dir, "top.cpp")
     with open(top, "w") as f:
-        f.write('#include "ec.cuh"\n')
+        f.write('#include "ec.cuh"\n#include "ntt_butterfly.cuh"\n')
     pre = subprocess.run(
         ["g++", "-E", "-P", "-nostdinc", "-I", fake, "-I", CSRC, "-D__device__=", "-D__forceinline__=",
          "-D__noinline__=", "-DBG_DEV=inline", "-x", "c++", top],
