@@ -203,15 +203,19 @@ BG_DEV Fp<P> inv(const Fp<P>& a) {
 
 // ---------------------------------------------------------------- inversion by division steps
 // 1/a for a Montgomery element a (0 -> 0): the division steps of Bernstein and Yang ("Fast
-// constant-time gcd computation and modular inversion", CHES 2019), in the variant that starts at
-// delta = 1/2 and needs at most 590 steps for inputs below 2^256.  30 steps at a time run on the
-// low words of f and g alone and give a 2 x 2 matrix (entries at most 2^30), which is then applied
+// constant-time gcd computation and modular inversion", CHES 2019),
+//   (delta, f, g) -> (1 - delta, g, (g - f) / 2)                 if delta > 0 and g is odd
+//                    (1 + delta, f, (g + (g mod 2) f) / 2)       otherwise
+// from delta = 1, f = p, g = a, which end at g = 0 and f = +-1 after at most floor((49 254 + 57) / 17) =
+// 735 steps (their Theorem 11.2 with f^2 + 4 g^2 <= 5 2^508).  30 steps at a time run on the low words of
+// f and g alone and give a 2 x 2 matrix (entries at most 2^30), which is then applied
 // to the whole f and g (exactly divisible by 2^30) and to d and e, which follow f and g modulo p:
 // (u d + v e + m p) / 2^30 with the m, centred in +-2^29, that makes it whole, so d and e grow by
 // at most p / 2 per matrix and need no reduction before the end.  e starts at R^2, so d ends as
 // +-(a R)^-1 R^2, the Montgomery inverse.  The inversion is what a CTA of the batch-affine bucket
-// accumulation waits for, so its latency counts: the steps are the same for every input (no
-// divergence between lanes that invert together), about 20 instructions each, and a matrix costs
+// accumulation waits for, so its latency counts: a step is the same few instructions for every input
+// (no divergence between lanes that invert together; the sign s of f is a factor of three
+// multiply-adds), and a matrix costs
 // 90 multiply-adds; binary Euclid with its compares and shifts of whole numbers took about three
 // times as long, the Fermat power is 320 dependent products.  Requires a < p (every stored element
 // is).
@@ -224,31 +228,31 @@ BG_DEV int32_t limb30(const uint32_t* w, int i) {
   const uint32_t hi = (s && l + 1 < 8) ? w[l + 1] << (32 - s) : 0u;
   return (int32_t)((lo | hi) & (uint32_t)kMask);
 }
-// 30 division steps on the low words: (f, g) -> matrix (u, v; q, r) / 2^30; eta = -delta - 1/2
-BG_DEV int32_t steps30(int32_t eta, uint32_t f, uint32_t g, int32_t* mat) {
-  uint32_t u = 1, v = 0, q = 0, r = 1;
+// 30 division steps on the low words of f and g.  With `mat` = (u v; q r), 2^i f_i = u f + v g and 2^i g_i =
+// q f + r g after i steps for the f and g at entry: a step adds s f to g (s = 0 for an even g, -1 where it
+// also moves g into f, else 1), so (q, r) take s (u, v), and f's row doubles where g is halved.
+BG_DEV int32_t steps30(int32_t delta, uint32_t f, uint32_t g, int32_t* mat) {
+  int32_t u = 1, v = 0, q = 0, r = 1;
 #pragma unroll 6
   for (int i = 0; i < 30; i++) {
-    uint32_t c1 = (uint32_t)(eta >> 31);  // delta > 0
-    const uint32_t c2 = 0u - (g & 1u);
-    const uint32_t x = (f ^ c1) - c1, y = (u ^ c1) - c1, z = (v ^ c1) - c1;  // +-f, u, v
-    g += x & c2;
-    q += y & c2;
-    r += z & c2;
-    c1 &= c2;  // swap: delta > 0 and g odd
-    eta = (int32_t)(((uint32_t)eta ^ c1) - 1u);
-    f += g & c1;
-    u += q & c1;
-    v += r & c1;
-    g >>= 1;
-    u <<= 1;
-    v <<= 1;
+    const int32_t odd = (int32_t)(g & 1u);
+    const bool move = odd && delta > 0;
+    const int32_t s = move ? -1 : odd;
+    const uint32_t sum = g + (uint32_t)s * f;
+    const int32_t q1 = q + s * u, r1 = r + s * v;
+    delta = 1 + (move ? -delta : delta);
+    f = move ? g : f;
+    u = 2 * (move ? q : u);
+    v = 2 * (move ? r : v);
+    g = sum >> 1;
+    q = q1;
+    r = r1;
   }
-  mat[0] = (int32_t)u;
-  mat[1] = (int32_t)v;
-  mat[2] = (int32_t)q;
-  mat[3] = (int32_t)r;
-  return eta;
+  mat[0] = u;
+  mat[1] = v;
+  mat[2] = q;
+  mat[3] = r;
+  return delta;
 }
 BG_DEV void update_fg(int32_t* f, int32_t* g, const int32_t* m) {
   int64_t cf = (int64_t)m[0] * f[0] + (int64_t)m[1] * g[0];
@@ -307,10 +311,10 @@ BG_DEV Fp<P> inv_binary(const Fp<P>& a) {
     d[i] = 0;
     e[i] = dsteps::limb30(r2, i);
   }
-  int32_t eta = -1;  // delta = 1/2
+  int32_t delta = 1;
 #pragma unroll 1
-  for (int b = 0; b < 20; b++) {  // 600 steps
-    eta = dsteps::steps30(eta, (uint32_t)(f[0] | (f[1] << 30)), (uint32_t)(g[0] | (g[1] << 30)), m);
+  for (int b = 0; b < 25; b++) {  // 750 steps
+    delta = dsteps::steps30(delta, (uint32_t)(f[0] | (f[1] << 30)), (uint32_t)(g[0] | (g[1] << 30)), m);
     dsteps::update_de(d, e, m, p, P::N0 & 0x3fffffffu);
     dsteps::update_fg(f, g, m);
     int32_t left = 0;
@@ -318,16 +322,16 @@ BG_DEV Fp<P> inv_binary(const Fp<P>& a) {
     for (int i = 0; i < 9; i++) left |= g[i];
     if (left == 0) break;
   }
-  // f = +-1, d = +-1/a with |d| <= (1/2 + 20/2) p: make it d f, then add 11 p and subtract 16 p, 8 p,
+  // f = +-1, d = +-1/a with |d| <= (1/2 + 25/2) p: make it d f, then add 13 p and subtract 16 p, 8 p,
   // 4 p, 2 p and p where they fit (a = 0 leaves d = 0)
   const int32_t sign = f[8] >> 31;
   int64_t c = 0;
   int32_t t[9];
 #pragma unroll
   for (int i = 0; i < 9; i++) {
-    c += (int64_t)((d[i] ^ sign) - sign) + (int64_t)11 * p[i];
+    c += (int64_t)((d[i] ^ sign) - sign) + (int64_t)13 * p[i];
     t[i] = (int32_t)c & dsteps::kMask;
-    c >>= 30;  // ends at zero: the sum is below 22 p < 2^259
+    c >>= 30;  // ends at zero: the sum lies in [0, 26 p], below 2^259
   }
 #pragma unroll
   for (int k = 4; k >= 0; k--) {

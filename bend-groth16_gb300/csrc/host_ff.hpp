@@ -200,8 +200,8 @@ inline Fe fe_pow_u64(const Mod& m, const Fe& a, uint64_t e) {
   return fe_pow(m, a, ee);
 }
 // 1/a for a Montgomery element below p (0 -> 0): Bernstein and Yang's division steps, as the
-// device's inversion (fp.cuh), 62 steps to a matrix and five signed 62-bit limbs.  2 us against the
-// Fermat power's 8; a proof's host tail makes three, a standalone MSM's one.
+// device's inversion (fp.cuh, which has the recurrence), 62 steps to a matrix and five signed 62-bit
+// limbs.  2 us against the Fermat power's 8; a proof's host tail makes three, a standalone MSM's one.
 namespace dsteps {
 constexpr int64_t kMask = ((int64_t)1 << 62) - 1;
 struct S62 {
@@ -211,29 +211,34 @@ inline S62 split(const uint64_t* w) {
   return {{(int64_t)(w[0] & kMask), (int64_t)((w[0] >> 62 | w[1] << 2) & kMask), (int64_t)((w[1] >> 60 | w[2] << 4) & kMask),
            (int64_t)((w[2] >> 58 | w[3] << 6) & kMask), (int64_t)(w[3] >> 56)}};
 }
-inline int64_t steps62(int64_t eta, uint64_t f, uint64_t g, int64_t* m) {
-  uint64_t u = 1, v = 0, q = 0, r = 1;
-  for (int i = 0; i < 62; i++) {
-    uint64_t c1 = (uint64_t)(eta >> 63);  // delta > 0
-    const uint64_t c2 = 0 - (g & 1);
-    const uint64_t x = (f ^ c1) - c1, y = (u ^ c1) - c1, z = (v ^ c1) - c1;
-    g += x & c2;
-    q += y & c2;
-    r += z & c2;
-    c1 &= c2;
-    eta = (int64_t)(((uint64_t)eta ^ c1) - 1);
-    f += g & c1;
-    u += q & c1;
-    v += r & c1;
-    g >>= 1;
-    u <<= 1;
-    v <<= 1;
+// (a run of even g is taken at once: the time depends on the input, as that of the additions does)
+inline int64_t steps62(int64_t delta, uint64_t f, uint64_t g, int64_t* m) {
+  int64_t u = 1, v = 0, q = 0, r = 1;
+  for (int left = 62;;) {
+    const int even = __builtin_ctzll(g | (uint64_t)1 << left);
+    delta += even;
+    g >>= even;
+    u = (int64_t)((uint64_t)u << even);
+    v = (int64_t)((uint64_t)v << even);
+    left -= even;
+    if (left == 0) break;
+    const bool move = delta > 0;
+    const uint64_t f0 = f;
+    const int64_t u0 = u, v0 = v;
+    f = move ? g : f;
+    u = 2 * (move ? q : u);
+    v = 2 * (move ? r : v);
+    g = (g + (move ? 0 - f0 : f0)) >> 1;
+    q += move ? -u0 : u0;
+    r += move ? -v0 : v0;
+    delta = 1 + (move ? -delta : delta);
+    left--;
   }
-  m[0] = (int64_t)u;
-  m[1] = (int64_t)v;
-  m[2] = (int64_t)q;
-  m[3] = (int64_t)r;
-  return eta;
+  m[0] = u;
+  m[1] = v;
+  m[2] = q;
+  m[3] = r;
+  return delta;
 }
 // (a, b) = (m0 a + m1 b + k p, m2 a + m3 b + l p) / 2^62 with the k, l (n62 = -p^-1 mod 2^62) that make
 // them whole, centred; without p (n62 = 0) for the pair that is divisible by itself
@@ -260,19 +265,19 @@ inline Fe fe_inv(const Mod& m, const Fe& a) {
   using dsteps::S62;
   const S62 p = dsteps::split(m.p);
   S62 f = p, g = dsteps::split(a.v), d = {{0, 0, 0, 0, 0}}, e = dsteps::split(m.r2);
-  int64_t eta = -1, mat[4];
-  for (int i = 0; i < 10; i++) {  // 620 steps, of which 590 suffice
-    eta = dsteps::steps62(eta, (uint64_t)f.v[0] | (uint64_t)f.v[1] << 62, (uint64_t)g.v[0] | (uint64_t)g.v[1] << 62, mat);
+  int64_t delta = 1, mat[4];
+  for (int i = 0; i < 12; i++) {  // 744 steps, of which 735 suffice
+    delta = dsteps::steps62(delta, (uint64_t)f.v[0] | (uint64_t)f.v[1] << 62, (uint64_t)g.v[0] | (uint64_t)g.v[1] << 62, mat);
     dsteps::apply(d, e, mat, p, m.n0 & (uint64_t)dsteps::kMask);
     dsteps::apply(f, g, mat, p, 0);
     if ((g.v[0] | g.v[1] | g.v[2] | g.v[3] | g.v[4]) == 0) break;
   }
-  // f = +-1 and |d| <= (1/2 + 10/2) p: d f + 6 p lies in (0, 12 p), below 2^258
+  // f = +-1 and |d| <= (1/2 + 12/2) p: d f + 7 p lies in (0, 14 p), below 2^258
   const int64_t sign = f.v[4] >> 63;
   __int128 c = 0;
   uint64_t t[5];
   for (int i = 0; i < 5; i++) {
-    c += (__int128)((d.v[i] ^ sign) - sign) + (__int128)6 * p.v[i];
+    c += (__int128)((d.v[i] ^ sign) - sign) + (__int128)7 * p.v[i];
     t[i] = (uint64_t)c & (uint64_t)dsteps::kMask;
     c >>= 62;
   }

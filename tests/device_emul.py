@@ -311,6 +311,7 @@ void fq2_inv_fast(const uint32_t* a, uint32_t* r) { st2(r, field_inv_fast(ld2(a)
 void g1_pair_add(const uint32_t* p, const uint32_t* q, uint32_t* kind, uint32_t* r) { pair_add_impl<Fq>(p, q, r, kind); }
 void g2_pair_add(const uint32_t* p, const uint32_t* q, uint32_t* kind, uint32_t* r) { pair_add_impl<Fq2>(p, q, r, kind); }
 
+int32_t dsteps30(int32_t delta, uint32_t f, uint32_t g, int32_t* mat) { return dsteps::steps30(delta, f, g, mat); }
 void fq_mul_loose(const uint32_t* a, const uint32_t* b, uint32_t* r) { st(r, mul_loose(ld<FqParams>(a), ld<FqParams>(b))); }
 void fr_mul_loose(const uint32_t* a, const uint32_t* b, uint32_t* r) { st(r, mul_loose(ld<FrParams>(a), ld<FrParams>(b))); }
 void fq_sub_loose(const uint32_t* a, const uint32_t* b, uint32_t* r) { st(r, sub_loose(ld<FqParams>(a), ld<FqParams>(b))); }

@@ -89,6 +89,24 @@ def test_inlined_additions(dev, g2):  # noqa: F811
             assert io.from_xyzz(got) == curve.add(A, B)
 
 
+def test_division_steps_follow_the_recurrence(dev):  # noqa: F811
+    """30 steps on the low words: the matrix takes the whole numbers where Bernstein and Yang's
+    recurrence does"""
+    from test_host_ff_cpu import divstep
+    rng = random.Random(35)
+    for i in range(400):
+        f, g = rng.getrandbits(254) | 1, rng.getrandbits(254) << rng.choice([0, 1, 7, 29, 40])
+        f, g = (f, g) if i % 3 else (-f, g)
+        delta = rng.randint(-40, 40)
+        m = (ctypes.c_int32 * 4)()
+        got = dev.lib.dsteps30(delta, ctypes.c_uint32(f & 0xffffffff), ctypes.c_uint32(g & 0xffffffff), m)
+        d, F, G = delta, f, g
+        for _ in range(30):
+            d, F, G = divstep(d, F, G)
+        u, v, q, r = m
+        assert (u * f + v * g, q * f + r * g, got) == (F << 30, G << 30, d)
+
+
 def test_pair_cases_of_x_zero(dev):  # noqa: F811
     """a point of x = 0 beside a missing one has a zero denominator without an addition due; two of
     equal x and opposite y have no sum, equal ones the tangent"""

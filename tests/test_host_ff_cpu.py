@@ -21,6 +21,8 @@ extern "C" {
 void t_mul(int fq, const uint64_t* a, const uint64_t* b, uint64_t* r) { st(r, fe_mul(fq ? FQ : FR, ld(a), ld(b))); }
 void t_to_mont(int fq, const uint64_t* a, uint64_t* r) { st(r, fe_to_mont(fq ? FQ : FR, ld(a))); }
 void t_from_mont(int fq, const uint64_t* a, uint64_t* r) { st(r, fe_from_mont(fq ? FQ : FR, ld(a))); }
+void t_inv(int fq, const uint64_t* a, uint64_t* r) { st(r, fe_inv(fq ? FQ : FR, ld(a))); }
+void t_steps(int64_t delta, uint64_t f, uint64_t g, int64_t* out) { out[4] = dsteps::steps62(delta, f, g, out); }
 void t_blinding(const uint32_t* rs16, uint64_t* out) { blinding_scalars(rs16, out, out + 4, out + 8); }
 void t_point(const uint32_t* w32, uint64_t* out) {
   const Aff<Fq2Ops> a = aff_from_input32<Fq2Ops>(w32);
@@ -96,3 +98,39 @@ def test_input_points_are_reduced(lib):
         out = (ctypes.c_uint64 * 16)()
         lib.t_point(w, out)
         assert [value(out[4 * i:4 * i + 4]) for i in range(4)] == [x % p for x in v]
+
+
+def divstep(delta, f, g):
+    """Bernstein and Yang's division step (CHES 2019, section 8)"""
+    if delta > 0 and g & 1:
+        return 1 - delta, g, (g - f) // 2
+    return 1 + delta, f, (g + (g & 1) * f) // 2
+
+
+def test_division_steps_follow_the_recurrence(lib):
+    """62 steps on the low words: the matrix takes the whole numbers where the recurrence does"""
+    rng = random.Random(74)
+    for i in range(400):
+        f, g = rng.getrandbits(254) | 1, rng.getrandbits(254) << rng.choice([0, 1, 7, 61, 70])
+        f, g = (f, g) if i % 3 else (-f, g)
+        delta = rng.randint(-40, 40)
+        out = (ctypes.c_int64 * 5)()
+        mask = (1 << 64) - 1
+        lib.t_steps(ctypes.c_int64(delta), ctypes.c_uint64(f & mask), ctypes.c_uint64(g & mask), out)
+        d, F, G = delta, f, g
+        for _ in range(62):
+            d, F, G = divstep(d, F, G)
+        u, v, q, r = out[:4]
+        assert (u * f + v * g, q * f + r * g, out[4]) == (F << 62, G << 62, d)
+
+
+@pytest.mark.parametrize("fq", [0, 1])
+def test_inverse(lib, fq):
+    p = o.P_FQ if fq else o.P_FR
+    rng = random.Random(75 + fq)
+    ri = pow(R, -1, p)
+    vals = [1, 2, 3, p - 1, p - 2, R % p, R * R % p] + [1 << k for k in range(0, 254, 5)] + \
+        [p - (1 << k) for k in range(1, 250, 11)] + [rng.randrange(1, p) for _ in range(3000)]
+    assert call(lib, "t_inv", fq, w64(0)) == 0
+    for a in vals:
+        assert call(lib, "t_inv", fq, w64(a)) == pow(a * ri, -1, p) * R % p
