@@ -270,6 +270,24 @@ enum : uint32_t {
   BG_DSTATUS_COLUMN = 8u,        // an R1CS column index was outside the assignment
 };
 
+// A positive number that is computed once per process and read by several threads (lanes and server
+// workers): threads that meet at the first use compute the same number.
+class CachedInt {
+ public:
+  template <class Fn>
+  int get(Fn&& compute) {
+    int v = v_.load(std::memory_order_relaxed);
+    if (v == 0) {
+      v = compute();
+      v_.store(v, std::memory_order_relaxed);
+    }
+    return v;
+  }
+
+ private:
+  std::atomic<int> v_{0};
+};
+
 inline unsigned ceil_div(size_t a, size_t b) { return (unsigned)((a + b - 1) / b); }
 
 void set_noctx_error(const std::string& msg);

@@ -507,21 +507,26 @@ uint32_t slice_entries(size_t max_entries, size_t nkeys) {
 // its tree, which the CTA's neighbours on the SM start together).  G1 MSM 2^20's two rounds: 1.82 ms
 // with at most 24 positions, 1.73 with 48, 1.71 with 128 (one wave of 115 and 57).
 constexpr double kPairPer = 64;
-// Resident threads of a pair round on the whole GPU (SMs x CTAs per SM x CTA size).
+// Threads of a kernel resident on the whole GPU at once (SMs x CTAs per SM x CTA size).
+template <class K>
+int resident_threads(K kernel, int threads, size_t smem) {
+  int dev = 0, sms = 0, occ = 0;
+  BG_CUDA(cudaGetDevice(&dev));
+  BG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  BG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem));
+  return sms * (occ > 0 ? occ : 1) * threads;
+}
+// of a pair round
 template <class F>
 double pair_slots() {
-  static std::atomic<double> slots{0.0};
-  double s = slots.load();
-  if (s == 0.0) {
-    int dev = 0, sms = 0, occ = 0;
-    BG_CUDA(cudaGetDevice(&dev));
-    BG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    BG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pair_round<F, true>, kPairThreads<F>,
-                                                          pair_smem_bytes<F>()));
-    s = (double)sms * (occ > 0 ? occ : 1) * kPairThreads<F>;
-    slots.store(s);
-  }
-  return s;
+  static CachedInt slots;
+  return slots.get([] { return resident_threads(k_pair_round<F, true>, kPairThreads<F>, pair_smem_bytes<F>()); });
+}
+// of the accumulation
+template <class F>
+double acc_slots() {
+  static CachedInt slots;
+  return slots.get([] { return resident_threads(k_bucket_acc<F>, kAccThreads<F>, 0); });
 }
 
 // Pieces after the first from which a bucket goes to k_bucket_heavy, whose tree costs its eight
@@ -543,20 +548,6 @@ struct BucketScratch {
   uint32_t* heavy = nullptr;  // 1 + slices / limit + 1
 };
 inline size_t bucket_slices(size_t max_entries, uint32_t K) { return (max_entries + K - 1) / K; }
-
-// Accumulation threads resident on the whole GPU at once (SMs x CTAs per SM x CTA size).
-template <class F>
-double acc_slots() {
-  static double slots = 0;
-  if (slots == 0) {
-    int dev = 0, sms = 0, occ = 0;
-    BG_CUDA(cudaGetDevice(&dev));
-    BG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    BG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bucket_acc<F>, kAccThreads<F>, 0));
-    slots = (double)sms * (occ > 0 ? occ : 1) * kAccThreads<F>;
-  }
-  return slots;
-}
 
 // Every slice costs the same K additions, so an accumulation grid of 1.6 waves takes as long
 // as 2.  When the model's slices need more than one wave, K is rounded so that the grid is a
@@ -796,14 +787,12 @@ inline int log2_of(uint32_t x) {
 }
 template <class F>
 int reduce_blocks_per_sm(uint32_t RT) {
-  static int cache[9] = {};
-  const int lrt = log2_of(RT);
-  if (!cache[lrt]) {
+  static CachedInt cache[9];
+  return cache[log2_of(RT)].get([&] {
     int n = 0;
     BG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_window_reduce<F>, (int)RT, reduce_sm_bytes<F>(RT, 2)));
-    cache[lrt] = n > 0 ? n : 1;
-  }
-  return cache[lrt];
+    return n > 0 ? n : 1;
+  });
 }
 // dependent additions over a thread's own buckets
 inline double reduce_chain(uint32_t M, double entries_per_slice) {
@@ -900,15 +889,13 @@ ReduceShape reduce_shape_work(uint32_t nb, int sets, size_t entries, uint32_t K,
 // group's exchanges) with one warp per scheduler and kCoopWarpCost more for each further one.
 template <class F>
 int reduce_coop_blocks_per_sm(uint32_t RT) {
-  static int cache[6] = {};
-  const int lrt = log2_of(RT);
-  if (!cache[lrt]) {
+  static CachedInt cache[6];
+  return cache[log2_of(RT)].get([&] {
     int n = 0;
     BG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_window_reduce_coop<F>, (int)RT * kCoopLanes,
                                                           RT * coop_group_words<F>() * sizeof(uint32_t)));
-    cache[lrt] = n > 0 ? n : 1;
-  }
-  return cache[lrt];
+    return n > 0 ? n : 1;
+  });
 }
 template <class F>
 ReduceShape reduce_shape_coop(uint32_t nb, int sets, size_t entries, uint32_t K, int sm_count) {

@@ -115,3 +115,37 @@ def test_a_stream_still_running_is_no_error(lib):
     assert (lib.t_stream_drained(600, ctypes.byref(last)), last.value) == (0, 0)
     assert (lib.t_stream_drained(0, ctypes.byref(last)), last.value) == (1, 0)
     assert lib.t_stream_drained(999, ctypes.byref(last)) == 2
+
+
+def test_cached_numbers_are_shared_without_a_race(tmp_path):
+    """what lanes compute at the same first use, under the thread sanitizer"""
+    src = SRC + r"""
+#include <thread>
+int main() {
+  static CachedInt cache[4];
+  std::vector<std::thread> t;
+  std::atomic<int> bad{0};
+  for (int i = 0; i < 8; i++)
+    t.emplace_back([&] {
+      for (int k = 0; k < 4000; k++)
+        if (cache[k % 4].get([&] { return 7 + k % 4; }) != 7 + k % 4) bad++;
+    });
+  for (auto& x : t) x.join();
+  return bad.load();
+}
+"""
+    fake = tmp_path / "fake"
+    fake.mkdir()
+    (fake / "cuda_runtime.h").write_text(FAKE)
+    (tmp_path / "t.cpp").write_text(src)
+    exe = str(tmp_path / "t")
+    made = subprocess.run(["g++", "-O1", "-g", "-std=c++17", "-fsanitize=thread", "-pthread", "-I", str(fake), "-I",
+                           os.path.join(PKG, "csrc"), "-x", "c++", "-o", exe, str(tmp_path / "t.cpp")],
+                          capture_output=True, text=True)
+    if made.returncode and "tsan" in made.stderr:
+        pytest.skip("no thread sanitizer here")
+    assert made.returncode == 0, made.stderr[-2000:]
+    out = subprocess.run([exe], capture_output=True, text=True)
+    if "unexpected memory mapping" in out.stderr:  # the sanitizer and this kernel's address randomisation
+        out = subprocess.run(["setarch", "-R", exe], capture_output=True, text=True)
+    assert out.returncode == 0, out.stderr[-2000:]
