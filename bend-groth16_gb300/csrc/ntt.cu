@@ -120,6 +120,7 @@ __global__ void __launch_bounds__(NT, OCC) k_ntt_pass(NttVecs vecs, const uint32
       x = mul(load_fp<FrParams>(zinv), sub(mul(x, y), z));
     }
     if (pre_mode != SC_NONE) x = mul(scale_factor(pre_mode, j, L, sc), x);
+    else if (load_mode == LD_PLAIN) x = below2(x);
     tile_store(sm, E, e, x);
   }
   __syncthreads();

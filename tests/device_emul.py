@@ -318,6 +318,7 @@ void fq_sub_loose(const uint32_t* a, const uint32_t* b, uint32_t* r) { st(r, sub
 void fr_add_raw(const uint32_t* a, const uint32_t* b, uint32_t* r) { st(r, add_raw(ld<FrParams>(a), ld<FrParams>(b))); }
 void fr_sub_plus2(const uint32_t* a, const uint32_t* b, uint32_t* r) { st(r, sub_plus2(ld<FrParams>(a), ld<FrParams>(b))); }
 void fr_reduce2(const uint32_t* a, uint32_t* r) { st(r, reduce2(ld<FrParams>(a))); }
+void fr_below2(const uint32_t* a, uint32_t* r) { st(r, below2(ld<FrParams>(a))); }
 void fr_reduce1(const uint32_t* a, uint32_t* r) { st(r, reduce1(ld<FrParams>(a))); }
 void butterfly_dit(uint32_t* x0, uint32_t* x1, const uint32_t* w, int unit) { butterfly_impl<true>(x0, x1, w, unit); }
 void butterfly_dif(uint32_t* x0, uint32_t* x1, const uint32_t* w, int unit) { butterfly_impl<false>(x0, x1, w, unit); }

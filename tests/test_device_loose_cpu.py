@@ -49,6 +49,9 @@ def test_ntt_helpers(dev):  # noqa: F811
     rng, W, r = random.Random(32), dev.words, PR
     for a in ends(r, 4, rng):
         assert dev.call("fr_reduce2", [W(a)], 8) == (a - 2 * r if a >= 2 * r else a)
+    for a in ends(r, 6, rng) + [R - 1, R - 2, R >> 1]:  # a caller's word: any of 256 bits
+        got = dev.call("fr_below2", [W(a)], 8)
+        assert got % r == a % r and got < 2 * r
     two = ends(r, 2, rng)
     for a in two:
         assert dev.call("fr_reduce1", [W(a)], 8) == a % r

@@ -18,6 +18,33 @@ def lifted(words, p):
     return bendg.ints_to_wire([v + (2**256 - 1 - v) // p * p if v else 0 for v in vals]).reshape(words.shape)
 
 
+@pytest.mark.parametrize("log2n", [0, 1, 5, 9, 13, 16])
+@pytest.mark.parametrize("mode", [bendg.NTT_FORWARD, bendg.NTT_INVERSE, bendg.NTT_COSET_FORWARD,
+                                  bendg.NTT_COSET_INVERSE])
+def test_ntt_of_lifted_words(ctx, log2n, mode):
+    rng = np.random.default_rng(60 + log2n)
+    vals = [int.from_bytes(rng.bytes(32), "little") % o.P_FR for _ in range(1 << log2n)]
+    words = bendg.ints_to_wire(vals)
+    up = lifted(words.reshape(-1), o.P_FR).reshape(words.shape)
+    some = np.where(rng.random(len(vals))[:, None] < 0.5, up, words)
+    want = ctx.ntt(words.reshape(-1), log2n, mode)
+    for w in (up, some):
+        got = ctx.ntt(np.ascontiguousarray(w).reshape(-1), log2n, mode)
+        if log2n:
+            assert np.array_equal(got, want)
+        else:  # nothing is computed: the word comes back
+            assert bendg.wire_to_ints(got)[0] % o.P_FR == bendg.wire_to_ints(want)[0]
+
+
+@pytest.mark.parametrize("log2d", [1, 7, 14, 15])
+def test_qap_of_lifted_words(ctx, log2d):
+    rng = np.random.default_rng(61 + log2d)
+    abc = [bendg.ints_to_wire([int.from_bytes(rng.bytes(32), "little") % o.P_FR for _ in range(1 << log2d)]).reshape(-1)
+           for _ in range(3)]
+    want = ctx.qap_h(*abc, log2d)
+    assert np.array_equal(ctx.qap_h(*[lifted(v, o.P_FR) for v in abc], log2d), want)
+
+
 def test_blinding_words_and_key_points(ctx, tmp_path):
     import shutil
     d = os.path.join(GOLDEN, "k4")
