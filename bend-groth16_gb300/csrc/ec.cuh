@@ -46,10 +46,10 @@ BG_DEV Fq2 field_inv_any(const Fq2& a) {
   return {fmul(a.c0, ni), neg(fmul(a.c1, ni))};
 }
 
-// 1/a by binary Euclid (fp.cuh): the latency-critical single inversion of a batch
-BG_DEV Fq field_inv_fast(const Fq& a) { return inv_binary(a); }
+// 1/a by division steps (fp.cuh): the latency-critical inversions of a batch
+BG_DEV Fq field_inv_fast(const Fq& a) { return inv_divsteps(a); }
 BG_DEV Fq2 field_inv_fast(const Fq2& a) {
-  const Fq ni = inv_binary(add(fsqr(a.c0), fsqr(a.c1)));
+  const Fq ni = inv_divsteps(add(fsqr(a.c0), fsqr(a.c1)));
   return {fmul(a.c0, ni), neg(fmul(a.c1, ni))};
 }
 

@@ -300,7 +300,7 @@ BG_DEV void update_de(int32_t* d, int32_t* e, const int32_t* m, const int32_t* p
 }  // namespace dsteps
 
 template <class P>
-BG_DEV Fp<P> inv_binary(const Fp<P>& a) {
+BG_DEV Fp<P> inv_divsteps(const Fp<P>& a) {
   const uint32_t pw[8] = {P::P0, P::P1, P::P2, P::P3, P::P4, P::P5, P::P6, P::P7};
   const uint32_t r2[8] = {P::R2_0, P::R2_1, P::R2_2, P::R2_3, P::R2_4, P::R2_5, P::R2_6, P::R2_7};
   int32_t p[9], f[9], g[9], d[9], e[9], m[4];

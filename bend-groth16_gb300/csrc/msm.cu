@@ -310,11 +310,11 @@ __global__ void __launch_bounds__(128) k_build_table(const uint32_t* __restrict_
 // repeated thousands of times) is joined beforehand by k_bucket_heavy: the thread that owns its
 // first piece lists it in heavy[1 + i] (heavy[0] counts, cleared before the accumulation).
 // G2's accumulation stages the next entry's point in shared memory (cp.async) instead of
-// registers, where a prefetched Fq2 point held 32 registers across the whole addition: 222
-// registers instead of 242 and 1% of the G2 accumulation.  The registers saved do
+// registers, where a prefetched Fq2 point held 32 registers across the whole addition: 20 registers
+// fewer (214 now) and 1% of the G2 accumulation.  The registers saved do
 // not buy more warps: with 9, 10 or 12 per SM instead of 8 the accumulation of a 2^18 MSM measured
 // 2.25-2.29 ms against 1.89.  G1 keeps its register
-// prefetch (126 registers, four 128-thread CTAs per SM either way).
+// prefetch (128 registers, four 128-thread CTAs per SM either way).
 template <class F>
 constexpr bool kAccStaged = FieldWords<F>::value == 16;
 // CTA size of the accumulation

@@ -5,9 +5,9 @@
 // every bucket: a round adds the points of each bucket in pairs, in affine coordinates, and
 // writes the sums as the bucket's points for the next round.  The additions of a round are
 // independent, so they share their field inversions: each thread multiplies its denominators
-// into a running product, the CTA multiplies the threads' products in a tree in shared memory,
-// one thread inverts the root (binary Euclid, inv_binary), and the tree and the running products
-// are walked back to give every addition 1 / d (Montgomery's simultaneous inversion).  An
+// into a running product, the CTA multiplies the threads' products in a tree in shared memory up to
+// 32 nodes, a warp inverts those side by side (division steps, inv_divsteps), and the tree and the
+// running products are walked back to give every addition 1 / d (Montgomery's simultaneous inversion).  An
 // addition then costs 5 products and a square (3 of them for the shared inversion) against
 // madd-2008-s's 8 products and 2 squares; the XYZZ accumulation that follows adds what the
 // rounds left, and the window reduction is unchanged.
@@ -26,7 +26,7 @@
 // a null entry of a padded bucket
 constexpr uint32_t kNullEntry = 0xffffffffu;
 
-// CTA size; four CTAs per SM in G1 (118 registers; five at 96 registers measured 1.57 -> 1.95 ms for
+// CTA size; four CTAs per SM in G1 (at most 122 registers; five at 96 measured 1.57 -> 1.95 ms for
 // G1 MSM 2^20's two rounds), two in G2
 template <class F>
 constexpr int kPairThreads = 128;

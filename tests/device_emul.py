@@ -5,8 +5,8 @@ Fr/Fq/Fq2 product, every G1/G2 addition and the NTT butterflies with PTX carry c
 module checks those chains without a GPU: it runs the C preprocessor over the headers,
 rewrites each `asm(...)` statement into C++ that executes the same PTX instructions on 32-bit
 integers with an explicit carry flag, compiles the result with g++ into a shared library and
-binds it with ctypes.  Everything outside the asm statements (the CIOS row loop, the Karatsuba
-split, the lazy-reduction bookkeeping, the XYZZ formulas and their special cases) is the
+binds it with ctypes.  Everything outside the asm statements (the CIOS row loop, the
+lazy-reduction bookkeeping, the XYZZ formulas and their special cases) is the
 device source itself, compiled for the host.
 
 PTX semantics emulated (PTX ISA, integer arithmetic instructions, extended precision):
@@ -283,7 +283,7 @@ template <bool DIT> static void butterfly_impl(uint32_t* x0, uint32_t* x1, const
   void PFX##_mul(const uint32_t* a, const uint32_t* b, uint32_t* r) { st(r, mul(ld<PARAMS>(a), ld<PARAMS>(b))); } \
   void PFX##_sqr(const uint32_t* a, uint32_t* r) { st(r, sqr(ld<PARAMS>(a))); }                 \
   void PFX##_inv(const uint32_t* a, uint32_t* r) { st(r, inv(ld<PARAMS>(a))); }                 \
-  void PFX##_inv_binary(const uint32_t* a, uint32_t* r) { st(r, inv_binary(ld<PARAMS>(a))); }   \
+  void PFX##_inv_binary(const uint32_t* a, uint32_t* r) { st(r, inv_divsteps(ld<PARAMS>(a))); }   \
   void PFX##_from_mont(const uint32_t* a, uint32_t* r) { st(r, from_mont(ld<PARAMS>(a))); }     \
   void PFX##_redc(const uint32_t* t16, uint32_t* r) { Wide t; memcpy(t.v, t16, 64); st(r, redc<PARAMS>(t)); }
 
