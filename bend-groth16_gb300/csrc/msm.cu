@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(kAccThreads<F>) k_bucket_acc(const uint32_t* _
 // CTA; the sum goes to the bucket.  The grid is fixed; CTAs loop over however many the
 // accumulation listed (none for uniformly spread scalars).
 template <class F>
-__global__ void __launch_bounds__(128) k_bucket_heavy(const uint32_t* __restrict__ offsets,
+__global__ void __launch_bounds__(256) k_bucket_heavy(const uint32_t* __restrict__ offsets,
                                                       const uint32_t* __restrict__ parts, uint32_t K,
                                                       const uint32_t* __restrict__ heavy,
                                                       uint32_t* __restrict__ buckets) {
@@ -473,7 +473,13 @@ __global__ void __launch_bounds__(128) k_bucket_heavy(const uint32_t* __restrict
     __syncthreads();
   }
 }
-constexpr uint32_t kHeavyThreads = 128;
+// CTA size: a bucket with a large part of an MSM's entries (the top bit of scalars of 16 bits under 15-bit
+// windows: 4000 pieces) is one CTA's strided sum, so a standalone G1 MSM takes as many threads as the
+// shared memory that needs no opt-in holds; a proof's pass fits beside other kernels' CTAs.
+template <class F>
+constexpr uint32_t heavy_threads(bool in_proof) {
+  return FieldWords<F>::value == 8 && !in_proof ? 256 : 128;
+}
 constexpr uint32_t kHeavyGrid = 152;
 
 #include "msm_pairs.cuh"
@@ -624,13 +630,15 @@ void bucket_accumulate(Ctx* prof, cudaStream_t st, const uint32_t* points, const
 
 // Heavy buckets on `st` (a pass that exits at once when there are none).
 template <class F>
-void bucket_heavy(Ctx* prof, cudaStream_t st, const uint32_t* offsets, uint32_t* buckets, const BucketScratch& s) {
+void bucket_heavy(Ctx* prof, cudaStream_t st, const uint32_t* offsets, uint32_t* buckets, const BucketScratch& s,
+                  bool in_proof) {
   constexpr int FW = FieldWords<F>::value;
   constexpr int PW = 4 * FW;
   std::unique_ptr<KernelTimer> kt(prof ? new KernelTimer(*prof, FW == 8 ? "msm_heavy_g1" : "msm_heavy_g2", st)
                                        : nullptr);
-  k_bucket_heavy<F><<<kHeavyGrid, kHeavyThreads, kHeavyThreads * PW * sizeof(uint32_t), st>>>(
-      offsets, s.parts, s.K, s.heavy, buckets);
+  const uint32_t threads = heavy_threads<F>(in_proof);
+  k_bucket_heavy<F><<<kHeavyGrid, threads, threads * PW * sizeof(uint32_t), st>>>(offsets, s.parts, s.K, s.heavy,
+                                                                                  buckets);
   BG_CHECK_LAUNCH();
 }
 
@@ -1134,7 +1142,7 @@ void msm_accumulate(Ctx& ctx, cudaStream_t st, const std::string& tag, const uin
     BG_CUDA(cudaStreamWaitEvent(st_reduce, ev, 0));
     rs = st_reduce;
   }
-  bucket_heavy<F>(prof, rs, acc_offsets, buckets, bs);
+  bucket_heavy<F>(prof, rs, acc_offsets, buckets, bs, plan.in_proof);
 
   // A reduction hidden under a later accumulation runs in CTAs of 128 threads: 256 leave no room for
   // an accumulation CTA on their SM for their whole (latency-bound) life, and smaller ones spread
@@ -1486,7 +1494,7 @@ void msm_g1_noalloc(const uint32_t* d_points, const uint32_t* d_scalars, size_t 
   k_scatter<<<ceil_div(n, 256), 256, 0, st>>>(d_scalars, n, c, W, nb, 0, cursor, sorted);
   BG_CHECK_LAUNCH();
   bucket_accumulate<Fq>(nullptr, st, d_points, offsets, sorted, (uint32_t)nkeys, max_entries, buckets, bs);
-  bucket_heavy<Fq>(nullptr, st, offsets, buckets, bs);
+  bucket_heavy<Fq>(nullptr, st, offsets, buckets, bs, false);
   const uint32_t* sums = window_reduce<Fq>(st, rsh, offsets, buckets, bs, nb, W, parts);
   BG_CUDA(cudaMemcpyAsync(g_noalloc_host_parts, sums, host_words * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   BG_CUDA(cudaMemcpyAsync(&g_noalloc_host_status, status, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
