@@ -1,8 +1,6 @@
 """Scalars of a few bits, as most of a circuit's assignment has: they leave all but a few hundred buckets
 empty and put many pieces into each of those (k_bucket_heavy's limit, msm.cu).  Results are checked
 through the discrete logarithms, and proofs against the same proof by another route."""
-import time
-
 import numpy as np
 import pytest
 
@@ -48,18 +46,18 @@ def test_scalars_of_8_bits_take_no_longer_than_uniform_ones(ctx, curve):
     rng = np.random.default_rng(640)
     ks = [int.from_bytes(rng.bytes(32), "little") % o.P_FR for _ in range(4096)]
     pts = np.tile(np.asarray(gpu_points(ctx, curve, ks)).reshape(len(ks), -1), (n // len(ks), 1))
+    run, g = (ctx.msm_g1, "g1") if curve == bendg.CURVE_G1 else (ctx.msm_g2, "g2")
     times = {}
     for name, bits in (("few", 8), ("uniform", 62)):
-        sc = few_bits(rng, n, bits, 1.0 if name == "uniform" else 0.0)
-        words = scalars_wire(sc)
-        run = ctx.msm_g1 if curve == bendg.CURVE_G1 else ctx.msm_g2
+        words = scalars_wire(few_bits(rng, n, bits, 1.0 if name == "uniform" else 0.0))
         got = []
-        for _ in range(9):
-            t = time.perf_counter()
+        for _ in range(5):  # the buckets' kernels on the device
+            ctx.profile(True)
             run(pts, words, n)
-            got.append(time.perf_counter() - t)
-        times[name] = sorted(got)[4]
-    assert times["few"] < times["uniform"], times
+            got.append(sum(ctx.kernel_stats(k + g)[1] for k in ("msm_bucket_acc_", "msm_heavy_", "msm_reduce_")))
+            ctx.profile(False)
+        times[name] = min(got)
+    assert 0 < times["few"] < times["uniform"], times
 
 
 @pytest.mark.parametrize("bits,spread", [(1, 0.0), (8, 0.1)])
