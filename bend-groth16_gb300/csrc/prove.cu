@@ -701,7 +701,7 @@ static size_t msm_footprint_c(size_t n, bool g2, int c) {
 // and a one-shot proof's.  They are wider than the tuned ones in places and stay as they are when
 // those change, so that a budget admits what it admitted.  A proof's scratch lies below the
 // reservation (SquareChain(2^10): 15 of 30 MB, 2^18: 0.8 of 1.5 GB, 2^20: 2.6 of 7.7 GB): without
-// pair rounds at most three quarters of it for any header, and prove_round_cap allows only the
+// pair rounds below four fifths of it for any header, and prove_round_cap allows only the
 // rounds that fit.
 static int reserved_c(size_t n, bool g2, bool in_proof) {
   static const signed char sets[2][13] = {{8, 8, 9, 9, 9, 10, 11, 12, 15, 15, 15, 15, 17},
